@@ -437,7 +437,15 @@ __device__ __forceinline__ int tc_b_off(int n, int k) {    // BF16 index in a pa
     return (((k >> 3) * 2 + (n >> 3)) * 128 + (n & 7) * 16 + (k & 7) * 2) >> 1;
 }
 
-__global__ void __launch_bounds__(kTcM) k_conv2d_tc_tap(TcConv a, int PWp) {
+constexpr int kTapCtas = 5;             // resident CTAs per SM (registers)
+// ICT, OCT, ACT: the channel counts and the activation fixed at compile time (0,
+// 0, -1: read from the arguments).  What bounds a tile is instruction issue
+// around 9 small MMAs: dividing an element index into (row, pixel) and testing
+// every channel cost 2,570 warp instructions per tile and layer (16 -> 16
+// channels at 640x480: 36 us); a fixed pixel per thread, all loads of a tile
+// before the first packing and the counts known take 21 us.
+template <int ICT, int OCT, int ACT>
+__global__ void __launch_bounds__(kTcM, kTapCtas) k_conv2d_tc_tap(TcConv a, int PWp) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_slot;
@@ -453,11 +461,16 @@ __global__ void __launch_bounds__(kTcM) k_conv2d_tc_tap(TcConv a, int PWp) {
     }
     {
         uint16_t *wd = reinterpret_cast<uint16_t *>(sB);
-        for (int i = tid; i < 9 * 256; i += kTcM) {
-            const int t = i >> 8, n = (i >> 4) & 15, c = i & 15;
-            uint16_t v = 0;
-            if (c < a.IC) v = a.wB[tc_b_off(n, c * 9 + t)];
-            wd[tc_b_off(n, t * 16 + c)] = v;
+        uint16_t v[9 * 256 / kTcM];
+#pragma unroll
+        for (int u = 0; u < 9 * 256 / kTcM; ++u) {
+            const int i = tid + u * kTcM, t = i >> 8, n = (i >> 4) & 15, c = i & 15;
+            v[u] = c < a.IC ? a.wB[tc_b_off(n, c * 9 + t)] : (uint16_t)0;
+        }
+#pragma unroll
+        for (int u = 0; u < 9 * 256 / kTcM; ++u) {
+            const int i = tid + u * kTcM, t = i >> 8, n = (i >> 4) & 15, c = i & 15;
+            wd[tc_b_off(n, t * 16 + c)] = v[u];
         }
     }
     if (tid == 0) {
@@ -476,6 +489,10 @@ __global__ void __launch_bounds__(kTcM) k_conv2d_tc_tap(TcConv a, int PWp) {
     const long tiles = tiles_img * a.nimg * nb;
     const long plane = (long)a.H * a.W, M = (long)a.OH * a.OW;
     const uint32_t lbo = 3u * (uint32_t)PWp * 16u;               // one 8-channel plane
+    // this thread's pixel of the rows' tails (6 rows of 2 dil pixels <= 96)
+    const int tail = 2 * a.dil, hr = tid / tail, hpx = tid - hr * tail;
+    const int IC = ICT > 0 ? ICT : a.IC, OC = OCT > 0 ? OCT : a.OC, act = ACT >= 0 ? ACT : a.act;
+    const bool halo = hr < 6, two = IC > 8;
     unsigned phase = 0;
     for (long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int item = (int)(tile / tiles_img);
@@ -483,26 +500,36 @@ __global__ void __launch_bounds__(kTcM) k_conv2d_tc_tap(TcConv a, int PWp) {
         const int t2 = (int)(tile - item * tiles_img);
         const int oy = t2 / tiles_x, ox0 = (t2 - oy * tiles_x) * kTapW;
         const float *x0 = (img ? a.x[1] : a.x[0]) + bi * a.xs;
-        // ---- stage rows oy - pad + ky * dil: consecutive threads take
-        // consecutive pixels, each 8 channels packed into one 16-byte store
-        for (int e = tid; e < 2 * 3 * PWp; e += kTcM) {
-            const int r = e / PWp, px = e - r * PWp;
-            const int ch = r / 3, ky = r - ch * 3;
+        // ---- stage rows oy - pad + ky * dil: thread t packs 8 channels of
+        // pixel t of each row (and one pixel of the rows' 2 dil tail) into one
+        // 16-byte store.  All loads of a tile are issued before the first is
+        // packed: one memory latency per tile.
+        float f[7][8];
+        auto load8 = [&](int ch, int ky, int px, bool on, float (&v)[8]) {
             const int iy = oy - a.pad + ky * a.dil, ix = ox0 - a.pad + px;
-            const bool ok = iy >= 0 && iy < a.H && ix >= 0 && ix < a.W;
-            const float *src = x0 + (long)iy * a.W + ix;
+            const bool ok = on && (unsigned)iy < (unsigned)a.H && (unsigned)ix < (unsigned)a.W;
+            // a channel plane's base is the same for the whole CTA
+            const unsigned off = ok ? (unsigned)(iy * a.W + ix) : 0u;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                v[j] = ok && ch * 8 + j < IC ? __ldg(x0 + (ch * 8 + j) * plane + off) : 0.f;
+        };
+        auto put8 = [&](int r, int px, const float (&v)[8]) {
             uint32_t q[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const int c0 = ch * 8 + 2 * j;
-                const float f0 = ok && c0 < a.IC ? __ldg(src + c0 * plane) : 0.f;
-                const float f1 = ok && c0 + 1 < a.IC ? __ldg(src + (c0 + 1) * plane) : 0.f;
-                const __nv_bfloat162 h2 = __floats2bfloat162_rn(f0, f1);
+                const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
                 q[j] = *reinterpret_cast<const uint32_t *>(&h2);
             }
             *reinterpret_cast<uint4 *>(patch + (size_t)(r * PWp + px) * 16) =
                 make_uint4(q[0], q[1], q[2], q[3]);
-        }
+        };
+#pragma unroll
+        for (int r = 0; r < 6; ++r) load8(r / 3, r % 3, tid, r < 3 || two, f[r]);
+        load8(hr / 3, hr % 3, kTapW + hpx, halo && (hr < 3 || two), f[6]);
+#pragma unroll
+        for (int r = 0; r < 6; ++r) put8(r, tid, f[r]);
+        if (halo) put8(hr, kTapW + hpx, f[6]);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;");
@@ -549,11 +576,11 @@ __global__ void __launch_bounds__(kTcM) k_conv2d_tc_tap(TcConv a, int PWp) {
             const float *aux = a.aux ? a.aux + bi * a.ys : nullptr;
 #pragma unroll
             for (int n = 0; n < kTcN; ++n) {
-                if (n < a.OC) {
+                if (n < OC) {
                     float v = __uint_as_float(r[n]);
                     if (a.bias) v += __ldg(a.bias + n);
-                    if (a.act == 1) v = v > 0.f ? v : v * 0.2f;
-                    if (a.act == 2) v = __ldg(aux + (long)n * M + mi) > 0.f ? v : v * 0.2f;
+                    if (act == 1) v = v > 0.f ? v : v * 0.2f;
+                    if (act == 2) v = __ldg(aux + (long)n * M + mi) > 0.f ? v : v * 0.2f;
                     y[(long)n * M + mi] = v;
                 }
             }
@@ -611,12 +638,27 @@ static int launch_conv2d_tc(const TcConv &a, cudaStream_t st) {
                            (a.nb > 0 ? a.nb : 1);
         if (tiles == 0) return SV_OK;
         int sms = 148;
-        const int rc = tc_setup(kKConv2dTap, (const void *)k_conv2d_tc_tap, &sms);
+        const int rc = tc_setup(kKConv2dTap, (const void *)k_conv2d_tc_tap<0, 0, -1>, &sms);
         if (rc) return rc;
-        const long cap = (long)sms * 8;               // 8 CTAs (32 TMEM columns each) per SM
-        const unsigned blocks = (unsigned)(tiles < cap ? tiles : cap);
+        // up to kTapCtas CTAs (32 TMEM columns each) per SM, as many as give every
+        // CTA the same number of tiles (2,400 tiles at 640x480 over 8 x 148 CTAs
+        // were a third round for the last 32)
+        const long cap = (long)sms * kTapCtas, rounds = (tiles + cap - 1) / cap;
+        const unsigned blocks = (unsigned)((tiles + rounds - 1) / rounds);
         count_launch();
-        k_conv2d_tc_tap<<<blocks, kTcM, smem, st>>>(a, PWp);
+        // FeatureNet c3 / c4 of the shipped checkpoint and the band net's layers
+        if (a.IC == 12 && a.OC == 12 && a.act == 1)
+            k_conv2d_tc_tap<12, 12, 1><<<blocks, kTcM, smem, st>>>(a, PWp);
+        else if (a.IC == 12 && a.OC == 12 && a.act == 0)
+            k_conv2d_tc_tap<12, 12, 0><<<blocks, kTcM, smem, st>>>(a, PWp);
+        else if (a.IC == 8 && a.OC == 16 && a.act == 1)
+            k_conv2d_tc_tap<8, 16, 1><<<blocks, kTcM, smem, st>>>(a, PWp);
+        else if (a.IC == 16 && a.OC == 16 && a.act == 1)
+            k_conv2d_tc_tap<16, 16, 1><<<blocks, kTcM, smem, st>>>(a, PWp);
+        else if (a.IC == 16 && a.OC == 2 && a.act == 0)
+            k_conv2d_tc_tap<16, 2, 0><<<blocks, kTcM, smem, st>>>(a, PWp);
+        else
+            k_conv2d_tc_tap<0, 0, -1><<<blocks, kTcM, smem, st>>>(a, PWp);
         SV_LAUNCH_CHECK();
         return SV_OK;
     }
