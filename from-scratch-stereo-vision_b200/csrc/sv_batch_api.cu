@@ -26,8 +26,7 @@ constexpr int kTileW = 32, kTileH = 8;   // census tile (k_census)
 int plan_batch(const sv_pair_desc *in, int n, const RefineCfg &c, int px_per_block, char *ws,
                BatchPlan *pl) {
     BatchPlan &P = *pl;
-    const int Kp = slot_width(c.K);
-    const size_t lt = c.l16 ? 2 : 1;
+    const size_t crow = cost_row_bytes(c.K), lrow = path_row_bytes(c.K, c.l16, true);
     Carver cv(ws);
     cv.take<DevFlags>(1);
     cv.take<int>(64);                                      // queue counter (+ padding)
@@ -76,9 +75,9 @@ int plan_batch(const sv_pair_desc *in, int n, const RefineCfg &c, int px_per_blo
         b.dr = cv.take<double>(N);
         b.cen0 = cv.take<uint64_t>(N);
         b.cen1 = cv.take<uint64_t>(N);
-        b.C0 = cv.take<uint8_t>(N * Kp);
-        b.C1 = cv.take<uint8_t>(N * Kp);
-        b.L = cv.take<uint8_t>(2 * (size_t)c.npaths * N * Kp * lt);
+        b.C0 = cv.take<uint8_t>(N * crow);
+        b.C1 = cv.take<uint8_t>(N * crow);
+        b.L = cv.take<uint8_t>(2 * (size_t)c.npaths * N * lrow);
         P.px_blk[i + 1] = P.px_blk[i] + (long long)((N + px_per_block - 1) / px_per_block);
         P.row_blk[i + 1] = P.row_blk[i] + d.H;
         P.tile_blk[i + 1] = P.tile_blk[i] + (long long)((d.W + kTileW - 1) / kTileW) *
@@ -89,21 +88,29 @@ int plan_batch(const sv_pair_desc *in, int n, const RefineCfg &c, int px_per_blo
     P.px_blocks = P.px_blk[n];
     P.rows = P.row_blk[n];
     P.tiles = P.tile_blk[n];
-    // SGM segments, longest scanlines first
+    // SGM segments: pair by pair, so that a pair's 8 directions read its costs
+    // from L2 rather than each from memory, the largest pair first (the last
+    // ones drain the queue), and within a pair the longest scanlines first
     struct Seg { int pair, vd, count, len; };
     std::vector<Seg> segs;
     segs.reserve(nseg);
-    for (int i = 0; i < n; ++i) {
+    std::vector<int> order(n);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        return (long long)in[a].W * in[a].H > (long long)in[b].W * in[b].H;
+    });
+    for (int i : order) {
         const int W = in[i].W, H = in[i].H;
+        const size_t first = segs.size();
         for (int v = 0; v < 2; ++v)
             for (int d = 0; d < c.npaths; ++d) {
                 const int cnt = d < 2 ? H : d < 4 ? W : W + H - 1;
                 const int len = d < 2 ? W : d < 4 ? H : std::min(W, H);
                 segs.push_back({i, v * 8 + d, cnt, len});
             }
+        std::stable_sort(segs.begin() + first, segs.end(),
+                         [](const Seg &a, const Seg &b) { return a.len > b.len; });
     }
-    std::stable_sort(segs.begin(), segs.end(),
-                     [](const Seg &a, const Seg &b) { return a.len > b.len; });
     P.seg_start.assign(nseg + 1, 0);
     P.seg_pair.resize(nseg);
     P.seg_vd.resize(nseg);

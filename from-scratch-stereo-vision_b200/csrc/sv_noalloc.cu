@@ -151,20 +151,34 @@ extern "C" int sv_refine_fullres_noalloc(const void *left, const void *right, in
     const int P1 = (int)p->P1, P2 = (int)p->P2;
     const int npaths = p->paths == 8 ? 8 : 4;
     const bool l16 = invalid + P2 > 255;
-    const size_t N = (size_t)W * H, NK = N * slot_width(K);
-    // layout: header | base | census left | census right | costs | path costs
-    const size_t o_base = 256;
-    const size_t o_cl = o_base + up256(N * 4);
-    const size_t o_cr = o_cl + up256(N * 8);
-    const size_t o_c = o_cr + up256(N * 8);
-    const size_t o_l = o_c + up256(NK);
-    const size_t need = o_l + up256(NK * npaths * (l16 ? 2 : 1));
+    const size_t N = (size_t)W * H;
+    // capacity, as documented: slots rounded up to one of these widths
+    static const int widths[] = {8, 16, 24, 32, 48, 64, 96, 128, 192, 256};
+    int width = 256;
+    for (int w : widths)
+        if (w >= K + 2) {
+            width = w;
+            break;
+        }
+    const size_t NK = N * width, lbytes = NK * npaths * (l16 ? 2 : 1);
+    // header | base | census left | census right | costs | path costs
+    const size_t need = 256 + up256(N * 4) + 2 * up256(N * 8) + up256(NK) + up256(lbytes);
     if (need > SV_NOALLOC_SCRATCH_BYTES) {
         set_error("%dx%d with K=%d needs %zu scratch bytes; the static scratch holds %u "
                   "(use sv_refine_fullres with a workspace)", W, H, K, need,
                   (unsigned)SV_NOALLOC_SCRATCH_BYTES);
         return SV_ERR_SHAPE;
     }
+    // layout: header | base | costs | path costs, the census maps (read by the
+    // band costs only) where the path costs are written after them: never
+    // more than the capacity above, since a row's slots are at most `width`, a
+    // cost row is at most 8 bytes longer than them and the two census maps of
+    // the sum above take 16 bytes per pixel
+    const size_t o_base = 256;
+    const size_t o_c = o_base + up256(N * 4);
+    const size_t o_l = o_c + up256(N * cost_row_bytes(K));
+    const size_t o_cl = o_l;
+    const size_t o_cr = o_cl + up256(N * 8);
     char *s = nullptr;
     int rc = scratch_address(reinterpret_cast<void **>(&s));
     if (rc) return rc;
@@ -181,9 +195,9 @@ extern "C" int sv_refine_fullres_noalloc(const void *left, const void *right, in
     if ((rc = launch_band_costs_slot(cl, cr, base, nullptr, W, H, p->R, invalid, C, nullptr, 1,
                                     st)))
         return rc;
-    if ((rc = launch_sgm_packed(C, nullptr, base, nullptr, W, H, K, P1, P2, L, l16, 1, npaths,
-                               st)))
+    if ((rc = launch_sgm_packed(C, nullptr, base, nullptr, W, H, K, P1, P2, L, l16, false, 1,
+                               npaths, st)))
         return rc;
-    return launch_wta_slot(L, l16, npaths, 1, W, H, p->R, base, nullptr, disp0, nullptr, p->uniq,
+    return launch_wta_slot(L, l16, false, npaths, 1, W, H, p->R, base, nullptr, disp0, nullptr, p->uniq,
                       out, nullptr, nullptr, st);
 }

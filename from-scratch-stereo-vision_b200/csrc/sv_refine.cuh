@@ -46,9 +46,12 @@ inline SgmTasks make_sgm_tasks(int W, int H, int nviews, int npaths, const int *
     return t;
 }
 
-// Bytes per pixel of the slot layout used by the fused refinement (K + 2
-// slots rounded up to a multiple of 8).
+// Slots per pixel of the fused refinement's layout (K + 2 rounded up to a
+// table width) and the bytes of a pixel's cost and path-cost rows (sv_sgm.cu).
+// pad: path-cost rows of the 24-slot layout padded to 32 bytes.
 int slot_width(int K);
+size_t cost_row_bytes(int K);
+size_t path_row_bytes(int K, bool l16, bool pad);
 
 // Validated refinement parameters (sv_api.cu).
 struct RefineCfg {
@@ -145,8 +148,8 @@ int launch_band_costs_slot(const uint64_t *cl, const uint64_t *cr, const int32_t
                            const uint8_t *rad0 = nullptr);
 int launch_sgm_packed(const uint8_t *C0, const uint8_t *C1, const int32_t *b0,
                       const int32_t *b1, int W, int H, int K, int P1, int P2, void *Lout,
-                      bool l16, int nviews, int npaths, cudaStream_t st);
-int launch_wta_slot(const void *L, bool l16, int npaths, int nviews, int W, int H, int R,
+                      bool l16, bool pad, int nviews, int npaths, cudaStream_t st);
+int launch_wta_slot(const void *L, bool l16, bool pad, int npaths, int nviews, int W, int H, int R,
                     const int32_t *b0, const int32_t *b1, const double *d00, const double *d01,
                     double uniq, double *out0, double *out1, double *conf0, cudaStream_t st);
 // base_l (optional): also k_base's band centres of dl, errors into flag.

@@ -37,17 +37,12 @@ _NP_CODE = {np.dtype(np.uint8): _lib.SV_U8, np.dtype(np.float32): _lib.SV_F32,
 
 
 def sgm_kernel_name(K: int = 21) -> str:
-    """Name of the single-pair SGM kernel the library runs for a band of K
-    (the library reads SV_SGM_KERNEL = group8 | group4 | thread once)."""
-    import os
-    Kp = next((k for k in (8, 16, 24, 32) if k >= K + 2), None)
-    if Kp is None:
-        return "k_sgm_packed"
-    v = os.environ.get("SV_SGM_KERNEL", "group8")
-    if v == "thread":
-        return "k_sgm_thread"
-    sl = 4 if v == "group4" else 8
-    return "k_sgm_group<%d slots x %d lanes>" % (sl, Kp // sl)
+    """Name of the SGM kernel the library runs for a band of K, with its split
+    of a scanline: registers of two 16-bit slots per lane x lanes."""
+    split = {8: (4, 1), 16: (4, 2), 24: (6, 2), 32: (8, 2), 48: (12, 2), 64: (16, 2),
+             96: (12, 4), 128: (16, 4), 160: (20, 4), 192: (24, 4), 224: (28, 4), 256: (32, 4)}
+    Kp = next((k for k in sorted(split) if k >= K + 2), 256)
+    return "k_sgm_scan<%d registers x %d lanes>" % split[Kp]
 
 
 def _device() -> torch.device:
