@@ -10,10 +10,9 @@
 //  * B (weights) is packed once at checkpoint upload into the canonical
 //    K-major, no-swizzle UMMA layout (8 x 16-byte core matrices, 128
 //    contiguous bytes each) and copied to shared memory once per CTA;
-//  * A (the im2col tile) is gathered by the CTA's 128 threads straight into
-//    that layout -- thread m owns output row m and writes 16-byte chunks of
-//    8 consecutive k -- and fenced into the async proxy; a shared table maps
-//    k to (channel, tap offsets);
+//  * A (the im2col tile) is gathered from an input patch in shared memory
+//    straight into that layout -- one output row per thread, in 16-byte
+//    chunks of 8 consecutive k -- and fenced into the async proxy;
 //  * one thread issues Kpad/16 tcgen05.mma (M=128, N=16, K=16) into a
 //    32-column tensor-memory accumulator and commits them to an mbarrier;
 //  * each warp reads its 32 accumulator rows back with tcgen05.ld
@@ -25,6 +24,7 @@
 #include <cuda_bf16.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "sv_common.cuh"
 #include "sv_tc.cuh"
@@ -82,17 +82,75 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity,
 
 }  // namespace
 
-// ktab[k] = {channel (-1: K padding), dz, dy, dx}: mode 0 input offsets
-// (input z = od + dz, y = oy * stride + dy, x = ox * stride + dx); mode 1
-// cost-volume offsets (d = od + dz, y = oy + dy, x = ox + dx).
-__global__ void __launch_bounds__(kTcM) k_conv_tc(TcConv a) {
+// 3x3x3 convolutions, stride 1, same padding: of a tensor (mode 0) or of the cost
+// volume of two feature maps, made here (mode 1).  A tile is one disparity of
+// 4 rows x 32 columns, and a CTA walks the disparities of one place in order: a
+// ring of three planes (every channel, 6 x 34 values with the halo) in shared
+// memory as BF16, the plane after next read from memory while the operand of this
+// one is built.  Operand A is the im2col tile, two threads per row, K halves
+// apart: element k is the ring's at a distance that k and the row's place give,
+// known at compile time for the shipped channel counts.  k stays channel-major, 16
+// to an MMA, so every output is the same sum as with any other tiling.
+// What bounds it is the copy into A, some 600 warp instructions a step and warp.
+// At 160 x 120 x 12, fetching each element of A from memory with its own bounds
+// tests took 381 us for 12 -> 6 channels and 113 for 6 -> 6; from the ring 41 and 26
+// (45 with two-byte reads, 58 when a plane was made as it was read).
+constexpr int kC3Threads = 256, kC3Pitch = 36, kC3Rows = 6, kC3W = 32, kC3H = 4;
+constexpr int kC3Pairs = 17;            // column pairs of a plane row
+
+// Chunks [G0, G1) of 8 elements of one row of A; b0, b1, b2 are the row's place
+// in the ring's planes of taps kd = 0, 1, 2, rounded down to a word.  Six elements
+// (two rows of taps, three words of A) come from four words of the ring; odd
+// columns pick the other halves (s0, s1, s2).
+template <int IC, int G0, int G1>
+__device__ __forceinline__ void c3_gather(const unsigned char *b0, const unsigned char *b1,
+                                          const unsigned char *b2, unsigned s0, unsigned s1,
+                                          unsigned s2, unsigned char *row) {
+    static_assert(G0 % 3 == 0, "whole row pairs");
+    constexpr int NW = (G1 - G0) * 4;                      // words of A
+    uint32_t w[4];
+#pragma unroll
+    for (int p = 0; p < (NW + 2) / 3; ++p) {
+        uint32_t q[2][2] = {};
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int t = G0 * 8 / 3 + 2 * p + u;          // row of taps (c, kd, ky)
+            if (t >= IC * 9) continue;
+            const int c = t / 9, kd = t % 9 / 3, ky = t % 3;
+            const unsigned char *b = kd == 0 ? b0 : kd == 1 ? b1 : b2;
+            const uint32_t *r = reinterpret_cast<const uint32_t *>(
+                b + (c * kC3Rows + ky) * kC3Pitch * 2);
+            q[u][0] = r[0];
+            q[u][1] = r[1];
+        }
+        const uint32_t o[3] = {__byte_perm(q[0][0], q[0][1], s0), __byte_perm(q[0][1], q[1][0], s1),
+                               __byte_perm(q[1][0], q[1][1], s2)};
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            const int n = 3 * p + e;
+            if (n >= NW) continue;
+            w[n % 4] = o[e];
+            if (n % 4 == 3)
+                *reinterpret_cast<uint4 *>(row + (size_t)(G0 + n / 4) * (kTcM / 8) * 128) =
+                    make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    }
+}
+
+// ICT: the channel count, 0 to read it from the arguments; MODE: a.mode
+template <int ICT, int MODE>
+__global__ void __launch_bounds__(kC3Threads) k_conv3d_tc(TcConv a, int per_cta) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_slot;
     __shared__ int failed;
-    __shared__ int4 ktab[kTcMaxK];
+    __shared__ int ktab[ICT > 0 ? 1 : kTcMaxK];    // ring offset of k without its plane, and kd
+    const int IC = ICT > 0 ? ICT : a.IC;
+    const int Kpad = ICT > 0 ? (ICT * 27 + 15) / 16 * 16 : a.Kpad;
     unsigned char *sA = smem;                                   // 128 x Kpad BF16
-    unsigned char *sB = smem + (size_t)a.Kpad * kTcM * 2;        // 16 x Kpad BF16
+    unsigned char *sB = smem + (size_t)Kpad * kTcM * 2;          // 16 x Kpad BF16
+    __nv_bfloat16 *ring = reinterpret_cast<__nv_bfloat16 *>(sB + (size_t)Kpad * kTcN * 2);
+    const int psize = IC * kC3Rows * kC3Pitch;                  // one plane
     const int tid = threadIdx.x, warp = tid >> 5;
 
     if (warp == 0) {
@@ -102,23 +160,12 @@ __global__ void __launch_bounds__(kTcM) k_conv_tc(TcConv a) {
     }
     const uint4 *wsrc = reinterpret_cast<const uint4 *>(a.wB);
     uint4 *wdst = reinterpret_cast<uint4 *>(sB);
-    for (int i = tid; i < a.Kpad * kTcN * 2 / 16; i += kTcM) wdst[i] = __ldg(wsrc + i);
-    const int taps = a.nd == 3 ? 27 : 9;
-    for (int k = tid; k < a.Kpad; k += kTcM) {
-        int4 e = make_int4(-1, 0, 0, 0);
-        if (k < a.K) {
-            const int c = k / taps;
-            int t = k - c * taps;
-            const int kd = a.nd == 3 ? t / 9 : 1;
-            if (a.nd == 3) t -= kd * 9;
-            const int ky = t / 3, kx = t - (t / 3) * 3;
-            if (a.mode == 0)
-                e = make_int4(c, kd - 1, ky * a.dil - a.pad, kx * a.dil - a.pad);
-            else
-                e = make_int4(c, kd - 1, ky - 1, kx - 1);
+    for (int i = tid; i < Kpad * kTcN * 2 / 16; i += kC3Threads) wdst[i] = __ldg(wsrc + i);
+    if constexpr (ICT == 0)
+        for (int k = tid; k < Kpad; k += kC3Threads) {
+            const int c = k / 27, t = k - c * 27, kd = t / 9, ky = t % 9 / 3, kx = t % 3;
+            ktab[k] = k < a.K ? ((c * kC3Rows + ky) * kC3Pitch + kx) * 4 + kd : -1;
         }
-        ktab[k] = e;
-    }
     if (tid == 0) {
         mbar_init(&mbar, 1);
         failed = 0;
@@ -129,60 +176,131 @@ __global__ void __launch_bounds__(kTcM) k_conv_tc(TcConv a) {
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = tmem_slot;
 
-    const long M = (long)a.OD * a.OH * a.OW;
-    const long tiles_img = (M + kTcM - 1) / kTcM;
-    const int nb = a.nb > 0 ? a.nb : 1;
-    const long tiles = tiles_img * (a.mode == 0 ? a.nimg : 1) * nb;
-    const int ohw = a.OH * a.OW;
-    const long plane = (long)a.D * a.H * a.W;     // one input channel (mode 0)
-    const long fplane = (long)a.H * a.W;          // one feature channel (mode 1)
-    unsigned phase = 0;
-    for (long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int item = (int)(tile / tiles_img);
-        const int img = item / nb, bi = item - img * nb;
-        const long mi = (tile - item * tiles_img) * kTcM + tid;
-        const bool row_ok = mi < M;
-        int od = 0, oy = 0, ox = 0;
-        if (row_ok) {
-            od = (int)(mi / ohw);
-            const int r = (int)(mi - (long)od * ohw);
-            oy = r / a.OW;
-            ox = r - oy * a.OW;
-        }
-        // ---- gather this thread's im2col row, 8 k at a time
-        const float *x0 = (img ? a.x[1] : a.x[0]) + bi * a.xs, *x1 = a.x[1] + bi * a.xs;
-        const int by = a.mode == 0 ? oy * a.stride : oy, bx = a.mode == 0 ? ox * a.stride : ox;
-        for (int kg = 0; kg < a.Kpad / 8; ++kg) {
-            __align__(16) __nv_bfloat16 v[8];
+    const int D = a.D, H = a.H, W = a.W;
+    const int tx_n = (W + kC3W - 1) / kC3W, ty_n = (H + kC3H - 1) / kC3H;
+    const int places = tx_n * ty_n, nb = a.nb > 0 ? a.nb : 1;
+    const long steps = (long)places * (MODE == 0 ? a.nimg : 1) * nb * D;
+    const long hw = (long)H * W, M = hw * D;
+    const int m = tid & 127, my = m >> 5, mx = m & 31;
+
+    // A plane's column pairs, up to kU per thread, their places fixed while the CTA
+    // stays at one place: off the pair's offset, at = its column (+ 1) and whether
+    // either column is inside.  A plane is read into registers, without a branch or
+    // a use before the operand is built, and rounded into the ring after.
+    constexpr int kU = ((ICT > 0 ? ICT : 16) * kC3Rows * kC3Pairs + kC3Threads - 1) / kC3Threads;
+    const int npairs = IC * kC3Rows * kC3Pairs;
+    float2 v[kU], left[MODE == 1 ? kU : 1];
+    std::conditional_t<MODE == 0, long, int> off[kU];     // a volume may pass 2^31 values
+    int at[kU];
+    const float *x0 = nullptr, *x1 = nullptr;
+    int ty0 = 0, tx0 = 0;
+    auto places_of = [&]() {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int4 e = ktab[kg * 8 + j];
-                float f = 0.f;
-                const int z = od + e.y, yy = by + e.z, xx = bx + e.w;
-                if (row_ok && e.x >= 0 && z >= 0 && z < a.D && yy >= 0 && yy < a.H && xx >= 0 &&
-                    xx < a.W) {
-                    if (a.mode == 0) {
-                        f = __ldg(x0 + e.x * plane + ((long)z * a.H + yy) * a.W + xx);
-                    } else if (xx < z) {
-                        f = 2.0f;
-                    } else {
-                        const long o = e.x * fplane + (long)yy * a.W + xx;
-                        f = fabsf(__ldg(x0 + o) - __ldg(x1 + o - z));
-                    }
-                }
-                v[j] = __float2bfloat16_rn(f);
+        for (int u = 0; u < kU; ++u) {
+            const int i = tid + u * kC3Threads;
+            const int r = i / kC3Pairs, xx = tx0 - 1 + 2 * (i - r * kC3Pairs);
+            const int c = r / kC3Rows, yy = ty0 - 1 + r - c * kC3Rows;
+            const bool row = i < npairs && yy >= 0 && yy < H;
+            off[u] = c * (MODE == 0 ? D * hw : hw) + (long)yy * W + xx;
+            at[u] = (xx + 1) * 4 + (row && xx >= 0 && xx < W ? 1 : 0) + (row && xx + 1 < W ? 2 : 0);
+            if constexpr (MODE == 1) {
+                left[u].x = at[u] & 1 ? __ldg(x0 + off[u]) : 0.f;
+                left[u].y = at[u] & 2 ? __ldg(x0 + off[u] + 1) : 0.f;
             }
-            *reinterpret_cast<uint4 *>(sA + (size_t)(kg * (kTcM / 8) + (tid >> 3)) * 128 +
-                                       (tid & 7) * 16) = *reinterpret_cast<const uint4 *>(v);
+        }
+    };
+    auto fetch = [&](int z) {
+        const bool in = z >= 0 && z < D;
+        const float *p = MODE == 0 ? x0 + (in ? z * hw : 0) : x1 - z;
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int xx = (at[u] >> 2) - 1;
+            const bool on0 = in && (at[u] & 1) && (MODE == 0 || xx >= z);
+            const bool on1 = in && (at[u] & 2) && (MODE == 0 || xx + 1 >= z);
+            v[u].x = on0 ? __ldg(p + off[u]) : 0.f;
+            v[u].y = on1 ? __ldg(p + off[u] + 1) : 0.f;
+        }
+    };
+    auto put = [&](int z) {
+        const bool in = z >= 0 && z < D;
+        __nv_bfloat16 *dst = ring + (z + 3) % 3 * psize;
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int i = tid + u * kC3Threads;
+            if (i >= npairs) break;
+            const int r = i / kC3Pairs, j = i - r * kC3Pairs;
+            float2 f = v[u];
+            if constexpr (MODE == 1) {
+                const int xx = (at[u] >> 2) - 1;
+                f.x = !in || !(at[u] & 1) ? 0.f : xx < z ? 2.0f : fabsf(left[u].x - f.x);
+                f.y = !in || !(at[u] & 2) ? 0.f : xx + 1 < z ? 2.0f : fabsf(left[u].y - f.y);
+            }
+            *reinterpret_cast<__nv_bfloat162 *>(dst + r * kC3Pitch + 2 * j) =
+                __floats2bfloat162_rn(f.x, f.y);
+        }
+    };
+
+    unsigned phase = 0;
+    const long s0 = (long)blockIdx.x * per_cta, s1 = min(s0 + per_cta, steps);
+    int item = -1, img = 0, bi = 0;
+    for (long s = s0; s < s1; ++s) {
+        const long place = s / D;
+        const int d = (int)(s - place * D);
+        if (s == s0 || d == 0) {                           // a new place: its first planes
+            item = (int)(place / places);
+            const int pl = (int)(place - (long)item * places);
+            img = item / nb;
+            bi = item - img * nb;
+            ty0 = pl / tx_n * kC3H;
+            tx0 = pl % tx_n * kC3W;
+            x0 = (img ? a.x[1] : a.x[0]) + bi * a.xs;
+            x1 = a.x[1] + bi * a.xs;
+            places_of();
+            for (int z = d - 1; z <= d + 1; ++z) {
+                fetch(z);
+                put(z);
+            }
+            __syncthreads();
+        }
+        const bool more = s + 1 < s1 && d + 1 < D;
+        if (more) fetch(d + 2);
+        {
+            const __nv_bfloat16 *b = ring + my * kC3Pitch + mx;
+            const __nv_bfloat16 *b0 = b + (d + 2) % 3 * psize, *b1 = b + d % 3 * psize,
+                                *b2 = b + (d + 1) % 3 * psize;
+            unsigned char *row = sA + (m >> 3) * 128 + (m & 7) * 16;
+            if constexpr (ICT > 0) {
+                constexpr int G = (ICT * 27 + 15) / 16 * 2, G2 = (G / 2 + 1) / 3 * 3;
+                const unsigned odd = mx & 1;
+                const unsigned e0 = odd ? 0x5432 : 0x3210, e1 = odd ? 0x7632 : 0x5410,
+                               e2 = odd ? 0x7654 : 0x5432;
+                const unsigned char *c0 = reinterpret_cast<const unsigned char *>(b0 - odd),
+                                    *c1 = reinterpret_cast<const unsigned char *>(b1 - odd),
+                                    *c2 = reinterpret_cast<const unsigned char *>(b2 - odd);
+                if (tid < kTcM) c3_gather<ICT, 0, G2>(c0, c1, c2, e0, e1, e2, row);
+                else c3_gather<ICT, G2, G>(c0, c1, c2, e0, e1, e2, row);
+            } else {
+                for (int g = tid >> 7; g < Kpad / 8; g += 2) {
+                    __align__(16) __nv_bfloat16 e[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const int t = ktab[g * 8 + j], kd = t & 3;
+                        const __nv_bfloat16 *p = kd == 0 ? b0 : kd == 1 ? b1 : b2;
+                        e[j] = t >= 0 ? p[t >> 2] : __float2bfloat16_rn(0.f);
+                    }
+                    *reinterpret_cast<uint4 *>(row + (size_t)g * (kTcM / 8) * 128) =
+                        *reinterpret_cast<const uint4 *>(e);
+                }
+            }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;");
         if (tid == 0 && !failed) {
-            const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
-            for (int ks = 0; ks < a.Kpad / 16; ++ks) {
+            const uint32_t a0 = smem_u32(sA), w0 = smem_u32(sB);
+            for (int ks = 0; ks < Kpad / 16; ++ks) {
                 const uint64_t da = umma_desc(a0 + ks * 2 * (kTcM / 8) * 128, (kTcM / 8) * 128, 128);
-                const uint64_t db = umma_desc(b0 + ks * 2 * (kTcN / 8) * 128, (kTcN / 8) * 128, 128);
+                const uint64_t db = umma_desc(w0 + ks * 2 * (kTcN / 8) * 128, (kTcN / 8) * 128, 128);
                 asm volatile(
                     "{\n\t.reg .pred p;\n\t"
                     "setp.ne.b32 p, %4, 0;\n\t"
@@ -194,6 +312,7 @@ __global__ void __launch_bounds__(kTcM) k_conv_tc(TcConv a) {
                 ::"r"(smem_u32(&mbar))
                 : "memory");
         }
+        if (more) put(d + 2);                              // over plane d - 1, read by all
         // ---- wait for the accumulator (bounded), then the epilogue
         if (!failed && !mbar_wait(&mbar, phase)) {
             failed = 1;
@@ -203,26 +322,30 @@ __global__ void __launch_bounds__(kTcM) k_conv_tc(TcConv a) {
         __syncthreads();
         if (failed) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
-        uint32_t r[16];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-              "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-              "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(tmem + ((uint32_t)(warp * 32) << 16)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (row_ok) {
-            float *y = (img ? a.y[1] : a.y[0]) + bi * a.ys;
-            const float *aux = a.aux ? a.aux + bi * a.ys : nullptr;
+        if (warp < 4) {
+            uint32_t r[16];
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                  "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+                  "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                : "r"(tmem + ((uint32_t)(warp * 32) << 16)));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            const int oy = ty0 + my, ox = tx0 + mx;
+            if (oy < H && ox < W) {
+                const long mi = (long)d * hw + (long)oy * W + ox;
+                float *y = (img ? a.y[1] : a.y[0]) + bi * a.ys;
+                const float *aux = a.aux ? a.aux + bi * a.ys : nullptr;
 #pragma unroll
-            for (int n = 0; n < kTcN; ++n) {
-                if (n < a.OC) {
-                    float v = __uint_as_float(r[n]);
-                    if (a.bias) v += __ldg(a.bias + n);
-                    if (a.act == 1) v = v > 0.f ? v : v * 0.2f;
-                    if (a.act == 2) v = __ldg(aux + (long)n * M + mi) > 0.f ? v : v * 0.2f;
-                    y[(long)n * M + mi] = v;
+                for (int n = 0; n < kTcN; ++n) {
+                    if (n < a.OC) {
+                        float f = __uint_as_float(r[n]);
+                        if (a.bias) f += __ldg(a.bias + n);
+                        if (a.act == 1) f = f > 0.f ? f : f * 0.2f;
+                        if (a.act == 2) f = __ldg(aux + (long)n * M + mi) > 0.f ? f : f * 0.2f;
+                        y[(long)n * M + mi] = f;
+                    }
                 }
             }
         }
@@ -256,7 +379,7 @@ void tc_pack_weights(const double *w, int OC, int K, uint16_t *out) {
 // shared memory as BF16 by whole warps reading rows (coalesced, all loads
 // independent), and the im2col operand A is then built from shared memory:
 // element (m, k) is patch[ktab[k] + base(m)].  The MMA issue, the bounded
-// wait and the epilogue are those of k_conv_tc.
+// wait and the epilogue are those of k_conv3d_tc.
 constexpr int kT2W = 32, kT2H = 4;
 constexpr int kT2Cols = 3;              // patch columns per lane: PW <= 96
 
@@ -599,7 +722,7 @@ __global__ void __launch_bounds__(kTcM, kTapCtas) k_conv2d_tc_tap(TcConv a, int 
 // dynamic shared-memory limit (raised to kTcSmemMax; every launch checks
 // its own size against it).  Launches stay free of attribute calls.
 constexpr size_t kTcSmemMax = 200 * 1024;
-enum { kKConv = 0, kKConv2d = 1, kKWgrad = 2, kKConv2dTap = 3, kKCount = 4 };
+enum { kKConv3d, kKConv3dV, kKConv3d12, kKConv3d6, kKConv2d, kKWgrad, kKConv2dTap, kKCount };
 
 static int tc_setup(int which, const void *fn, int *sms) {
     static std::mutex mu;
@@ -745,18 +868,31 @@ int launch_conv_tc(const TcConv &a, cudaStream_t st) {
         }
         return launch_conv2d_tc(a, st);
     }
-    const size_t smem = (size_t)a.Kpad * (kTcM + kTcN) * 2;
-    const long M = (long)a.OD * a.OH * a.OW;
-    if (M == 0) return SV_OK;
-    const long tiles =
-        (M + kTcM - 1) / kTcM * (a.mode == 0 ? a.nimg : 1) * (a.nb > 0 ? a.nb : 1);
+    if (a.nd != 3 || a.K != a.IC * 27 || a.stride != 1 || a.pad != 1 || a.dil != 1 ||
+        a.OD != a.D || a.OH != a.H || a.OW != a.W) {
+        set_error("tensor-core conv3d: inconsistent shape");
+        return SV_ERR_PARAM;
+    }
+    const size_t smem = (size_t)a.Kpad * (kTcM + kTcN) * 2 +
+                        (size_t)3 * a.IC * kC3Rows * kC3Pitch * 2;
+    const long steps = (long)((a.W + kC3W - 1) / kC3W) * ((a.H + kC3H - 1) / kC3H) * a.D *
+                       (a.mode == 0 ? a.nimg : 1) * (a.nb > 0 ? a.nb : 1);
+    if (steps == 0) return SV_OK;
     int sms = 148;
-    const int rc = tc_setup(kKConv, (const void *)k_conv_tc, &sms);
+    // the shipped checkpoint's cost filter (12, then 6 channels), and any other
+    void (*f)(TcConv, int) = a.mode == 1 ? k_conv3d_tc<0, 1> : k_conv3d_tc<0, 0>;
+    int which = a.mode == 1 ? kKConv3dV : kKConv3d;
+    if (a.mode == 1 && a.IC == 12) f = k_conv3d_tc<12, 1>, which = kKConv3d12;
+    if (a.mode == 0 && a.IC == 6) f = k_conv3d_tc<6, 0>, which = kKConv3d6;
+    const int rc = tc_setup(which, (const void *)f, &sms);
     if (rc) return rc;
-    const long cap = (long)sms * tc_ctas_per_sm(smem);
-    const unsigned blocks = (unsigned)(tiles < cap ? tiles : cap);
+    // consecutive steps (disparities of a place) to a CTA, the same number to each
+    // (two CTAs of 12 channels fill the SM's 228 KB)
+    const long cap = (long)sms * (smem + 2 * 1024 <= 114 * 1024 ? 2 : 1);
+    const int per = (int)((steps + cap - 1) / cap);
+    const unsigned blocks = (unsigned)((steps + per - 1) / per);
     count_launch();
-    k_conv_tc<<<blocks, kTcM, smem, st>>>(a);
+    f<<<blocks, kC3Threads, smem, st>>>(a, per);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
