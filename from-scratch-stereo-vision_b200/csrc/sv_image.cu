@@ -137,16 +137,63 @@ const int kDistExtra[30] = {0, 0, 0, 0, 1, 1, 2, 2, 3, 3, 4, 4, 5, 5, 6,
                             6, 7, 7, 8, 8, 9, 9, 10, 10, 11, 11, 12, 12, 13, 13};
 const int kClOrder[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11, 4, 12, 3, 13, 2, 14, 1, 15};
 
+// Tables of the fast loop, over the next kLitBits / kDistBits bits.  An entry says
+// all that a symbol needs: bits 0-3 the code's length, 4-7 the extra bits', 8-9 the
+// kind, 16-31 the literal or the base of the length or distance.  A code longer
+// than the table, an unused one and the end of the block have the kind kOther.
+constexpr int kLitBits = 12, kDistBits = 11;
+constexpr uint32_t kLiteral = 0u << 8, kCopy = 1u << 8, kOther = 2u << 8;
+struct FastTables {
+    uint32_t lit[1 << kLitBits], dist[1 << kDistBits];
+};
+
+// `bits`-bit table of code c (its lengths len[0, n)); entry(s) is symbol s's
+template <typename E>
+void fast_table(const Code &c, const uint8_t *len, int n, int bits, uint32_t *t, E entry) {
+    int next[16], code = 0;
+    next[0] = 0;
+    for (int l = 1; l < 16; ++l) {
+        code = (code + c.count[l - 1]) << 1;
+        next[l] = code;
+    }
+    for (int i = 0; i < 1 << bits; ++i) t[i] = kOther;
+    for (int s = 0; s < n; ++s) {
+        const int l = len[s];
+        if (!l) continue;
+        const int cd = next[l]++;
+        if (l > bits) continue;
+        int rev = 0;
+        for (int k = 0; k < l; ++k) rev |= ((cd >> k) & 1) << (l - 1 - k);
+        const uint32_t e = entry(s) | (uint32_t)l;
+        for (int i = rev; i < 1 << bits; i += 1 << l) t[i] = e;
+    }
+}
+
+void build_fast(FastTables &f, const Code &lit, const uint8_t *llen, int nl, const Code &dist,
+                const uint8_t *dlen, int nd) {
+    fast_table(lit, llen, nl, kLitBits, f.lit, [](int s) -> uint32_t {
+        if (s < 256) return kLiteral | (uint32_t)s << 16;
+        if (s == 256 || s > 285) return kOther;
+        return kCopy | (uint32_t)kLenBase[s - 257] << 16 | (uint32_t)kLenExtra[s - 257] << 4;
+    });
+    fast_table(dist, dlen, nd, kDistBits, f.dist, [](int s) -> uint32_t {
+        if (s > 29) return kOther;
+        return kCopy | (uint32_t)kDistBase[s] << 16 | (uint32_t)kDistExtra[s] << 4;
+    });
+}
+
 // The fixed codes of RFC 1951 section 3.2.6, built once (thread-safe
 // static initialisation).
 struct FixedCodes {
     Code lit, dist;
+    FastTables fast;
     FixedCodes() {
         uint8_t l[288], d[30];
         for (int s = 0; s < 288; ++s) l[s] = s < 144 ? 8 : s < 256 ? 9 : s < 280 ? 7 : 8;
         for (int s = 0; s < 30; ++s) d[s] = 5;
         build(lit, l, 288);
         build(dist, d, 30);
+        build_fast(fast, lit, l, 288, dist, d, 30);
     }
 };
 const FixedCodes &fixed_codes() {
@@ -166,11 +213,90 @@ struct Out {
     }
 };
 
+// The symbols of a Huffman block as long as nothing special comes up: whole words
+// of input left, room in the output for the longest copy and the 8 bytes that it
+// may write past its end, codes that the tables hold, distances inside the output.
+// Stops before any other symbol, which codes() then decodes (or rejects).  What
+// bounds it is the chain from one symbol's length to the next one's bits and the
+// branch between literals and copies; so a word of input serves three literals, a
+// copy's length and distance each take one table entry, and copies go 8 bytes at a
+// time.  A 450 x 375 RGB image of 260,000 symbols inflates in 2.1 ms (3.0 symbol by
+// symbol through codes(); 3.1 with one branch-free path for literals and copies).
+void codes_fast(BitIn &b, const FastTables &f, Out &out) {
+    uint64_t buf = b.buf;
+    unsigned cnt = (unsigned)b.cnt;
+    const uint8_t *p = b.p + b.pos, *const pend = b.p + b.n;
+    uint8_t *const base = out.v.data(), *o = base + out.size, *const oend = base + out.v.size();
+    constexpr uint32_t LM = (1u << kLitBits) - 1, DM = (1u << kDistBits) - 1;
+    while (pend - p >= 8 && oend - o >= 3 + 258 + 8) {
+        uint64_t w;
+        memcpy(&w, p, 8);
+        buf |= w << cnt;
+        p += (63 - cnt) >> 3;
+        cnt |= 56;
+        uint32_t e = f.lit[buf & LM];
+        if ((e & 0x300) == kLiteral) {
+            buf >>= e & 15;
+            cnt -= e & 15;
+            *o++ = (uint8_t)(e >> 16);
+            e = f.lit[buf & LM];
+            if ((e & 0x300) == kLiteral) {
+                buf >>= e & 15;
+                cnt -= e & 15;
+                *o++ = (uint8_t)(e >> 16);
+                e = f.lit[buf & LM];
+                if ((e & 0x300) == kLiteral) {
+                    buf >>= e & 15;
+                    cnt -= e & 15;
+                    *o++ = (uint8_t)(e >> 16);
+                    continue;
+                }
+            }
+            if (e & kOther) break;
+            if (pend - p < 8) break;
+            memcpy(&w, p, 8);
+            buf |= w << cnt;
+            p += (63 - cnt) >> 3;
+            cnt |= 56;
+        }
+        if (e & kOther) break;
+        // length (12 + 5 bits at most), distance (11 + 13): 41 of at least 56 bits
+        const unsigned lc = e & 15, le = (e >> 4) & 15;
+        const uint64_t b1 = buf >> lc, b2 = b1 >> le;
+        const uint32_t ed = f.dist[b2 & DM];
+        if (ed & kOther) break;
+        const unsigned dc = ed & 15, de = (ed >> 4) & 15;
+        const unsigned len = (e >> 16) + (unsigned)(b1 & ((1u << le) - 1));
+        const size_t d = (ed >> 16) + (size_t)((b2 >> dc) & ((1u << de) - 1));
+        if (d > (size_t)(o - base)) break;
+        buf = b2 >> (dc + de);
+        cnt -= lc + le + dc + de;
+        const uint8_t *q = o - d;
+        uint8_t *const end = o + len;
+        if (d >= 8) {
+            do {
+                memcpy(&w, q, 8);
+                memcpy(o, &w, 8);
+                q += 8;
+                o += 8;
+            } while (o < end);
+        } else {
+            do *o++ = *q++; while (o < end);
+        }
+        o = end;
+    }
+    // the buffer's bytes past cnt are read again: drop them
+    b.buf = cnt < 64 ? buf & ((1ull << cnt) - 1) : buf;
+    b.cnt = (int)cnt;
+    b.pos = (size_t)(p - b.p);
+    out.size = (size_t)(o - base);
+}
+
 // The symbols of one Huffman block.  The bit buffer and the output cursor
 // live in locals for the loop (stores of output bytes may alias anything
 // reachable through a pointer); the slow bit-at-a-time decode and buffer
 // growth write them back first.
-bool codes(BitIn &b, const Code &lit, const Code &dist, Out &out) {
+bool codes(BitIn &b, const Code &lit, const Code &dist, const FastTables &fast, Out &out) {
     uint64_t buf = b.buf;
     int cnt = b.cnt;
     size_t pos = b.pos, size = out.size;
@@ -219,6 +345,13 @@ bool codes(BitIn &b, const Code &lit, const Code &dist, Out &out) {
         return v;
     };
     for (;;) {
+        if (pos + 8 <= n && size + 3 + 258 + 8 <= cap) {    // up to the next special symbol
+            sync_out();
+            out.size = size;
+            codes_fast(b, fast, out);
+            sync_in();
+            size = out.size;
+        }
         const int s = sym(lit);
         if (s < 0) break;
         if (size + 258 > cap) {                 // room for the longest match, or
@@ -256,6 +389,7 @@ bool codes(BitIn &b, const Code &lit, const Code &dist, Out &out) {
 
 bool inflate_raw(const uint8_t *p, size_t n, Out &out) {
     BitIn b{p, n, 0};
+    FastTables fast;
     for (;;) {
         const uint32_t last = b.get(1), type = b.get(2);
         if (b.fail) return false;
@@ -272,7 +406,8 @@ bool inflate_raw(const uint8_t *p, size_t n, Out &out) {
             out.size += rest;
             b.pos += rest;
         } else if (type == 1) {
-            if (!codes(b, fixed_codes().lit, fixed_codes().dist, out)) return false;
+            if (!codes(b, fixed_codes().lit, fixed_codes().dist, fixed_codes().fast, out))
+                return false;
         } else if (type == 2) {
             const int nlen = (int)b.get(5) + 257, ndist = (int)b.get(5) + 1,
                       ncode = (int)b.get(4) + 4;
@@ -308,7 +443,8 @@ bool inflate_raw(const uint8_t *p, size_t n, Out &out) {
             }
             Code lit, dist;
             if (!build(lit, lens, nlen) || !build(dist, lens + nlen, ndist)) return false;
-            if (!codes(b, lit, dist, out)) return false;
+            build_fast(fast, lit, lens, nlen, dist, lens + nlen, ndist);
+            if (!codes(b, lit, dist, fast, out)) return false;
         } else {
             return false;
         }
