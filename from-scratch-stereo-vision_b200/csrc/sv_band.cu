@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(32 * kFeatDG)
     k_band_features(const uint64_t *__restrict__ cl, const uint64_t *__restrict__ cr,
                     const double *__restrict__ d0, const T *__restrict__ left, int W, int H,
                     int dmax, float *__restrict__ feat, int *__restrict__ err) {
+    pdl_sync();
     __shared__ unsigned s_best[kFeatRows][32];
     __shared__ int s_band[kFeatRows][32];
     __shared__ int s_cd0[kFeatRows][32];
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(256)
     k_band_loss(const float *__restrict__ O, const float *__restrict__ target,
                 const uint8_t *__restrict__ mask, long HW, long total, float inv_n,
                 float *__restrict__ gO, double *__restrict__ loss) {
+    pdl_sync();
     double acc = 0.0;
     for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < total;
          q += (long)gridDim.x * blockDim.x) {
@@ -252,6 +254,7 @@ __global__ void __launch_bounds__(256)
 __global__ void k_band_adam(float *__restrict__ p, const float *__restrict__ g,
                             float *__restrict__ m, float *__restrict__ v, long n, float lr,
                             float b1, float b2, float eps, float clip, float c1, float c2) {
+    pdl_sync();
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gi = fminf(fmaxf(g[i], -clip), clip);
@@ -266,6 +269,7 @@ __global__ void k_band_adam(float *__restrict__ p, const float *__restrict__ g,
 __global__ void k_band_targets(const double *__restrict__ label, const uint8_t *__restrict__ st,
                                const double *__restrict__ d0, long n, double shift_max,
                                float *__restrict__ target, uint8_t *__restrict__ mask) {
+    pdl_sync();
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i >= n) return;
     double t = __dsub_rn(label[i], d0[i]);
@@ -278,6 +282,7 @@ __global__ void k_band_apply(const float *__restrict__ out, const double *__rest
                              long HW, double b_thr, double rad_k, int rad_min, int R,
                              double shift_max, double *__restrict__ centre,
                              uint8_t *__restrict__ rad) {
+    pdl_sync();
     const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (p >= HW) return;
     double rho = __dadd_rn((double)out[HW + p], 1.0);
@@ -395,7 +400,7 @@ int band_grads_impl(sv_band *b, const float *feat, const float *target, const ui
     int rc = band_forward_impl(b, feat, nb, W, H, w.O, w, st);
     if (rc) return rc;
     count_launch();
-    k_band_loss<<<grid_for(total, 256, 148 * 8), 256, 0, st>>>(
+    pdl(k_band_loss, grid_for(total, 256, 148 * 8), 256, 0, st)(
         w.O, target, mask, HW, total, (float)(1.0 / (double)total), w.gO, w.loss);
     SV_LAUNCH_CHECK();
     // layer l's output gradient (w.r.t. its pre-activation) is gcur
@@ -453,6 +458,7 @@ namespace sv {
 // is below tau.  The learned band refines around it.
 __global__ void k_band_rule(const float *__restrict__ feat, const double *__restrict__ d0,
                             long N, double tau, double *__restrict__ centre) {
+    pdl_sync();
     for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < N;
          p += (long)gridDim.x * blockDim.x) {
         const double f1 = (double)feat[N + p], f2 = (double)feat[2 * N + p];
@@ -464,6 +470,7 @@ __global__ void k_band_rule(const float *__restrict__ feat, const double *__rest
 // and its peak probability - 0.5, per pixel of the last pass.
 __global__ void k_band_conf(const double *__restrict__ spread, const double *__restrict__ pmax,
                             long N, float *__restrict__ feat) {
+    pdl_sync();
     for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < N;
          p += (long)gridDim.x * blockDim.x) {
         feat[6 * N + p] = (float)__ddiv_rn(spread[p], 16.0);
@@ -560,7 +567,7 @@ int sv_band_rule_centre(const float *feat, const double *disp0, int W, int H, do
     if (!std::isfinite(tau)) { set_error("tau must be finite"); return SV_ERR_PARAM; }
     const long N = (long)W * H;
     count_launch();
-    k_band_rule<<<grid_for(N, 256), 256, 0, (cudaStream_t)stream>>>(feat, disp0, N, tau, centre);
+    pdl(k_band_rule, grid_for(N, 256), 256, 0, (cudaStream_t)stream)(feat, disp0, N, tau, centre);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -571,7 +578,7 @@ int sv_band_conf_features(const double *spread, const double *pmax, int W, int H
     if (W < 1 || H < 1) { set_error("bad shape %dx%d", W, H); return SV_ERR_SHAPE; }
     const long N = (long)W * H;
     count_launch();
-    k_band_conf<<<grid_for(N, 256), 256, 0, (cudaStream_t)stream>>>(spread, pmax, N, feat);
+    pdl(k_band_conf, grid_for(N, 256), 256, 0, (cudaStream_t)stream)(spread, pmax, N, feat);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -602,13 +609,13 @@ int sv_band_features(const void *left, const void *right, int dtype, const doubl
     const dim3 grd((W + 31) / 32, (H + kFeatRows - 1) / kFeatRows);
     count_launch();
     if (dtype == SV_U8)
-        k_band_features<uint8_t><<<grd, blk, band_features_smem(dmax), st>>>(cl, cr, disp0, (const uint8_t *)left, W, H,
+        pdl(k_band_features<uint8_t>, grd, blk, band_features_smem(dmax), st)(cl, cr, disp0, (const uint8_t *)left, W, H,
                                                       dmax, feat, &flags->status);
     else if (dtype == SV_F32)
-        k_band_features<float><<<grd, blk, band_features_smem(dmax), st>>>(cl, cr, disp0, (const float *)left, W, H,
+        pdl(k_band_features<float>, grd, blk, band_features_smem(dmax), st)(cl, cr, disp0, (const float *)left, W, H,
                                                     dmax, feat, &flags->status);
     else
-        k_band_features<double><<<grd, blk, band_features_smem(dmax), st>>>(cl, cr, disp0, (const double *)left, W, H,
+        pdl(k_band_features<double>, grd, blk, band_features_smem(dmax), st)(cl, cr, disp0, (const double *)left, W, H,
                                                       dmax, feat, &flags->status);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -662,7 +669,7 @@ int sv_band_train_step(sv_band *b, const float *feat, const float *target, const
     b->b2t *= b2;
     const double c1 = 1.0 / (1.0 - b->b1t), c2 = 1.0 / (1.0 - b->b2t);
     count_launch();
-    k_band_adam<<<(unsigned)((b->n + 255) / 256), 256, 0, st>>>(
+    pdl(k_band_adam, (unsigned)((b->n + 255) / 256), 256, 0, st)(
         b->p, b->g, b->m, b->v, b->n, (float)lr, (float)b1, (float)b2, 1.0e-8f, 5.0f, (float)c1,
         (float)c2);
     SV_LAUNCH_CHECK();
@@ -677,7 +684,7 @@ int sv_band_targets(const double *label, const uint8_t *status, const double *di
     }
     if (n < 1) { set_error("bad size"); return SV_ERR_SHAPE; }
     count_launch();
-    k_band_targets<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+    pdl(k_band_targets, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream)(
         label, status, disp0, n, shift_max, target, mask);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -695,7 +702,7 @@ int sv_band_apply(const float *out, const double *disp0, int W, int H, double b_
     }
     const long HW = (long)W * H;
     count_launch();
-    k_band_apply<<<(unsigned)((HW + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+    pdl(k_band_apply, (unsigned)((HW + 255) / 256), 256, 0, (cudaStream_t)stream)(
         out, disp0, HW, b_thr, rad_k, rad_min, R, shift_max, centre, rad);
     SV_LAUNCH_CHECK();
     return SV_OK;

@@ -67,6 +67,39 @@ struct DevFlags {
         }                                                                        \
     } while (0)
 
+// Launch of a kernel that may be set up before the kernel ahead of it in the stream
+// has ended (programmatic stream serialization): pdl(kernel, grid, block, shared
+// bytes, stream)(arguments...).  The kernel starts with pdl_sync().  Most launches
+// here last 4 to 10 us, 2 of them the gap to the one ahead: a 320 x 266 forward of 15
+// launches takes 237 us instead of 267, a 450 x 375 pair of 57 takes 400 instead of
+// 429.  No kernel lets the next one start early (launch_dependents): blocks that wait
+// beside working ones cost more than the set-up they hide (pair 457 us).
+template <typename... P>
+struct PdlLaunch {
+    void (*kernel)(P...);
+    cudaLaunchConfig_t cfg;
+    void operator()(P... args) const {
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t c = cfg;
+        c.attrs = &at;
+        c.numAttrs = 1;
+        void *a[] = {(void *)&args...};
+        cudaLaunchKernelExC(&c, (const void *)kernel, a);
+    }
+};
+template <typename... P>
+inline PdlLaunch<P...> pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                           cudaStream_t st) {
+    PdlLaunch<P...> l{kernel, {}};
+    l.cfg.gridDim = grid;
+    l.cfg.blockDim = block;
+    l.cfg.dynamicSmemBytes = smem;
+    l.cfg.stream = st;
+    return l;
+}
+
 inline int grid_for(long n, int block, int max_blocks = 148 * 16) {
     long g = (n + block - 1) / block;
     if (g < 1) g = 1;
@@ -75,10 +108,16 @@ inline int grid_for(long n, int block, int max_blocks = 148 * 16) {
 }
 
 // ---------------------------------------------------------------- device
+// In a kernel launched by pdl(), ahead of everything else and of any return: waits
+// for the end of the kernel ahead and for what it wrote.  (No effect in a plain
+// launch.)
+__device__ __forceinline__ void pdl_sync() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ void flag_error(int *flag, int code) {
     atomicCAS(flag, 0, code);
 }
-
 // Order-preserving map of a double to uint64 (NaN excluded by the caller).
 __device__ __forceinline__ unsigned long long ordkey(double d) {
     long long b = __double_as_longlong(d);

@@ -65,6 +65,7 @@ __device__ inline void nb_set_work(NetPair &p, int work) {
 
 // Before the probe: every pair runs, at its probe size, resampled.
 __global__ void k_nb_probe_init(NetPair *pairs, int n) {
+    pdl_sync();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     NetPair &p = pairs[i];
@@ -85,6 +86,7 @@ __global__ void k_nb_probe_init(NetPair *pairs, int n) {
 // decision, not a value select).
 __global__ void k_nb_decide(NetPair *pairs, int n, const char *slab0, long long slab,
                             long long sel_off, double tp, int max_width, int stage, int by_rule) {
+    pdl_sync();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     NetPair &p = pairs[i];
@@ -241,7 +243,7 @@ int nb_enqueue(sv_netbatch *nb, cudaStream_t st, bool refine) {
     int rc;
     // probe (stereonet.py:3900-3907)
     count_launch();
-    k_nb_probe_init<<<nbk, tb, 0, st>>>(pairs, n);
+    pdl(k_nb_probe_init, nbk, tb, 0, st)(pairs, n);
     SV_LAUNCH_CHECK();
     if ((rc = launch_b_resize(g[0], lt, rt, nb->dtype, s, false, st))) return rc;
     if ((rc = launch_b_forward(nb->view, g[0], s, st))) return rc;
@@ -257,7 +259,7 @@ int nb_enqueue(sv_netbatch *nb, cudaStream_t st, bool refine) {
     else rc = launch_b_sel_probe(Lone, s, st);
     if (rc) return rc;
     count_launch();
-    k_nb_decide<<<nbk, tb, 0, st>>>(pairs, n, s0, slab, sel_off, nb->target_peak, nb->max_width,
+    pdl(k_nb_decide, nbk, tb, 0, st)(pairs, n, s0, slab, sel_off, nb->target_peak, nb->max_width,
                                     0, by_rule);
     SV_LAUNCH_CHECK();
     // passes (stereonet.py:3918-3929)
@@ -271,7 +273,7 @@ int nb_enqueue(sv_netbatch *nb, cudaStream_t st, bool refine) {
         if (!with_sel) break;
         if (!by_rule && (rc = launch_b_sel_rest(Lsel, tsel, s, st))) return rc;
         count_launch();
-        k_nb_decide<<<nbk, tb, 0, st>>>(pairs, n, s0, slab, sel_off, nb->target_peak,
+        pdl(k_nb_decide, nbk, tb, 0, st)(pairs, n, s0, slab, sel_off, nb->target_peak,
                                         nb->max_width, pass, by_rule);
         SV_LAUNCH_CHECK();
     }

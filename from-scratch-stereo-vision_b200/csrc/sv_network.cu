@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(256)
     k_resize_pair(const T *__restrict__ l, const T *__restrict__ r, int W, int H, int W2, int H2,
                   float *__restrict__ lo, float *__restrict__ ro, float *__restrict__ gh,
                   SelState *sel, unsigned *sel_hist, long long sel_rank) {
+    pdl_sync();
     resize_pair_body<T>(blockIdx.x, blockIdx.y, blockIdx.z,
                         blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0, false, l, r, W,
                         H, W2, H2,
@@ -107,6 +108,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     k_b_resize_pair(NetLaunch L, const void *const *lt, const void *const *rt, float *lo,
                     float *ro, float *gh, SelState *sel, unsigned *sel_hist) {
+    pdl_sync();
     long long c;
     const int p = net_pair(L, c);
     const NetPair &P = L.pairs[p];
@@ -127,6 +129,7 @@ __global__ void __launch_bounds__(256)
 template <typename T>
 __global__ void k_to_f32_pair(const T *__restrict__ l, const T *__restrict__ r, long n,
                               float *__restrict__ lo, float *__restrict__ ro) {
+    pdl_sync();
     const T *src = blockIdx.y ? r : l;
     float *dst = blockIdx.y ? ro : lo;
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
@@ -139,6 +142,7 @@ __global__ void k_to_f32_pair(const T *__restrict__ l, const T *__restrict__ r, 
 template <typename T>
 __global__ void k_resize_scale(const T *__restrict__ x, int W, int H, int W2, int H2,
                                double inv, int scale, double *__restrict__ out) {
+    pdl_sync();
     int ox = blockIdx.x * blockDim.x + threadIdx.x;
     int oy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ox >= W2 || oy >= H2) return;
@@ -199,6 +203,7 @@ __global__ void __launch_bounds__(256)
     k_work_outputs(const float *__restrict__ d, int Ww, int Hw, int W, int H, double inv,
                    double *__restrict__ work64, double *__restrict__ full64, SelState *sel,
                    unsigned *ghist, WidthFuse wf, double *mirror) {
+    pdl_sync();
     work_outputs_body(blockIdx.x, blockIdx.y, gridDim.x * gridDim.y * gridDim.z, false, d, Ww,
                       Hw, W, H, inv, work64, full64, sel, ghist, wf.m >= 0 ? &wf : nullptr,
                       mirror);
@@ -211,6 +216,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     k_b_work_outputs(NetLaunch L, const float *d, double *work64, double *full64, SelState *sel,
                      unsigned *ghist, double target, int max_width) {
+    pdl_sync();
     long long c;
     const int p = net_pair(L, c);
     const NetPair &P = L.pairs[p];
@@ -229,6 +235,7 @@ __global__ void __launch_bounds__(256)
 
 template <typename T>
 __global__ void k_promote(const T *__restrict__ x, long n, double *__restrict__ out) {
+    pdl_sync();
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
          i += (long)gridDim.x * blockDim.x)
         out[i] = (double)x[i];
@@ -237,6 +244,7 @@ __global__ void k_promote(const T *__restrict__ x, long n, double *__restrict__ 
 // avgpool2, stereonet.py:979-995: 0.25 * (((a + b) + c) + d).
 __global__ void k_avgpool2(const float *__restrict__ img, int H, int W,
                            float *__restrict__ out) {
+    pdl_sync();
     int H2 = H / 2, W2 = W / 2;
     int x = blockIdx.x * blockDim.x + threadIdx.x;
     int y = blockIdx.y * blockDim.y + threadIdx.y;
@@ -249,6 +257,7 @@ __global__ void k_avgpool2(const float *__restrict__ img, int H, int W,
 // avgpool2 in FP64 over C planes (the drop-in for the reference function).
 __global__ void k_avgpool2_f64(const double *__restrict__ img, int C, int H, int W,
                                double *__restrict__ out) {
+    pdl_sync();
     const int H2 = H / 2, W2 = W / 2;
     const long n = (long)C * H2 * W2;
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
@@ -381,6 +390,7 @@ __global__ void __launch_bounds__(CT2_TW *CT2_TH *CS)
                    int OH, int OW, int stride, int pad, int dil, const float *__restrict__ w,
                    const float *__restrict__ b, float *y0, float *y1,
                    const float *__restrict__ resid) {
+    pdl_sync();
     conv2d_tiled_body<IC, OC, OCG, ACT, CS>(blockIdx.x, blockIdx.y, blockIdx.z, x0, x1, H, W,
                                             OH, OW, stride, pad, dil, w, b, y0, y1, resid);
 }
@@ -406,6 +416,7 @@ __global__ void __launch_bounds__(CT2_TW *CT2_TH *CS)
     k_b_conv2d_tiled(NetLaunch L, int lv, int Z, const float *x0, const float *x1, int stride,
                      int pad, int dil, const float *__restrict__ w, const float *__restrict__ b,
                      float *y0, float *y1, const float *resid) {
+    pdl_sync();
     long long c;
     const int p = net_pair(L, c);
     const NetPair &P = L.pairs[p];
@@ -537,6 +548,7 @@ __global__ void __launch_bounds__(CT2_TW *CT2_TH * 4)
     k_conv2d_out_decide(const float *__restrict__ x, int H, int W, const float *__restrict__ w,
                         const float *__restrict__ b, float *y, const float *__restrict__ resid,
                         WidthFuse f, SelState *s, unsigned *ghist, double *mirror) {
+    pdl_sync();
     __shared__ unsigned hist[kWidthBins + 1];
     const int t = threadIdx.x;
     for (int i = t; i <= f.m; i += CT2_TW * CT2_TH * 4) hist[i] = 0u;
@@ -559,6 +571,7 @@ __global__ void __launch_bounds__(CTB_TW / PX * CTB_TH)
     k_b_conv2d_wide(NetLaunch L, int lv, int Z, const float *x0, const float *x1, int dil,
                     const float *__restrict__ w, const float *__restrict__ b, float *y0,
                     float *y1, const float *resid) {
+    pdl_sync();
     long long c;
     const int p = net_pair(L, c);
     const NetPair &P = L.pairs[p];
@@ -589,7 +602,7 @@ static void b_conv2d_wide(const NetLaunch &L, unsigned ctas, int lv, int Z, cons
     if (smem + kStatic > 48 * 1024)
         cudaFuncSetAttribute(k_b_conv2d_wide<IC, OC, ACT, CS, PX, S>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_b_conv2d_wide<IC, OC, ACT, CS, PX, S><<<ctas, CTB_TW / PX * CTB_TH, smem, st>>>(
+    pdl(k_b_conv2d_wide<IC, OC, ACT, CS, PX, S>, ctas, CTB_TW / PX * CTB_TH, smem, st)(
         L, lv, Z, x0, x1, dil, w, b, y0, y1, resid);
 }
 
@@ -666,6 +679,7 @@ __global__ void __launch_bounds__(CT2_TW *CT2_TH)
     k_conv2d_up(const float *__restrict__ prev, int ph, int pw, const float *__restrict__ guide,
                 int H, int W, int dil, const float *__restrict__ w, const float *__restrict__ b,
                 float *__restrict__ y, float *__restrict__ rin0) {
+    pdl_sync();
     conv2d_up_body<RC, OCG>(blockIdx.x, blockIdx.y, blockIdx.z, prev, ph, pw, guide, H, W, dil,
                             w, b, y, rin0);
 }
@@ -677,6 +691,7 @@ __global__ void __launch_bounds__(CT2_TW *CT2_TH)
     k_b_conv2d_up(NetLaunch L, int lv, const float *prev, const float *guide, int dil,
                   const float *__restrict__ w, const float *__restrict__ b, float *y,
                   float *rin0) {
+    pdl_sync();
     long long c;
     const int p = net_pair(L, c);
     const NetPair &P = L.pairs[p];
@@ -926,6 +941,7 @@ __global__ void __launch_bounds__(128)
     k_conv3d_split(const float *__restrict__ a, const float *__restrict__ bsrc, int D, int h,
                    int w, const float *__restrict__ wt, const float *__restrict__ bias,
                    float *__restrict__ y) {
+    pdl_sync();
     conv3d_split_body<C, OCG, CS, CV>(blockIdx.x, blockIdx.y, blockIdx.z, a, bsrc, D, h, w, wt,
                                       bias, y);
 }
@@ -936,6 +952,7 @@ template <int C, int OCG, int CS, bool CV>
 __global__ void __launch_bounds__(128)
     k_b_conv3d_split(NetLaunch L, int Z, const float *a, const float *bsrc, int D,
                      const float *__restrict__ wt, const float *__restrict__ bias, float *y) {
+    pdl_sync();
     long long c;
     const int p = net_pair(L, c);
     const NetPair &P = L.pairs[p];
@@ -1094,6 +1111,7 @@ template <int C, int OC, int CS, bool CV>
 __global__ void __launch_bounds__(128)
     k_b_conv3d_wide(NetLaunch L, const float *a, const float *bsrc, int D,
                     const float *__restrict__ wt, const float *__restrict__ bias, float *y) {
+    pdl_sync();
     using G = C3W<C, CS>;
     long long c;
     const int p = net_pair(L, c);
@@ -1183,6 +1201,7 @@ __global__ void __launch_bounds__(128 * CS)
                         const float *__restrict__ wt, const float *__restrict__ b,
                         float *__restrict__ disp, float *__restrict__ spread,
                         float *__restrict__ pmax) {
+    pdl_sync();
     conv3d_softargmin_body<IC, CS>(blockIdx.x, blockIdx.y, x, D, h, w, wt, b, disp, spread, pmax);
 }
 
@@ -1190,6 +1209,7 @@ template <int IC, int CS>
 __global__ void __launch_bounds__(128 * CS)
     k_b_conv3d_softargmin(NetLaunch L, const float *x, int D, const float *__restrict__ wt,
                           const float *__restrict__ b, float *disp) {
+    pdl_sync();
     long long c;
     const int p = net_pair(L, c);
     const NetPair &P = L.pairs[p];
@@ -1222,9 +1242,9 @@ int launch_resize_pair(const void *l, const void *r, int dtype, int W, int H, in
         // a resample to the same size still runs the reference's arithmetic
     }
     switch (dtype) {
-    case SV_U8: count_launch(); k_resize_pair<uint8_t><<<g, blk, 0, st>>>((const uint8_t *)l, (const uint8_t *)r, W, H, W2, H2, lo, ro, gh, ss, sh, sr); break;
-    case SV_F32: count_launch(); k_resize_pair<float><<<g, blk, 0, st>>>((const float *)l, (const float *)r, W, H, W2, H2, lo, ro, gh, ss, sh, sr); break;
-    case SV_F64: count_launch(); k_resize_pair<double><<<g, blk, 0, st>>>((const double *)l, (const double *)r, W, H, W2, H2, lo, ro, gh, ss, sh, sr); break;
+    case SV_U8: count_launch(); pdl(k_resize_pair<uint8_t>, g, blk, 0, st)((const uint8_t *)l, (const uint8_t *)r, W, H, W2, H2, lo, ro, gh, ss, sh, sr); break;
+    case SV_F32: count_launch(); pdl(k_resize_pair<float>, g, blk, 0, st)((const float *)l, (const float *)r, W, H, W2, H2, lo, ro, gh, ss, sh, sr); break;
+    case SV_F64: count_launch(); pdl(k_resize_pair<double>, g, blk, 0, st)((const double *)l, (const double *)r, W, H, W2, H2, lo, ro, gh, ss, sh, sr); break;
     default: set_error("unknown dtype %d", dtype); return SV_ERR_PARAM;
     }
     SV_LAUNCH_CHECK();
@@ -1235,9 +1255,9 @@ int launch_to_f32_pair(const void *l, const void *r, int dtype, long n, float *l
                        cudaStream_t st) {
     dim3 g(grid_for(n, 256), 2);
     switch (dtype) {
-    case SV_U8: count_launch(); k_to_f32_pair<uint8_t><<<g, 256, 0, st>>>((const uint8_t *)l, (const uint8_t *)r, n, lo, ro); break;
-    case SV_F32: count_launch(); k_to_f32_pair<float><<<g, 256, 0, st>>>((const float *)l, (const float *)r, n, lo, ro); break;
-    case SV_F64: count_launch(); k_to_f32_pair<double><<<g, 256, 0, st>>>((const double *)l, (const double *)r, n, lo, ro); break;
+    case SV_U8: count_launch(); pdl(k_to_f32_pair<uint8_t>, g, 256, 0, st)((const uint8_t *)l, (const uint8_t *)r, n, lo, ro); break;
+    case SV_F32: count_launch(); pdl(k_to_f32_pair<float>, g, 256, 0, st)((const float *)l, (const float *)r, n, lo, ro); break;
+    case SV_F64: count_launch(); pdl(k_to_f32_pair<double>, g, 256, 0, st)((const double *)l, (const double *)r, n, lo, ro); break;
     default: set_error("unknown dtype %d", dtype); return SV_ERR_PARAM;
     }
     SV_LAUNCH_CHECK();
@@ -1247,7 +1267,7 @@ int launch_to_f32_pair(const void *l, const void *r, int dtype, long n, float *l
 int launch_resize_f64(const double *x, int W, int H, int W2, int H2, double *out,
                       cudaStream_t st) {
     dim3 blk(32, 8);
-    count_launch(); k_resize_scale<double><<<grid2d(W2, H2, blk), blk, 0, st>>>(x, W, H, W2, H2, 1.0, 0, out);
+    count_launch(); pdl(k_resize_scale<double>, grid2d(W2, H2, blk), blk, 0, st)(x, W, H, W2, H2, 1.0, 0, out);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -1255,7 +1275,7 @@ int launch_resize_f64(const double *x, int W, int H, int W2, int H2, double *out
 int launch_upscale_disp(const float *dw, int Ww, int Hw, int W, int H, double inv,
                         double *out, cudaStream_t st) {
     dim3 blk(32, 8);
-    count_launch(); k_resize_scale<float><<<grid2d(W, H, blk), blk, 0, st>>>(dw, Ww, Hw, W, H, inv, 1, out);
+    count_launch(); pdl(k_resize_scale<float>, grid2d(W, H, blk), blk, 0, st)(dw, Ww, Hw, W, H, inv, 1, out);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -1263,7 +1283,7 @@ int launch_upscale_disp(const float *dw, int Ww, int Hw, int W, int H, double in
 int launch_resize_f32(const float *x, int W, int H, int W2, int H2, double *out,
                       cudaStream_t st) {
     dim3 blk(32, 8);
-    count_launch(); k_resize_scale<float><<<grid2d(W2, H2, blk), blk, 0, st>>>(x, W, H, W2, H2, 1.0, 0, out);
+    count_launch(); pdl(k_resize_scale<float>, grid2d(W2, H2, blk), blk, 0, st)(x, W, H, W2, H2, 1.0, 0, out);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -1277,7 +1297,7 @@ int launch_work_outputs(const float *d, int Ww, int Hw, int W, int H, double inv
     dim3 blk(32, 8);
     count_launch();
     const WidthFuse wf = fuse && fuse->width ? *fuse->width : WidthFuse{{0, 0, 0.0, 0.0}, -1, 0, 0};
-    k_work_outputs<<<grid2d(W, H, blk), blk, 0, st>>>(d, Ww, Hw, W, H, inv, work64, full64,
+    pdl(k_work_outputs, grid2d(W, H, blk), blk, 0, st)(d, Ww, Hw, W, H, inv, work64, full64,
                                                        fuse ? fuse->state : nullptr,
                                                        fuse ? fuse->hist : nullptr, wf,
                                                        fuse ? fuse->mirror : nullptr);
@@ -1286,7 +1306,7 @@ int launch_work_outputs(const float *d, int Ww, int Hw, int W, int H, double inv
 }
 
 int launch_promote(const float *x, long n, double *out, cudaStream_t st) {
-    count_launch(); k_promote<float><<<grid_for(n, 256), 256, 0, st>>>(x, n, out);
+    count_launch(); pdl(k_promote<float>, grid_for(n, 256), 256, 0, st)(x, n, out);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -1295,7 +1315,7 @@ int launch_avgpool2_f64(const double *img, int C, int H, int W, double *out, cud
     long n = (long)C * (H / 2) * (W / 2);
     if (n > 0) {
         count_launch();
-        k_avgpool2_f64<<<grid_for(n, 256), 256, 0, st>>>(img, C, H, W, out);
+        pdl(k_avgpool2_f64, grid_for(n, 256), 256, 0, st)(img, C, H, W, out);
     }
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -1303,7 +1323,7 @@ int launch_avgpool2_f64(const double *img, int C, int H, int W, double *out, cud
 
 int launch_avgpool2(const float *img, int H, int W, float *out, cudaStream_t st) {
     dim3 blk(32, 8);
-    count_launch(); k_avgpool2<<<grid2d(W / 2, H / 2, blk), blk, 0, st>>>(img, H, W, out);
+    count_launch(); pdl(k_avgpool2, grid2d(W / 2, H / 2, blk), blk, 0, st)(img, H, W, out);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -1411,18 +1431,18 @@ static int forward_impl(const NetView &n, const float *left, const float *right,
         constexpr int FG = C % 4 == 0 ? 4 : C, FG2 = C % 2 == 0 ? 2 : C;
         const dim3 fg1 = tgrid(w1, h1, 2 * (C / FG)), fg = tgrid(w, h, 2 * (C / FG2));
         count_launch();
-        k_conv2d_tiled<1, C, FG, 1, 1><<<fg1, tb1, conv2d_tile_bytes(1, 2, 1), st>>>(
+        pdl(k_conv2d_tiled<1, C, FG, 1, 1>, fg1, tb1, conv2d_tile_bytes(1, 2, 1), st)(
             left, right, H, W, h1, w1, 2, 1, 1, n.fw[0], n.fb[0], b.fa[0], b.fa[1], nullptr);
         count_launch();
-        k_conv2d_tiled<C, C, FG2, 1, 2><<<fg, tb2, conv2d_tile_bytes(C, 2, 1, 2), st>>>(
+        pdl(k_conv2d_tiled<C, C, FG2, 1, 2>, fg, tb2, conv2d_tile_bytes(C, 2, 1, 2), st)(
             b.fa[0], b.fa[1], h1, w1, h, w, 2, 1, 1, n.fw[1], n.fb[1], b.fb[0], b.fb[1],
             nullptr);
         count_launch();
-        k_conv2d_tiled<C, C, FG2, 1, 2><<<fg, tb2, conv2d_tile_bytes(C, 1, 1, 2), st>>>(
+        pdl(k_conv2d_tiled<C, C, FG2, 1, 2>, fg, tb2, conv2d_tile_bytes(C, 1, 1, 2), st)(
             b.fb[0], b.fb[1], h, w, h, w, 1, 1, 1, n.fw[2], n.fb[2], b.fa[0], b.fa[1],
             nullptr);
         count_launch();
-        k_conv2d_tiled<C, C, FG2, 0, 2><<<fg, tb2, conv2d_tile_bytes(C, 1, 1, 2), st>>>(
+        pdl(k_conv2d_tiled<C, C, FG2, 0, 2>, fg, tb2, conv2d_tile_bytes(C, 1, 1, 2), st)(
             b.fa[0], b.fa[1], h, w, h, w, 1, 1, 1, n.fw[3], n.fb[3], b.fb[0], b.fb[1],
             nullptr);
         SV_LAUNCH_CHECK();
@@ -1433,15 +1453,15 @@ static int forward_impl(const NetView &n, const float *left, const float *right,
         const dim3 vg1((w + C3_TX - 1) / C3_TX, h * ((D + 16 / S1 - 1) / (16 / S1)), CM / CG);
         const dim3 vg2((w + C3_TX - 1) / C3_TX, h * ((D + 16 / S2 - 1) / (16 / S2)), CM / CG);
         count_launch();
-        k_conv3d_split<C, CG, S1, true><<<vg1, 128, 0, st>>>(b.fb[0], b.fb[1], D, h, w, n.cw[0],
+        pdl(k_conv3d_split<C, CG, S1, true>, vg1, 128, 0, st)(b.fb[0], b.fb[1], D, h, w, n.cw[0],
                                                              n.cb[0], b.v0);
         count_launch();
-        k_conv3d_split<CM, CG, S2, false><<<vg2, 128, 0, st>>>(b.v0, nullptr, D, h, w, n.cw[1],
+        pdl(k_conv3d_split<CM, CG, S2, false>, vg2, 128, 0, st)(b.v0, nullptr, D, h, w, n.cw[1],
                                                                n.cb[1], b.v1);
     }
     constexpr int S3 = CM % 2 == 0 ? 2 : 1;
     count_launch();
-    k_conv3d_softargmin<CM, S3><<<dim3((w + C3_TX - 1) / C3_TX, h), 128 * S3, 0, st>>>(
+    pdl(k_conv3d_softargmin<CM, S3>, dim3((w + C3_TX - 1) / C3_TX, h), 128 * S3, 0, st)(
         b.v1, D, h, w, n.cw[2], n.cb[2], d0, b.qspread, b.qspread ? b.qpmax : nullptr);
     SV_LAUNCH_CHECK();
     // Refinement levels
@@ -1461,26 +1481,26 @@ static int forward_impl(const NetView &n, const float *left, const float *right,
             const int dl = n.dil[i];
             count_launch();
             if (i == 0)     // up-sample + concat built into the first convolution
-                k_conv2d_up<RC, RG><<<tgrid(Wl, Hl, RC / RG), tb, conv2d_tile_bytes(2, 1, dl),
-                                      st>>>(prev, ph, pw, guides[lv], Hl, Wl, dl, n.rw[lv][i],
+                pdl(k_conv2d_up<RC, RG>, tgrid(Wl, Hl, RC / RG), tb, conv2d_tile_bytes(2, 1, dl),
+                                      st)(prev, ph, pw, guides[lv], Hl, Wl, dl, n.rw[lv][i],
                                             n.rb[lv][i], dst, b.rin);
             else            // every output channel per thread (measured faster)
-                k_conv2d_tiled<RC, RC, RC, 1, RS><<<tgrid(Wl, Hl, 1), RS * tb1,
-                                                    conv2d_tile_bytes(RC, 1, dl, RS), st>>>(
+                pdl(k_conv2d_tiled<RC, RC, RC, 1, RS>, tgrid(Wl, Hl, 1), RS * tb1,
+                                                    conv2d_tile_bytes(RC, 1, dl, RS), st)(
                     cur, cur, Hl, Wl, Hl, Wl, 1, dl, dl, n.rw[lv][i], n.rb[lv][i], dst, dst,
                     nullptr);
             cur = dst;
         }
         count_launch();
         if (lv == 1 && b.decide && b.decide->width)
-            k_conv2d_out_decide<RC><<<tgrid(Wl, Hl, 1), tb4, conv2d_tile_bytes(RC, 1, 1, 4),
-                                      st>>>(cur, Hl, Wl, n.rw[lv][n.ndil], n.rb[lv][n.ndil],
+            pdl(k_conv2d_out_decide<RC>, tgrid(Wl, Hl, 1), tb4, conv2d_tile_bytes(RC, 1, 1, 4),
+                                      st)(cur, Hl, Wl, n.rw[lv][n.ndil], n.rb[lv][n.ndil],
                                             outs[lv], b.rin, *b.decide->width,
                                             b.decide->state, b.decide->hist,
                                             b.decide->mirror);
         else
-            k_conv2d_tiled<RC, 1, 1, 2, 4><<<tgrid(Wl, Hl, 1), tb4,
-                                             conv2d_tile_bytes(RC, 1, 1, 4), st>>>(
+            pdl(k_conv2d_tiled<RC, 1, 1, 2, 4>, tgrid(Wl, Hl, 1), tb4,
+                                             conv2d_tile_bytes(RC, 1, 1, 4), st)(
                 cur, cur, Hl, Wl, Hl, Wl, 1, 1, 1, n.rw[lv][n.ndil], n.rb[lv][n.ndil], outs[lv],
                 outs[lv], b.rin);
         SV_LAUNCH_CHECK();
@@ -1602,14 +1622,14 @@ static int b_forward_impl(const NetView &n, const NetStageLaunch &g, const NetSl
     SV_LAUNCH_CHECK();
     constexpr int S1 = C % 4 == 0 ? 4 : 2, S2 = CM % 4 == 0 && CM > 4 ? 4 : 2;
     count_launch();
-    k_b_conv3d_wide<C, CM, S1, true><<<B(NK_V1), 128, 0, st>>>(
+    pdl(k_b_conv3d_wide<C, CM, S1, true>, B(NK_V1), 128, 0, st)(
         L(NK_V1), s.f.fb[0], s.f.fb[1], D, n.cw[0], n.cb[0], s.f.v0);
     count_launch();
-    k_b_conv3d_wide<CM, CM, S2, false><<<B(NK_V2), 128, 0, st>>>(
+    pdl(k_b_conv3d_wide<CM, CM, S2, false>, B(NK_V2), 128, 0, st)(
         L(NK_V2), s.f.v0, nullptr, D, n.cw[1], n.cb[1], s.f.v1);
     constexpr int S3 = CM % 2 == 0 ? 2 : 1;
     count_launch();
-    k_b_conv3d_softargmin<CM, S3><<<B(NK_SA), 128 * S3, 0, st>>>(L(NK_SA), s.f.v1, D, n.cw[2],
+    pdl(k_b_conv3d_softargmin<CM, S3>, B(NK_SA), 128 * S3, 0, st)(L(NK_SA), s.f.v1, D, n.cw[2],
                                                                   n.cb[2], s.d0);
     SV_LAUNCH_CHECK();
     constexpr int RG = RC % 4 == 0 ? 4 : RC;
@@ -1627,15 +1647,15 @@ static int b_forward_impl(const NetView &n, const NetStageLaunch &g, const NetSl
             const int dl = n.dil[i];
             count_launch();
             if (i == 0)
-                k_b_conv2d_up<RC, RG><<<B(kk), tb, conv2d_tile_bytes(2, 1, dl), st>>>(
+                pdl(k_b_conv2d_up<RC, RG>, B(kk), tb, conv2d_tile_bytes(2, 1, dl), st)(
                     L(kk), lv, prevs[lv], guides[lv], dl, n.rw[lv][i], n.rb[lv][i], dst, s.f.rin);
             else if (!tiled)
                 b_conv2d_wide<RC, RC, 1, RS, 2, 1>(L(kf), B(kf), lv + 3, 1, cur, cur, dl,
                                                    n.rw[lv][i], n.rb[lv][i], dst, dst, nullptr,
                                                    st);
             else
-                k_b_conv2d_tiled<RC, RC, RG, 1, RS><<<B(kk), RS * tb1,
-                                                      conv2d_tile_bytes(RC, 1, dl, RS), st>>>(
+                pdl(k_b_conv2d_tiled<RC, RC, RG, 1, RS>, B(kk), RS * tb1,
+                                                      conv2d_tile_bytes(RC, 1, dl, RS), st)(
                     L(kk), 3 + lv, RC / RG, cur, cur, 1, dl, dl, n.rw[lv][i], n.rb[lv][i], dst,
                     dst, nullptr);
             cur = dst;
@@ -1646,8 +1666,8 @@ static int b_forward_impl(const NetView &n, const NetStageLaunch &g, const NetSl
                                              n.rw[lv][n.ndil], n.rb[lv][n.ndil], outs[lv],
                                              outs[lv], s.f.rin, st);
         else
-            k_b_conv2d_tiled<RC, 1, 1, 2, 4><<<B(kf), 4 * tb1, conv2d_tile_bytes(RC, 1, 1, 4),
-                                               st>>>(L(kf), 3 + lv, 1, cur, cur, 1, 1, 1,
+            pdl(k_b_conv2d_tiled<RC, 1, 1, 2, 4>, B(kf), 4 * tb1, conv2d_tile_bytes(RC, 1, 1, 4),
+                                               st)(L(kf), 3 + lv, 1, cur, cur, 1, 1, 1,
                                                      n.rw[lv][n.ndil], n.rb[lv][n.ndil],
                                                      outs[lv], outs[lv], s.f.rin);
         SV_LAUNCH_CHECK();
@@ -1678,9 +1698,9 @@ int launch_b_resize(const NetStageLaunch &g, const void *const *lt, const void *
     SelState *sel = with_sel ? s.sel : nullptr;
     count_launch();
     switch (dtype) {
-    case SV_U8: k_b_resize_pair<uint8_t><<<B, blk, 0, st>>>(L, lt, rt, s.lw, s.rw, s.gh, sel, s.hist); break;
-    case SV_F32: k_b_resize_pair<float><<<B, blk, 0, st>>>(L, lt, rt, s.lw, s.rw, s.gh, sel, s.hist); break;
-    case SV_F64: k_b_resize_pair<double><<<B, blk, 0, st>>>(L, lt, rt, s.lw, s.rw, s.gh, sel, s.hist); break;
+    case SV_U8: pdl(k_b_resize_pair<uint8_t>, B, blk, 0, st)(L, lt, rt, s.lw, s.rw, s.gh, sel, s.hist); break;
+    case SV_F32: pdl(k_b_resize_pair<float>, B, blk, 0, st)(L, lt, rt, s.lw, s.rw, s.gh, sel, s.hist); break;
+    case SV_F64: pdl(k_b_resize_pair<double>, B, blk, 0, st)(L, lt, rt, s.lw, s.rw, s.gh, sel, s.hist); break;
     default: set_error("unknown dtype %d", dtype); return SV_ERR_PARAM;
     }
     SV_LAUNCH_CHECK();
@@ -1690,7 +1710,7 @@ int launch_b_resize(const NetStageLaunch &g, const void *const *lt, const void *
 int launch_b_work_outputs(const NetLaunch &L, long long total, const NetSlab &s, bool with_sel,
                           double target, int rule_width, cudaStream_t st) {
     count_launch();
-    k_b_work_outputs<<<ctas_of(total), dim3(32, 8), 0, st>>>(
+    pdl(k_b_work_outputs, ctas_of(total), dim3(32, 8), 0, st)(
         L, s.d2, nullptr, s.full, with_sel ? s.sel : nullptr, with_sel ? s.hist : nullptr,
         target, rule_width);
     SV_LAUNCH_CHECK();

@@ -40,6 +40,7 @@ constexpr int kMedMaxR = 3;
 
 __global__ void k_median(const double *__restrict__ in, int W, int H, int r,
                          double *__restrict__ out) {
+    pdl_sync();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= W || y >= H) return;
@@ -79,7 +80,7 @@ int launch_median(const double *in, int W, int H, int radius, int passes, double
     for (int p = 0; p < passes; ++p) {
         double *dst = ((passes - 1 - p) & 1) ? tmp : out;
         count_launch();
-        k_median<<<grd, blk, 0, st>>>(src, W, H, radius, dst);
+        pdl(k_median, grd, blk, 0, st)(src, W, H, radius, dst);
         src = dst;
     }
     SV_LAUNCH_CHECK();
@@ -113,6 +114,7 @@ __device__ __forceinline__ double slic_dd(const double *__restrict__ rgb, long i
 
 __global__ void k_slic_init(const double *__restrict__ rgb, int W, int step, int ncx, int nc,
                             SlicCenter *__restrict__ cs) {
+    pdl_sync();
     const int ci = blockIdx.x * blockDim.x + threadIdx.x;
     if (ci >= nc) return;
     const int cx = step / 2 + (ci % ncx) * step, cy = step / 2 + (ci / ncx) * step;
@@ -123,6 +125,7 @@ __global__ void k_slic_init(const double *__restrict__ rgb, int W, int step, int
 
 __global__ void k_slic_reset(long N, unsigned long long *__restrict__ dist,
                              int *__restrict__ labtmp, int *__restrict__ flag) {
+    pdl_sync();
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i == 0) *flag = 0;
     if (i >= N) return;
@@ -135,6 +138,7 @@ __global__ void __launch_bounds__(256)
     k_slic_assign(const double *__restrict__ rgb, int W, int H, int step, double m2,
                   const SlicCenter *__restrict__ cs, int pass, unsigned long long *__restrict__ dist,
                   int *__restrict__ labtmp) {
+    pdl_sync();
     const int ci = blockIdx.x;
     const SlicCenter c = cs[ci];
     const int4 w = slic_window(c, step, W, H);
@@ -151,6 +155,7 @@ __global__ void __launch_bounds__(256)
 
 __global__ void k_slic_commit(long N, const int *__restrict__ labtmp, int *__restrict__ lab,
                               int *__restrict__ flag) {
+    pdl_sync();
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i >= N) return;
     const int l = labtmp[i];
@@ -170,6 +175,7 @@ __global__ void __launch_bounds__(32 * kUpdWarps)
                   SlicCenter *__restrict__ cs, const int *__restrict__ lab,
                   const int *__restrict__ flag, int4 *__restrict__ win,
                   double *__restrict__ acc, int cap) {
+    pdl_sync();
     __shared__ double sv[kUpdWarps][32][3];
     extern __shared__ __align__(16) unsigned char upd_smem[];   // [warps][cap] staged pixels
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
@@ -323,6 +329,7 @@ __global__ void __launch_bounds__(256)
                 const int *__restrict__ flag, int pass, int *__restrict__ count,
                 const int *__restrict__ start, int *__restrict__ list,
                 const uint8_t *__restrict__ valid, int *__restrict__ nvalid) {
+    pdl_sync();
     __shared__ int sbuf[32];
     if (*flag) {
         if (blockIdx.x != 0 || threadIdx.x != 0) return;
@@ -372,6 +379,7 @@ __global__ void __launch_bounds__(256)
 // Exclusive scan of count[] into start[] (one CTA of 1024 threads).
 __global__ void __launch_bounds__(1024)
     k_seg_scan(int nseg, const int *__restrict__ count, int *__restrict__ start) {
+    pdl_sync();
     __shared__ int sbuf[32];
     int base = 0;
     for (int g0 = 0; g0 < nseg; g0 += blockDim.x) {
@@ -410,6 +418,7 @@ constexpr int kJumpBits = 24;                // up to 2^24 segments
 __global__ void __launch_bounds__(1024)
     k_seg_rng(int nseg, const int *__restrict__ nvalid, int trials, uint32_t seed,
               uint32_t *__restrict__ state) {
+    pdl_sync();
     __shared__ uint32_t J[kJumpBits][32];
     __shared__ uint32_t T[2][32];
     __shared__ int sbuf[32];
@@ -500,6 +509,7 @@ __global__ void __launch_bounds__(256)
                const int *__restrict__ nvalid, const uint32_t *__restrict__ state, int trials,
                double thr, double min_inl, int *__restrict__ pts, int *__restrict__ inl,
                double *__restrict__ out) {
+    pdl_sync();
     __shared__ double planes[kMaxTrials][3];
     __shared__ int ok[kMaxTrials], cnt[kMaxTrials];
     __shared__ int sbuf[32];
@@ -656,6 +666,7 @@ __global__ void __launch_bounds__(256)
 
 __global__ void k_status_valid(long N, const uint8_t *__restrict__ status,
                                uint8_t *__restrict__ valid) {
+    pdl_sync();
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i < N) valid[i] = status[i] == 0;
 }
@@ -721,7 +732,7 @@ int launch_slic(const double *rgb, int W, int H, int step, double compactness, i
     SV_CUDA_TRY(cudaMemsetAsync(w.flag, 0, sizeof(int) * 4, st));
     if (nc == 0) return SV_OK;
     count_launch();
-    k_slic_init<<<(nc + 127) / 128, 128, 0, st>>>(rgb, W, step, ncx, nc, cs);
+    pdl(k_slic_init, (nc + 127) / 128, 128, 0, st)(rgb, W, step, ncx, nc, cs);
     const int nb = grid_for(N, 256, 1 << 30);
     // SLIC update staging: (2 step + 1)^2 pixels of 32 bytes per warp
     const long wmax = (long)(2 * step + 1) * (2 * step + 1);
@@ -731,15 +742,15 @@ int launch_slic(const double *rgb, int W, int H, int step, double compactness, i
     const int cap = wpb0 < 1 ? 0 : (int)wmax;
     for (int it = 0; it < iters; ++it) {
         count_launch();
-        k_slic_reset<<<nb, 256, 0, st>>>(N, w.dist, w.labtmp, w.flag);
+        pdl(k_slic_reset, nb, 256, 0, st)(N, w.dist, w.labtmp, w.flag);
         count_launch();
-        k_slic_assign<<<nc, 256, 0, st>>>(rgb, W, H, step, m2, cs, 0, w.dist, w.labtmp);
+        pdl(k_slic_assign, nc, 256, 0, st)(rgb, W, H, step, m2, cs, 0, w.dist, w.labtmp);
         count_launch();
-        k_slic_assign<<<nc, 256, 0, st>>>(rgb, W, H, step, m2, cs, 1, w.dist, w.labtmp);
+        pdl(k_slic_assign, nc, 256, 0, st)(rgb, W, H, step, m2, cs, 1, w.dist, w.labtmp);
         count_launch();
-        k_slic_commit<<<nb, 256, 0, st>>>(N, w.labtmp, w.lab, w.flag);
+        pdl(k_slic_commit, nb, 256, 0, st)(N, w.labtmp, w.lab, w.flag);
         count_launch();
-        k_slic_update<<<(nc + wpb - 1) / wpb, 32 * wpb, (size_t)wpb * cap * 32, st>>>(
+        pdl(k_slic_update, (nc + wpb - 1) / wpb, 32 * wpb, (size_t)wpb * cap * 32, st)(
             rgb, W, H, step, nc, cs, w.lab, w.flag, w.win, w.acc, cap);
     }
     SV_LAUNCH_CHECK();
@@ -760,17 +771,17 @@ int launch_plane_snap(const double *disp, const double *rgb, int W, int H, const
     SV_TRY_POST(launch_slic(rgb, W, H, step, 10.0, 5, w, st));
     if (nc == 0 || trials == 0) return SV_OK;
     count_launch();
-    k_seg_lists<<<nc, 256, 0, st>>>(W, H, nc, w.lab, w.win, w.flag, 0, w.count, w.start, w.list,
+    pdl(k_seg_lists, nc, 256, 0, st)(W, H, nc, w.lab, w.win, w.flag, 0, w.count, w.start, w.list,
                                     valid, w.nvalid);
     count_launch();
-    k_seg_scan<<<1, 1024, 0, st>>>(nc, w.count, w.start);
+    pdl(k_seg_scan, 1, 1024, 0, st)(nc, w.count, w.start);
     count_launch();
-    k_seg_lists<<<nc, 256, 0, st>>>(W, H, nc, w.lab, w.win, w.flag, 1, w.count, w.start, w.list,
+    pdl(k_seg_lists, nc, 256, 0, st)(W, H, nc, w.lab, w.win, w.flag, 1, w.count, w.start, w.list,
                                     valid, w.nvalid);
     count_launch();
-    k_seg_rng<<<1, 1024, 0, st>>>(nc, w.nvalid, trials, seed, w.state);
+    pdl(k_seg_rng, 1, 1024, 0, st)(nc, w.nvalid, trials, seed, w.state);
     count_launch();
-    k_seg_snap<<<nc, 256, 0, st>>>(disp, W, valid, w.start, w.list, w.nvalid, w.state, trials,
+    pdl(k_seg_snap, nc, 256, 0, st)(disp, W, valid, w.start, w.list, w.nvalid, w.state, trials,
                                    thr, min_inl, w.pts, w.inl, out);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -778,7 +789,7 @@ int launch_plane_snap(const double *disp, const double *rgb, int W, int H, const
 
 int launch_status_valid(const uint8_t *status, long N, uint8_t *valid, cudaStream_t st) {
     count_launch();
-    k_status_valid<<<grid_for(N, 256, 1 << 30), 256, 0, st>>>(N, status, valid);
+    pdl(k_status_valid, grid_for(N, 256, 1 << 30), 256, 0, st)(N, status, valid);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -791,6 +802,7 @@ namespace sv {
 // mirror_h (stereonet.py:4974-4983) of one [H][W] plane of esize-byte values
 __global__ void k_mirror(const unsigned char *__restrict__ in, int esize, int W, int H,
                          unsigned char *__restrict__ out) {
+    pdl_sync();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= W || y >= H) return;
     const long src = ((long)y * W + (W - 1 - x)) * esize, dst = ((long)y * W + x) * esize;
@@ -801,6 +813,7 @@ __global__ void k_mirror(const unsigned char *__restrict__ in, int esize, int W,
 __global__ void k_lr_consistency(const double *__restrict__ dl, const double *__restrict__ dr,
                                  int W, int H, double tol, uint8_t *__restrict__ valid,
                                  unsigned long long *__restrict__ kept) {
+    pdl_sync();
     const long N = (long)W * H;
     const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
     int ok = 0;
@@ -835,6 +848,7 @@ __global__ void k_lr_consistency(const double *__restrict__ dl, const double *__
 __global__ void __launch_bounds__(1024)
     k_fill_invalid(const double *__restrict__ disp, const uint8_t *__restrict__ valid, int W,
                    int H, int *__restrict__ left_idx, double *__restrict__ out) {
+    pdl_sync();
     __shared__ int sbuf[32];
     __shared__ int carry;
     const int y = blockIdx.x, t = threadIdx.x, bd = blockDim.x;
@@ -883,7 +897,7 @@ __global__ void __launch_bounds__(1024)
 
 int launch_mirror(const void *in, int esize, int W, int H, void *out, cudaStream_t st) {
     count_launch();
-    k_mirror<<<dim3((W + 255) / 256, H), 256, 0, st>>>((const unsigned char *)in, esize, W, H,
+    pdl(k_mirror, dim3((W + 255) / 256, H), 256, 0, st)((const unsigned char *)in, esize, W, H,
                                                        (unsigned char *)out);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -894,7 +908,7 @@ int launch_lr_consistency(const double *dl, const double *dr, int W, int H, doub
     SV_CUDA_TRY(cudaMemsetAsync(kept, 0, sizeof(unsigned long long), st));
     const long N = (long)W * H;
     count_launch();
-    k_lr_consistency<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(dl, dr, W, H, tol, valid, kept);
+    pdl(k_lr_consistency, (unsigned)((N + 255) / 256), 256, 0, st)(dl, dr, W, H, tol, valid, kept);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -903,7 +917,7 @@ int launch_fill_invalid(const double *disp, const uint8_t *valid, int W, int H, 
                         double *out, cudaStream_t st) {
     count_launch();
     const int bd = W >= 1024 ? 1024 : (W + 31) / 32 * 32;
-    k_fill_invalid<<<H, bd, 0, st>>>(disp, valid, W, H, scratch, out);
+    pdl(k_fill_invalid, H, bd, 0, st)(disp, valid, W, H, scratch, out);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }

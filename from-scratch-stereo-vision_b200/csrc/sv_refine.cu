@@ -30,6 +30,7 @@ __constant__ int c_dirs[8][2] = {{1, 0}, {-1, 0}, {0, 1}, {0, -1},
 // truncates toward zero: __double2int_rz.
 __global__ void k_base(const double *__restrict__ disp0, long N,
                        int32_t *__restrict__ base, int *flag) {
+    pdl_sync();
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < N;
          i += (long)gridDim.x * blockDim.x) {
         double d = disp0[i];
@@ -109,6 +110,7 @@ template <typename T>
 __global__ void __launch_bounds__(CT_W *CT_H)
     k_census(const T *__restrict__ img0, const T *__restrict__ img1, int W, int H,
              int rx, int ry, uint64_t *__restrict__ out0, uint64_t *__restrict__ out1) {
+    pdl_sync();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     census_tile<T>(blockIdx.z ? img1 : img0, W, H, rx, ry, blockIdx.z ? out1 : out0,
                    blockIdx.x * CT_W, blockIdx.y * CT_H, reinterpret_cast<T *>(smem_raw));
@@ -124,6 +126,7 @@ __global__ void k_band_costs(const uint64_t *__restrict__ cl,
                              const int32_t *__restrict__ base1, int W, long N,
                              int R, int K, int invalid, uint8_t *__restrict__ C0,
                              uint8_t *__restrict__ C1) {
+    pdl_sync();
     const int view = blockIdx.y;
     const uint64_t *ref = view ? cr : cl;
     const uint64_t *oth = view ? cl : cr;
@@ -191,6 +194,7 @@ __global__ void __launch_bounds__(256)
           const int32_t *__restrict__ base0, const int32_t *__restrict__ base1,
           int W, int H, int K, int P1, int P2, LT *__restrict__ Lout, int npaths,
           SgmTasks tasks) {
+    pdl_sync();
     const int lane = threadIdx.x & 31;
     const int gw = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5);
     if (gw >= tasks.start[tasks.nseg]) return;
@@ -409,6 +413,7 @@ __device__ __forceinline__ void l2r_row(const double *__restrict__ row, int W,
 __global__ void __launch_bounds__(256)
     k_left_to_right(const double *__restrict__ dl, int W, double *__restrict__ dr,
                     int32_t *__restrict__ base_r, int32_t *__restrict__ base_l, int *flag) {
+    pdl_sync();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int sbuf[32];
     const long r = (long)blockIdx.x * W;
@@ -478,6 +483,7 @@ __global__ void __launch_bounds__(256)
     k_lr_check(const double *__restrict__ dl, const double *__restrict__ drr,
                const double *__restrict__ disp0, int W, double tol,
                double *__restrict__ out, uint8_t *__restrict__ status) {
+    pdl_sync();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int sbuf[32];
     const long r = (long)blockIdx.x * W;
@@ -490,7 +496,7 @@ __global__ void __launch_bounds__(256)
 
 int launch_base(const double *disp0, long N, int32_t *base, int *flag,
                 cudaStream_t st) {
-    count_launch(); k_base<<<grid_for(N, 256), 256, 0, st>>>(disp0, N, base, flag);
+    count_launch(); pdl(k_base, grid_for(N, 256), 256, 0, st)(disp0, N, base, flag);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -502,15 +508,15 @@ int launch_census(const void *img0, const void *img1, int dtype, int W, int H,
     size_t cells = (size_t)(CT_W + 2 * rx) * (CT_H + 2 * ry);
     switch (dtype) {
     case SV_U8:
-        count_launch(); k_census<uint8_t><<<grd, blk, cells * 1, st>>>(
+        count_launch(); pdl(k_census<uint8_t>, grd, blk, cells * 1, st)(
             (const uint8_t *)img0, (const uint8_t *)img1, W, H, rx, ry, out0, out1);
         break;
     case SV_F32:
-        count_launch(); k_census<float><<<grd, blk, cells * 4, st>>>(
+        count_launch(); pdl(k_census<float>, grd, blk, cells * 4, st)(
             (const float *)img0, (const float *)img1, W, H, rx, ry, out0, out1);
         break;
     case SV_F64:
-        count_launch(); k_census<double><<<grd, blk, cells * 8, st>>>(
+        count_launch(); pdl(k_census<double>, grd, blk, cells * 8, st)(
             (const double *)img0, (const double *)img1, W, H, rx, ry, out0, out1);
         break;
     default:
@@ -527,7 +533,7 @@ int launch_band_costs(const uint64_t *cl, const uint64_t *cr, const int32_t *bas
     const long N = (long)W * H;
     const int K = 2 * R + 1;
     dim3 grd(grid_for(N * K, 256, 148 * 8), nviews);
-    count_launch(); k_band_costs<<<grd, 256, 0, st>>>(cl, cr, base0, base1, W, N, R, K, invalid, C0, C1);
+    count_launch(); pdl(k_band_costs, grd, 256, 0, st)(cl, cr, base0, base1, W, N, R, K, invalid, C0, C1);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -541,7 +547,7 @@ static int sgm_dispatch_lt(const uint8_t *C0, const uint8_t *C1, const int32_t *
                            cudaStream_t st) {
     long warps = tasks.start[tasks.nseg];
     int blocks = (int)((warps * 32 + 255) / 256);
-    count_launch(); k_sgm<V, LT, ADD><<<blocks, 256, 0, st>>>(C0, C1, b0, b1, W, H, K, P1, P2,
+    count_launch(); pdl(k_sgm<V, LT, ADD>, blocks, 256, 0, st)(C0, C1, b0, b1, W, H, K, P1, P2,
                                               (LT *)Lout, npaths, tasks);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -573,7 +579,7 @@ int launch_left_to_right(const double *dl, int W, int H, double *dr, int32_t *ba
         SV_CUDA_TRY(cudaFuncSetAttribute(k_left_to_right,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem));
-    count_launch(); k_left_to_right<<<H, 256, smem, st>>>(dl, W, dr, base_r, base_l, flag);
+    count_launch(); pdl(k_left_to_right, H, 256, smem, st)(dl, W, dr, base_r, base_l, flag);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -585,7 +591,7 @@ int launch_lr_check(const double *dl, const double *dr, const double *disp0, int
         SV_CUDA_TRY(cudaFuncSetAttribute(k_lr_check,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem));
-    count_launch(); k_lr_check<<<H, 256, smem, st>>>(dl, dr, disp0, W, tol, out, status);
+    count_launch(); pdl(k_lr_check, H, 256, smem, st)(dl, dr, disp0, W, tol, out, status);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -598,6 +604,7 @@ int launch_lr_check(const double *dl, const double *dr, const double *disp0, int
 // ====================================================================
 
 __global__ void __launch_bounds__(256) k_b_base(BatchTables t) {
+    pdl_sync();
     const int i = batch_find(t.px_blk, t.n, blockIdx.x);
     const BatchPair &P = t.pairs[i];
     const long N = (long)P.W * P.H;
@@ -617,6 +624,7 @@ __global__ void __launch_bounds__(256) k_b_base(BatchTables t) {
 }
 
 __global__ void __launch_bounds__(256) k_b_left_to_right(BatchTables t) {
+    pdl_sync();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int sbuf[32];
     const int i = batch_find(t.row_blk, t.n, blockIdx.x);
@@ -627,6 +635,7 @@ __global__ void __launch_bounds__(256) k_b_left_to_right(BatchTables t) {
 
 template <typename T>
 __global__ void __launch_bounds__(CT_W *CT_H) k_b_census(BatchTables t) {
+    pdl_sync();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int i = batch_find(t.tile_blk, t.n, blockIdx.x);
     const BatchPair &P = t.pairs[i];
@@ -639,6 +648,7 @@ __global__ void __launch_bounds__(CT_W *CT_H) k_b_census(BatchTables t) {
 }
 
 __global__ void __launch_bounds__(256) k_b_lr_check(BatchTables t) {
+    pdl_sync();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int sbuf[32];
     const int i = batch_find(t.row_blk, t.n, blockIdx.x);
@@ -650,21 +660,21 @@ __global__ void __launch_bounds__(256) k_b_lr_check(BatchTables t) {
 int launch_batch_front(const BatchTables &t, long long px_blocks, long long rows,
                        long long tiles, cudaStream_t st) {
     count_launch();
-    k_b_base<<<(unsigned)px_blocks, 256, 0, st>>>(t);
+    pdl(k_b_base, (unsigned)px_blocks, 256, 0, st)(t);
     const size_t row_smem = (size_t)t.maxW * (8 + 4 + 1) + 16;
     if (row_smem > 48 * 1024)
         SV_CUDA_TRY(cudaFuncSetAttribute(k_b_left_to_right,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)row_smem));
     count_launch();
-    k_b_left_to_right<<<(unsigned)rows, 256, row_smem, st>>>(t);
+    pdl(k_b_left_to_right, (unsigned)rows, 256, row_smem, st)(t);
     const size_t cells = (size_t)(CT_W + 2 * t.rx) * (CT_H + 2 * t.ry);
     const dim3 g((unsigned)tiles, 1, 2), blk(CT_W, CT_H);
     count_launch();
     switch (t.dtype) {
-    case SV_U8: k_b_census<uint8_t><<<g, blk, cells, st>>>(t); break;
-    case SV_F32: k_b_census<float><<<g, blk, cells * 4, st>>>(t); break;
-    case SV_F64: k_b_census<double><<<g, blk, cells * 8, st>>>(t); break;
+    case SV_U8: pdl(k_b_census<uint8_t>, g, blk, cells, st)(t); break;
+    case SV_F32: pdl(k_b_census<float>, g, blk, cells * 4, st)(t); break;
+    case SV_F64: pdl(k_b_census<double>, g, blk, cells * 8, st)(t); break;
     default: set_error("unknown image dtype %d", t.dtype); return SV_ERR_PARAM;
     }
     SV_LAUNCH_CHECK();
@@ -677,7 +687,7 @@ int launch_batch_back(const BatchTables &t, long long rows, cudaStream_t st) {
         SV_CUDA_TRY(cudaFuncSetAttribute(k_b_lr_check, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)row_smem));
     count_launch();
-    k_b_lr_check<<<(unsigned)rows, 256, row_smem, st>>>(t);
+    pdl(k_b_lr_check, (unsigned)rows, 256, row_smem, st)(t);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }

@@ -25,6 +25,7 @@ namespace sv {
 constexpr int SEL_LB = 4;              // values a thread loads before it histograms them
 
 __global__ void k_sel_init(SelState *s, long long rank, unsigned *hist) {
+    pdl_sync();
     sel_init_block(s, rank, hist);
 }
 
@@ -57,6 +58,7 @@ __device__ __forceinline__ void sel_pass_body(long blk, long nblk, const double 
 __global__ void __launch_bounds__(1024)
     k_sel_pass(const double *__restrict__ x, long n, int pass, SelState *__restrict__ s,
                unsigned *__restrict__ ghist) {
+    pdl_sync();
     sel_pass_body(blockIdx.x, gridDim.x, x, n, pass, s, ghist);
 }
 
@@ -64,6 +66,7 @@ __global__ void __launch_bounds__(1024)
 // pair's CTAs cover its W x H map).
 __global__ void __launch_bounds__(1024)
     k_b_sel_pass(NetLaunch L, const double *x, int pass, SelState *s, unsigned *ghist) {
+    pdl_sync();
     long long c;
     const int p = net_pair(L, c);
     const NetPair &P = L.pairs[p];
@@ -226,6 +229,7 @@ __device__ __forceinline__ void sel_compact_body(long blk, long nblk, const doub
 __global__ void __launch_bounds__(1024)
     k_sel_compact(const double *__restrict__ x, long n, SelState *__restrict__ s,
                   unsigned long long *__restrict__ cand, double *mirror) {
+    pdl_sync();
     sel_compact_body(blockIdx.x, gridDim.x, x, n, s, cand, mirror);
 }
 
@@ -233,6 +237,7 @@ __global__ void __launch_bounds__(1024)
 // The candidates follow the pair's two global histograms.
 __global__ void __launch_bounds__(1024)
     k_b_sel_compact(NetLaunch L, const double *x, SelState *s, unsigned *hist) {
+    pdl_sync();
     long long c;
     const int p = net_pair(L, c);
     const NetPair &P = L.pairs[p];
@@ -251,6 +256,7 @@ template <typename T>
 __global__ void __launch_bounds__(1024)
     k_sel_small(const T *__restrict__ x, long n, long long rank0, SelState *__restrict__ s,
                 double *mirror) {
+    pdl_sync();
     extern __shared__ __align__(16) unsigned long long keys[];
     __shared__ unsigned hist[SEL_NB];
     __shared__ unsigned wsum[32];
@@ -368,6 +374,7 @@ __device__ unsigned sel32_cta(const float *__restrict__ x, int n, unsigned rank0
 __global__ void __launch_bounds__(SEL32_T)
     k_sel_small_f32(const float *__restrict__ x, int n, unsigned rank0,
                     SelState *__restrict__ s, double *mirror) {
+    pdl_sync();
     const unsigned k = sel32_cta(x, n, rank0);
     if (threadIdx.x == 0) {
         const double v = (double)sel_unkey32(k);
@@ -382,6 +389,7 @@ __global__ void __launch_bounds__(SEL32_T)
 // pass's Ww x Hw values), rank int(0.95 n) as _peak takes it.
 __global__ void __launch_bounds__(SEL32_T)
     k_b_sel_probe(NetLaunch L, const float *x0, SelState *s0) {
+    pdl_sync();
     long long c;
     const int p = net_pair(L, c);
     const NetPair &P = L.pairs[p];
@@ -404,6 +412,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     k_width_map(const T *__restrict__ x, long n, WidthFuse f, SelState *s, unsigned *ghist,
                 double *mirror) {
+    pdl_sync();
     __shared__ unsigned hist[kWidthBins + 1];
     const int t = threadIdx.x;
     const long i = blockIdx.x * 256L + t;
@@ -423,6 +432,7 @@ constexpr long WIDTH_SMALL_CAP = (long)WIDTH_SMALL_T * WIDTH_SMALL_K;
 template <typename T>
 __global__ void __launch_bounds__(WIDTH_SMALL_T)
     k_width_small(const T *__restrict__ x, int n, WidthFuse f, SelState *s, double *mirror) {
+    pdl_sync();
     __shared__ unsigned hist[kWidthBins + 1];
     const int t = threadIdx.x;
     T v[WIDTH_SMALL_K];
@@ -452,6 +462,7 @@ __global__ void __launch_bounds__(WIDTH_SMALL_T)
 // Ww x Hw FP32 values, read from global memory), rule scale W / pw.
 __global__ void __launch_bounds__(WIDTH_SMALL_T)
     k_b_width_probe(NetLaunch L, const float *x0, SelState *s0, double target, int max_width) {
+    pdl_sync();
     __shared__ unsigned hist[kWidthBins + 1];
     long long c;
     const int p = net_pair(L, c);
@@ -477,7 +488,7 @@ __global__ void __launch_bounds__(WIDTH_SMALL_T)
 int launch_b_width_probe(const NetLaunch &L, const NetSlab &s, double target, int max_width,
                          cudaStream_t st) {
     count_launch();
-    k_b_width_probe<<<(unsigned)L.n, WIDTH_SMALL_T, 0, st>>>(L, s.d2, s.sel, target, max_width);
+    pdl(k_b_width_probe, (unsigned)L.n, WIDTH_SMALL_T, 0, st)(L, s.d2, s.sel, target, max_width);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -491,12 +502,12 @@ int launch_width_map(const T *x, long n, const WidthFuse &f, SelState *state, un
     }
     if (n <= WIDTH_SMALL_CAP) {
         count_launch();
-        k_width_small<T><<<1, WIDTH_SMALL_T, 0, st>>>(x, (int)n, f, state, mirror);
+        pdl(k_width_small<T>, 1, WIDTH_SMALL_T, 0, st)(x, (int)n, f, state, mirror);
     } else {
         count_launch();
-        k_sel_init<<<1, 1024, 0, st>>>(state, f.rank, hist);
+        pdl(k_sel_init, 1, 1024, 0, st)(state, f.rank, hist);
         count_launch();
-        k_width_map<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x, n, f, state, hist, mirror);
+        pdl(k_width_map<T>, (unsigned)((n + 255) / 256), 256, 0, st)(x, n, f, state, hist, mirror);
     }
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -539,22 +550,22 @@ int launch_select(const double *x, long n, long long rank, SelState *state, unsi
     }
     if (n <= SEL_SMALL_CAP) {
         count_launch();
-        k_sel_small<double><<<1, 1024, (size_t)n * sizeof(unsigned long long), st>>>(
+        pdl(k_sel_small<double>, 1, 1024, (size_t)n * sizeof(unsigned long long), st)(
             x, n, rank, state, mirror);
         SV_LAUNCH_CHECK();
         return SV_OK;
     }
     count_launch();
-    k_sel_init<<<1, 1024, 0, st>>>(state, rank, hist);       // also clears the histograms
+    pdl(k_sel_init, 1, 1024, 0, st)(state, rank, hist);       // also clears the histograms
     const int blocks = grid_for(n, 1024 * 4, 148);
     // the candidates follow the two global histograms (8-byte aligned)
     unsigned long long *cand = reinterpret_cast<unsigned long long *>(hist + 2 * SEL_NB);
     for (int p = 0; p < 2; ++p) {
         count_launch();
-        k_sel_pass<<<blocks, 1024, 0, st>>>(x, n, p, state, hist + (size_t)p * SEL_NB);
+        pdl(k_sel_pass, blocks, 1024, 0, st)(x, n, p, state, hist + (size_t)p * SEL_NB);
     }
     count_launch();
-    k_sel_compact<<<blocks, 1024, (size_t)SEL_CAND_CAP * sizeof(unsigned long long), st>>>(
+    pdl(k_sel_compact, blocks, 1024, (size_t)SEL_CAND_CAP * sizeof(unsigned long long), st)(
         x, n, state, cand, mirror);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -573,9 +584,9 @@ int launch_select_after_pass0(const double *x, long n, SelState *state, unsigned
     const int blocks = grid_for(n, 1024 * 4, 148);
     unsigned long long *cand = reinterpret_cast<unsigned long long *>(hist + 2 * SEL_NB);
     count_launch();
-    k_sel_pass<<<blocks, 1024, 0, st>>>(x, n, 1, state, hist + SEL_NB);
+    pdl(k_sel_pass, blocks, 1024, 0, st)(x, n, 1, state, hist + SEL_NB);
     count_launch();
-    k_sel_compact<<<blocks, 1024, (size_t)SEL_CAND_CAP * sizeof(unsigned long long), st>>>(
+    pdl(k_sel_compact, blocks, 1024, (size_t)SEL_CAND_CAP * sizeof(unsigned long long), st)(
         x, n, state, cand, mirror);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -583,7 +594,7 @@ int launch_select_after_pass0(const double *x, long n, SelState *state, unsigned
 
 int launch_b_sel_probe(const NetLaunch &L, const NetSlab &s, cudaStream_t st) {
     count_launch();
-    k_b_sel_probe<<<(unsigned)L.n, SEL32_T, 0, st>>>(L, s.d2, s.sel);
+    pdl(k_b_sel_probe, (unsigned)L.n, SEL32_T, 0, st)(L, s.d2, s.sel);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -595,9 +606,9 @@ int launch_b_sel_rest(const NetLaunch &L, long long total, const NetSlab &s, cud
     }
     const unsigned B = (unsigned)(total > 0 ? total : 1);
     count_launch();
-    k_b_sel_pass<<<B, 1024, 0, st>>>(L, s.full, 1, s.sel, s.hist + SEL_NB);
+    pdl(k_b_sel_pass, B, 1024, 0, st)(L, s.full, 1, s.sel, s.hist + SEL_NB);
     count_launch();
-    k_b_sel_compact<<<B, 1024, (size_t)SEL_CAND_CAP * sizeof(unsigned long long), st>>>(
+    pdl(k_b_sel_compact, B, 1024, (size_t)SEL_CAND_CAP * sizeof(unsigned long long), st)(
         L, s.full, s.sel, s.hist);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -617,7 +628,7 @@ int launch_select_small_f32(const float *x, long n, long long rank, SelState *st
     const int rc = select_setup();
     if (rc) return rc;
     count_launch();
-    k_sel_small_f32<<<1, SEL32_T, 0, st>>>(x, (int)n, (unsigned)rank, state, mirror);
+    pdl(k_sel_small_f32, 1, SEL32_T, 0, st)(x, (int)n, (unsigned)rank, state, mirror);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -630,6 +641,7 @@ size_t select_hist_words() { return 2 * (size_t)SEL_NB + 2 * (size_t)SEL_CAND_CA
 
 namespace {
 __global__ void k_peak_out(const sv::SelState *s, double *out) {
+    sv::pdl_sync();
     const double v = s->value;
     *out = v > 0.5 ? v : 0.5;
 }
@@ -661,7 +673,7 @@ int sv_peak(const double *disp, long n, double q, double *out, void *workspace,
     const int rc = sv::launch_select(disp, n, rank, s, hist, st);
     if (rc) return rc;
     sv::count_launch();
-    k_peak_out<<<1, 1, 0, st>>>(s, out);
+    sv::pdl(k_peak_out, 1, 1, 0, st)(s, out);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }

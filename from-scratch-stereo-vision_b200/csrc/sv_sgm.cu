@@ -191,6 +191,7 @@ __global__ void __launch_bounds__(256)
                       const int32_t *__restrict__ base0, const int32_t *__restrict__ base1, int W,
                       long N, int R, int K, int Kp, int invalid, uint8_t *__restrict__ C0,
                       uint8_t *__restrict__ C1, const uint8_t *__restrict__ rad0) {
+    pdl_sync();
     const int view = blockIdx.y;
     const uint64_t *ref = view ? cr : cl;
     const uint64_t *oth = view ? cl : cr;
@@ -568,6 +569,7 @@ __global__ void __launch_bounds__(SGM_WARPS * 32)
     k_sgm_scan(const uint8_t *__restrict__ C0, const uint8_t *__restrict__ C1,
                const int32_t *__restrict__ base0, const int32_t *__restrict__ base1, SgmPlan plan,
                int R, int K, int P1, int P2, LT *__restrict__ Lout) {
+    pdl_sync();
     constexpr int Kp = 2 * NR * GL;
     extern __shared__ __align__(16) unsigned char sgm_ring[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -790,6 +792,7 @@ __global__ void __launch_bounds__(256)
                const double *__restrict__ d00, const double *__restrict__ d01, double uniq,
                int want_conf, double *__restrict__ out0, double *__restrict__ out1,
                double *__restrict__ conf0) {
+    pdl_sync();
     constexpr int LPP = KP > 0 ? 1 : 8;                    // lanes per pixel
     const int row = path_row(KP > 0 ? KP : Kp, PAD);
     const long stride = N * row;                           // between path arrays
@@ -835,13 +838,13 @@ int launch_band_costs_slot(const uint64_t *cl, const uint64_t *cr, const int32_t
     const dim3 px(grid_for(N, Kp == 24 ? 256 : 256 / (Kp / 8), 148 * 8), nviews);
     count_launch();
     if (K == 21)    // R = 10, the refine_disparity default
-        k_band_costs_slot<true, 21><<<px, 256, 0, st>>>(cl, cr, base0, base1, W, N, R, K, Kp,
+        pdl(k_band_costs_slot<true, 21>, px, 256, 0, st)(cl, cr, base0, base1, W, N, R, K, Kp,
                                                         invalid, C0, C1, rad0);
     else if (Kp == 24)
-        k_band_costs_slot<true, 0><<<px, 256, 0, st>>>(cl, cr, base0, base1, W, N, R, K, Kp,
+        pdl(k_band_costs_slot<true, 0>, px, 256, 0, st)(cl, cr, base0, base1, W, N, R, K, Kp,
                                                        invalid, C0, C1, rad0);
     else
-        k_band_costs_slot<false, 0><<<px, 256, 0, st>>>(cl, cr, base0, base1, W, N, R, K, Kp,
+        pdl(k_band_costs_slot<false, 0>, px, 256, 0, st)(cl, cr, base0, base1, W, N, R, K, Kp,
                                                         invalid, C0, C1, rad0);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -861,7 +864,7 @@ static int sgm_go(const uint8_t *C0, const uint8_t *C1, const int32_t *b0, const
         SV_CUDA_TRY(cudaFuncSetAttribute(k_sgm_scan<NR, GL, LT, PAD>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     count_launch();
-    k_sgm_scan<NR, GL, LT, PAD><<<blocks, warps * 32, smem, st>>>(
+    pdl(k_sgm_scan<NR, GL, LT, PAD>, blocks, warps * 32, smem, st)(
         C0, C1, b0, b1, plan, (K - 1) / 2, K, P1, P2, (LT *)Lout);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -915,7 +918,7 @@ int launch_wta_slot(const void *L, bool l16, bool pad, int npaths, int nviews, i
         return SV_ERR_PARAM;
     }
 #define SV_WTA(LT, KP, PAD, NP, BLOCKS)                                                          \
-    k_wta_slot<LT, KP, PAD, NP><<<BLOCKS, 256, 0, st>>>((const LT *)L, npaths, nviews, N, K, Kp, \
+    pdl(k_wta_slot<LT, KP, PAD, NP>, BLOCKS, 256, 0, st)((const LT *)L, npaths, nviews, N, K, Kp, \
                                                         R, b0, b1, d00, d01, uniq,               \
                                                         conf0 != nullptr, out0, out1, conf0)
     const int blocks = grid_for(nviews * N, 256, 148 * 16);
@@ -946,6 +949,7 @@ int launch_wta_slot(const void *L, bool l16, bool pad, int npaths, int nviews, i
 // single-pair kernels (the whole batch shares K).
 template <bool KP24, int KC>
 __global__ void __launch_bounds__(256) k_b_costs(BatchTables t) {
+    pdl_sync();
     const int i = batch_find(t.px_blk, t.n, blockIdx.x);
     const BatchPair &P = t.pairs[i];
     const int view = blockIdx.y;
@@ -961,6 +965,7 @@ __global__ void __launch_bounds__(256) k_b_costs(BatchTables t) {
 
 template <int NR, int GL, typename LT, bool PAD>
 __global__ void __launch_bounds__(256) k_b_sgm(BatchTables t, long long total) {
+    pdl_sync();
     constexpr int SPW = 32 / GL;
     extern __shared__ __align__(16) unsigned char sgm_ring[];
     const int lane = threadIdx.x & 31;
@@ -994,6 +999,7 @@ __global__ void __launch_bounds__(256) k_b_sgm(BatchTables t, long long total) {
 
 template <typename LT, int KP, bool PAD, int NPC>
 __global__ void __launch_bounds__(256) k_b_wta(BatchTables t) {
+    pdl_sync();
     constexpr int LPP = KP > 0 ? 1 : 8;
     const int i = batch_find(t.px_blk, t.n, blockIdx.x);
     const BatchPair &P = t.pairs[i];
@@ -1040,7 +1046,7 @@ static int batch_sgm_go(const BatchTables &t, long long tasks, int threads, int 
         SV_CUDA_TRY(cudaFuncSetAttribute(k_b_sgm<NR, GL, LT, PAD>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     count_launch();
-    k_b_sgm<NR, GL, LT, PAD><<<blocks, threads, smem, st>>>(t, tasks);
+    pdl(k_b_sgm<NR, GL, LT, PAD>, blocks, threads, smem, st)(t, tasks);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -1052,9 +1058,9 @@ int launch_batch_refine(const BatchTables &t, long long px_blocks, long long row
     if (rc) return rc;
     const dim3 px((unsigned)px_blocks, 2);
     count_launch();
-    if (t.K == 21) k_b_costs<true, 21><<<px, 256, 0, st>>>(t);    // R = 10
-    else if (t.Kp == 24) k_b_costs<true, 0><<<px, 256, 0, st>>>(t);
-    else k_b_costs<false, 0><<<px, 256, 0, st>>>(t);
+    if (t.K == 21) pdl(k_b_costs<true, 21>, px, 256, 0, st)(t);    // R = 10
+    else if (t.Kp == 24) pdl(k_b_costs<true, 0>, px, 256, 0, st)(t);
+    else pdl(k_b_costs<false, 0>, px, 256, 0, st)(t);
     SV_LAUNCH_CHECK();
 #define SV_BGO(KP, NR, GL)                                                                   \
     case KP:                                                                                 \
@@ -1075,12 +1081,12 @@ int launch_batch_refine(const BatchTables &t, long long px_blocks, long long row
 #undef SV_BGO
     if (rc) return rc;
     count_launch();
-    if (l16) k_b_wta<uint16_t, 0, false, 0><<<px, 256, 0, st>>>(t);
-    else if (t.Kp == 24 && t.npaths == 8) k_b_wta<uint8_t, 24, true, 8><<<px, 256, 0, st>>>(t);
-    else if (t.Kp == 24) k_b_wta<uint8_t, 24, true, 0><<<px, 256, 0, st>>>(t);
-    else if (t.Kp == 8) k_b_wta<uint8_t, 8, true, 0><<<px, 256, 0, st>>>(t);
-    else if (t.Kp == 16) k_b_wta<uint8_t, 16, true, 0><<<px, 256, 0, st>>>(t);
-    else k_b_wta<uint8_t, 32, true, 0><<<px, 256, 0, st>>>(t);
+    if (l16) pdl(k_b_wta<uint16_t, 0, false, 0>, px, 256, 0, st)(t);
+    else if (t.Kp == 24 && t.npaths == 8) pdl(k_b_wta<uint8_t, 24, true, 8>, px, 256, 0, st)(t);
+    else if (t.Kp == 24) pdl(k_b_wta<uint8_t, 24, true, 0>, px, 256, 0, st)(t);
+    else if (t.Kp == 8) pdl(k_b_wta<uint8_t, 8, true, 0>, px, 256, 0, st)(t);
+    else if (t.Kp == 16) pdl(k_b_wta<uint8_t, 16, true, 0>, px, 256, 0, st)(t);
+    else pdl(k_b_wta<uint8_t, 32, true, 0>, px, 256, 0, st)(t);
     SV_LAUNCH_CHECK();
     return launch_batch_back(t, rows, st);
 }

@@ -140,6 +140,7 @@ __device__ __forceinline__ void c3_gather(const unsigned char *b0, const unsigne
 // ICT: the channel count, 0 to read it from the arguments; MODE: a.mode
 template <int ICT, int MODE>
 __global__ void __launch_bounds__(kC3Threads) k_conv3d_tc(TcConv a, int per_cta) {
+    pdl_sync();
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_slot;
@@ -384,6 +385,7 @@ constexpr int kT2W = 32, kT2H = 4;
 constexpr int kT2Cols = 3;              // patch columns per lane: PW <= 96
 
 __global__ void __launch_bounds__(kTcM) k_conv2d_tc(TcConv a, int PH, int PW) {
+    pdl_sync();
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_slot;
@@ -569,6 +571,7 @@ constexpr int kTapCtas = 5;             // resident CTAs per SM (registers)
 // before the first packing and the counts known take 21 us.
 template <int ICT, int OCT, int ACT>
 __global__ void __launch_bounds__(kTcM, kTapCtas) k_conv2d_tc_tap(TcConv a, int PWp) {
+    pdl_sync();
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_slot;
@@ -771,17 +774,17 @@ static int launch_conv2d_tc(const TcConv &a, cudaStream_t st) {
         count_launch();
         // FeatureNet c3 / c4 of the shipped checkpoint and the band net's layers
         if (a.IC == 12 && a.OC == 12 && a.act == 1)
-            k_conv2d_tc_tap<12, 12, 1><<<blocks, kTcM, smem, st>>>(a, PWp);
+            pdl(k_conv2d_tc_tap<12, 12, 1>, blocks, kTcM, smem, st)(a, PWp);
         else if (a.IC == 12 && a.OC == 12 && a.act == 0)
-            k_conv2d_tc_tap<12, 12, 0><<<blocks, kTcM, smem, st>>>(a, PWp);
+            pdl(k_conv2d_tc_tap<12, 12, 0>, blocks, kTcM, smem, st)(a, PWp);
         else if (a.IC == 8 && a.OC == 16 && a.act == 1)
-            k_conv2d_tc_tap<8, 16, 1><<<blocks, kTcM, smem, st>>>(a, PWp);
+            pdl(k_conv2d_tc_tap<8, 16, 1>, blocks, kTcM, smem, st)(a, PWp);
         else if (a.IC == 16 && a.OC == 16 && a.act == 1)
-            k_conv2d_tc_tap<16, 16, 1><<<blocks, kTcM, smem, st>>>(a, PWp);
+            pdl(k_conv2d_tc_tap<16, 16, 1>, blocks, kTcM, smem, st)(a, PWp);
         else if (a.IC == 16 && a.OC == 2 && a.act == 0)
-            k_conv2d_tc_tap<16, 2, 0><<<blocks, kTcM, smem, st>>>(a, PWp);
+            pdl(k_conv2d_tc_tap<16, 2, 0>, blocks, kTcM, smem, st)(a, PWp);
         else
-            k_conv2d_tc_tap<0, 0, -1><<<blocks, kTcM, smem, st>>>(a, PWp);
+            pdl(k_conv2d_tc_tap<0, 0, -1>, blocks, kTcM, smem, st)(a, PWp);
         SV_LAUNCH_CHECK();
         return SV_OK;
     }
@@ -803,7 +806,7 @@ static int launch_conv2d_tc(const TcConv &a, cudaStream_t st) {
     const long cap = (long)sms * tc_ctas_per_sm(smem);
     const unsigned blocks = (unsigned)(tiles < cap ? tiles : cap);
     count_launch();
-    k_conv2d_tc<<<blocks, kTcM, smem, st>>>(a, PH, PW);
+    pdl(k_conv2d_tc, blocks, kTcM, smem, st)(a, PH, PW);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -815,6 +818,7 @@ static int launch_conv2d_tc(const TcConv &a, cudaStream_t st) {
 // return, leaving the context usable.  done receives 1 once the CTA has
 // passed its dealloc.
 __global__ void __launch_bounds__(kTcM) k_selftest_wait(unsigned limit, int *flag, int *done) {
+    pdl_sync();
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_slot;
     __shared__ int failed;
@@ -848,7 +852,7 @@ __global__ void __launch_bounds__(kTcM) k_selftest_wait(unsigned limit, int *fla
 
 int launch_selftest_wait(unsigned limit, int *flag, int *done, cudaStream_t st) {
     count_launch();
-    k_selftest_wait<<<1, kTcM, 0, st>>>(limit, flag, done);
+    pdl(k_selftest_wait, 1, kTcM, 0, st)(limit, flag, done);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -892,7 +896,7 @@ int launch_conv_tc(const TcConv &a, cudaStream_t st) {
     const int per = (int)((steps + cap - 1) / cap);
     const unsigned blocks = (unsigned)((steps + per - 1) / per);
     count_launch();
-    f<<<blocks, kC3Threads, smem, st>>>(a, per);
+    pdl(f, blocks, kC3Threads, smem, st)(a, per);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
@@ -908,6 +912,7 @@ int launch_conv_tc(const TcConv &a, cudaStream_t st) {
 constexpr int kWgK = 64;
 
 __global__ void __launch_bounds__(kTcM) k_wgrad_tc(TcWgrad a, int mtiles) {
+    pdl_sync();
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t tmem_slot;
@@ -1091,13 +1096,14 @@ int launch_wgrad_tc(const TcWgrad &a, cudaStream_t st) {
     const long cap = (long)sms * 2;
     const unsigned blocks = (unsigned)(chunks < cap ? chunks : cap);
     count_launch();
-    k_wgrad_tc<<<blocks, kTcM, smem, st>>>(a, mtiles);
+    pdl(k_wgrad_tc, blocks, kTcM, smem, st)(a, mtiles);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
 
 __global__ void k_pack_weights(const float *__restrict__ w, int OC, int IC, int transpose,
                                int K, int Kpad, uint16_t *__restrict__ out) {
+    pdl_sync();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= kTcN * Kpad) return;
     const int n = i / Kpad, k = i - (i / Kpad) * Kpad;
@@ -1122,7 +1128,7 @@ int launch_pack_weights(const float *w, int OC, int IC, int transpose, uint16_t 
     }
     const int Kpad = tc_kpad(K);
     count_launch();
-    k_pack_weights<<<(kTcN * Kpad + 255) / 256, 256, 0, st>>>(w, OC, IC, transpose, K, Kpad,
+    pdl(k_pack_weights, (kTcN * Kpad + 255) / 256, 256, 0, st)(w, OC, IC, transpose, K, Kpad,
                                                               out);
     SV_LAUNCH_CHECK();
     return SV_OK;

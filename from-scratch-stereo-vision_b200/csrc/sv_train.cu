@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(8 * TR, OC <= 8 ? 6 : 1)
     k_tconv2d(const float *__restrict__ x, int H, int W, int OH, int OW, int dil_,
               const float *__restrict__ w, const float *__restrict__ b, float *__restrict__ y,
               const float *__restrict__ aux, long aux_stride) {
+    pdl_sync();
     constexpr int OCP = OC >= 4 ? (OC + 3) / 4 * 4 : OC, NT = 8 * TR;
     static_assert(!FLIP || S == 1, "flipped taps: stride 1");
     extern __shared__ __align__(16) float tile[];
@@ -250,6 +251,7 @@ __global__ void __launch_bounds__(128)
     k_tconv3d(const float *__restrict__ x, int D, int h, int w,
               const float *__restrict__ wt, const float *__restrict__ b, float *__restrict__ y,
               const float *__restrict__ xin) {
+    pdl_sync();
     constexpr int OCP = OC >= 2 ? (OC + 1) / 2 * 2 : OC;
     static_assert(IC % CCH == 0, "channel chunks");
     extern __shared__ __align__(16) float tile[];      // [CCH][D + 2][3][rs]
@@ -373,6 +375,7 @@ __global__ void __launch_bounds__(128)
 __global__ void __launch_bounds__(256)
     k_tcostvol(const float *__restrict__ f, int B, int C, int D, int h, int w,
                float *__restrict__ vol) {
+    pdl_sync();
     // one (sample, channel) per CTA; a warp takes whole rows of one disparity
     const int hw = h * w, bc = blockIdx.x, b = bc / C, c = bc - b * C;
     const float *l = f + ((long)b * C + c) * hw, *r = f + ((long)(B + b) * C + c) * hw;
@@ -388,6 +391,7 @@ __global__ void __launch_bounds__(256)
 // and disparity, FP32 with max-subtraction.
 __global__ void k_tsoftargmin(const float *__restrict__ cost, int B, int D, int h, int w,
                               float *__restrict__ probs, float *__restrict__ d0) {
+    pdl_sync();
     const long hw = (long)h * w;
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i >= B * hw) return;
@@ -420,6 +424,7 @@ __global__ void k_tsoftargmin(const float *__restrict__ cost, int B, int D, int 
 // A refinement level's input [b][2][H2][W2]: 2 * bilinear(prev), guide.
 __global__ void k_tupcat(const float *__restrict__ prev, int B, int h, int w, int H2, int W2,
                          const float *__restrict__ guide, float *__restrict__ rin) {
+    pdl_sync();
     const long n2 = (long)H2 * W2;
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i >= B * n2) return;
@@ -439,6 +444,7 @@ __global__ void k_tupcat(const float *__restrict__ prev, int B, int h, int w, in
 __global__ void k_tpool(const float *__restrict__ d, const uint8_t *__restrict__ v,
                         const float *__restrict__ g, int B, int H, int W, float *__restrict__ dd,
                         uint8_t *__restrict__ vv, float *__restrict__ gg) {
+    pdl_sync();
     const int H2 = H / 2, W2 = W / 2;
     const long n2 = (long)H2 * W2;
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -469,6 +475,7 @@ __global__ void __launch_bounds__(256)
     k_tcounts(const uint8_t *__restrict__ vq, const uint8_t *__restrict__ vh,
               const uint8_t *__restrict__ vf, const float *__restrict__ dq, long n4, long n2,
               long n1, int D, int *__restrict__ counts) {
+    pdl_sync();
     __shared__ int s[4][256];
     const int b = blockIdx.x, t = threadIdx.x;
     int c0 = 0, c1 = 0, c2 = 0, c3 = 0;
@@ -496,6 +503,7 @@ __global__ void k_thuber(const float *__restrict__ pred, const float *__restrict
                          const uint8_t *__restrict__ valid, int B, long n,
                          const int *__restrict__ counts, int lv, float wgt, float invB,
                          float *__restrict__ g, float *__restrict__ term) {
+    pdl_sync();
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i >= B * n) return;
     const int b = (int)(i / n);
@@ -518,6 +526,7 @@ __global__ void k_tsoft_bwd(const float *__restrict__ probs, const float *__rest
                             const uint8_t *__restrict__ vq, const int *__restrict__ counts,
                             int B, int D, long hw, float ce_w, float invB,
                             float *__restrict__ gcost, float *__restrict__ term) {
+    pdl_sync();
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i >= B * hw) return;
     const int b = (int)(i / hw);
@@ -563,6 +572,7 @@ __global__ void __launch_bounds__(256)
     k_tloss(const float *__restrict__ t0, const float *__restrict__ t1,
             const float *__restrict__ t2, const float *__restrict__ tce, long n4, long n2,
             long n1, const int *__restrict__ counts, double *__restrict__ loss) {
+    pdl_sync();
     __shared__ double s[4][256];
     const int b = blockIdx.x, t = threadIdx.x;
     double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
@@ -591,6 +601,7 @@ __global__ void __launch_bounds__(256)
 // Refinement output ReLU (slope 0): g where the output is positive.
 __global__ void k_tmask0(const float *__restrict__ g, const float *__restrict__ out, long n,
                          float *__restrict__ gs) {
+    pdl_sync();
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i < n) gs[i] = out[i] > 0.f ? g[i] : 0.f;
 }
@@ -604,6 +615,7 @@ __global__ void __launch_bounds__(128)
     k_tdgrad2d_s2(const float *__restrict__ gy, int nimg, int H, int W, int OH, int OW,
                   const float *__restrict__ w, const float *__restrict__ xin,
                   float *__restrict__ gx) {
+    pdl_sync();
     constexpr int ICP = (IC + 3) / 4 * 4;
     __shared__ __align__(16) float sw[OC * 9 * ICP];       // [o][tap][c]
     for (int i = threadIdx.x; i < OC * 9 * ICP; i += blockDim.x) {
@@ -819,6 +831,7 @@ template <int IC, int OC, int S, int DIL>
 __global__ void __launch_bounds__(kWgThreads)
     k_twgrad2d(const float *__restrict__ x, const float *__restrict__ gy, int nimg, int H, int W,
                int OH, int OW, int dil_, float *__restrict__ partial) {
+    pdl_sync();
     using G = WgSplit<OC, IC * 3 + 1>;
     using Rw = WgRow<S, DIL>;
     constexpr int K = IC * 9 + 1;
@@ -903,6 +916,7 @@ template <int IC, int OC>
 __global__ void __launch_bounds__(kWgThreads)
     k_twgrad3d(const float *__restrict__ x, const float *__restrict__ gy, int B, int D, int h,
                int w, float *__restrict__ partial) {
+    pdl_sync();
     using G = typename Wg3<IC, OC>::G;
     using Rw = typename Wg3<IC, OC>::Rw;
     constexpr int K = Wg3<IC, OC>::K;
@@ -974,6 +988,7 @@ struct ReduceJobs {
 
 __global__ void __launch_bounds__(1024)
     k_treduce(const float *__restrict__ partials, ReduceJobs jobs, double *__restrict__ grads) {
+    pdl_sync();
     __shared__ double rs[32][33];
     int l = 0;
     while ((int)blockIdx.x >= jobs.block[l + 1]) ++l;
@@ -997,6 +1012,7 @@ __global__ void __launch_bounds__(1024)
 // gradient times sign(fl - fr(x - d)); gfr[c][y][x] subtracts it at x + d.
 __global__ void k_tcostvol_bwd(const float *__restrict__ gvol, const float *__restrict__ f,
                                int B, int C, int D, int h, int w, float *__restrict__ gf) {
+    pdl_sync();
     const long hw = (long)h * w, n = (long)B * C * hw;
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -1033,6 +1049,7 @@ __global__ void k_tup_bwd(const float *__restrict__ grin, long grin_stride,
                           const float *__restrict__ gs, int B, int H2, int W2, int h, int w,
                           int ry, int rx, const float *__restrict__ add,
                           const float *__restrict__ mask, float *__restrict__ out) {
+    pdl_sync();
     const long hw = (long)h * w, n2 = (long)H2 * W2;
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i >= B * hw) return;
@@ -1095,6 +1112,7 @@ __global__ void k_tup_bwd(const float *__restrict__ grin, long grin_stride,
 __global__ void k_tadam(double *__restrict__ p, const double *__restrict__ g,
                         double *__restrict__ m, double *__restrict__ v, long n, double lr,
                         double c1, double c2, double clip, float *__restrict__ p32) {
+    pdl_sync();
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double b1 = 0.9, b2 = 0.999, eps = 1.0e-8;
@@ -1111,6 +1129,7 @@ __global__ void k_tadam(double *__restrict__ p, const double *__restrict__ g,
 }
 
 __global__ void k_f64_to_f32(const double *__restrict__ a, long n, float *__restrict__ b) {
+    pdl_sync();
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i < n) b[i] = (float)a[i];
 }
@@ -1271,7 +1290,7 @@ int conv2d_go(const float *x, int nimg, int H, int W, int OH, int OW, int dil, c
     if (rc) return rc;
     const dim3 g((OW + 31) / 32, (OH + TR - 1) / TR, nimg);
     count_launch();
-    k_tconv2d<IC, OC, WC, S, DIL, MODE, FLIP, TR><<<g, 8 * TR, sm, st>>>(x, H, W, OH, OW, dil, w, b,
+    pdl(k_tconv2d<IC, OC, WC, S, DIL, MODE, FLIP, TR>, g, 8 * TR, sm, st)(x, H, W, OH, OW, dil, w, b,
                                                                          y, aux, stride);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -1302,7 +1321,7 @@ int conv3d_go(const float *x, int B, int D, int h, int w, const float *wt, const
     if (rc) return rc;
     const dim3 g((w + 4 * nxg - 1) / (4 * nxg), h, B);
     count_launch();
-    k_tconv3d<IC, OC, WC, CCH, MODE, FLIP, nxg><<<g, (nxg * D + 31) / 32 * 32, sm, st>>>(
+    pdl(k_tconv3d<IC, OC, WC, CCH, MODE, FLIP, nxg>, g, (nxg * D + 31) / 32 * 32, sm, st)(
         x, D, h, w, wt, b, y, xin);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -1338,7 +1357,7 @@ int wgrad2d_go(const float *x, const float *gy, int nimg, int H, int W, int OH, 
     const int nblk = (int)(ntiles < kWgCtas ? ntiles : kWgCtas);
     const int l = g.add(nblk, OC, IC * 9 + 1, gw, gb);
     count_launch();
-    k_twgrad2d<IC, OC, S, DIL><<<nblk, kWgThreads, sm, st>>>(x, gy, nimg, H, W, OH, OW, dil,
+    pdl(k_twgrad2d<IC, OC, S, DIL>, nblk, kWgThreads, sm, st)(x, gy, nimg, H, W, OH, OW, dil,
                                                              g.partial + g.jobs.partial[l]);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -1369,7 +1388,7 @@ int wgrad3d(const float *x, const float *gy, int B, int D, int h, int w, WGrads 
     const int nblk = (int)(ntiles < kWgCtas ? ntiles : kWgCtas);
     const int l = g.add(nblk, OC, Gm::K, gw, gb);
     count_launch();
-    k_twgrad3d<IC, OC><<<nblk, kWgThreads, Gm::SMEM, st>>>(x, gy, B, D, h, w,
+    pdl(k_twgrad3d<IC, OC>, nblk, kWgThreads, Gm::SMEM, st)(x, gy, B, D, h, w,
                                                        g.partial + g.jobs.partial[l]);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -1396,12 +1415,12 @@ int train_impl(sv_trainer *t, const float *left, const float *right, const float
     }
     // ---- targets (build_targets) and counts
     count_launch();
-    k_tpool<<<nblocks(B * d.HW2), 256, 0, st>>>(disp, valid, left, B, d.H, d.W, b.dh, b.vh, b.gh);
+    pdl(k_tpool, nblocks(B * d.HW2), 256, 0, st)(disp, valid, left, B, d.H, d.W, b.dh, b.vh, b.gh);
     count_launch();
-    k_tpool<<<nblocks(B * d.hw), 256, 0, st>>>(b.dh, b.vh, nullptr, B, d.H2, d.W2, b.dq, b.vq,
+    pdl(k_tpool, nblocks(B * d.hw), 256, 0, st)(b.dh, b.vh, nullptr, B, d.H2, d.W2, b.dq, b.vq,
                                                nullptr);
     count_launch();
-    k_tcounts<<<B, 256, 0, st>>>(b.vq, b.vh, valid, b.dq, d.hw, d.HW2, d.HW, D, b.counts);
+    pdl(k_tcounts, B, 256, 0, st)(b.vq, b.vh, valid, b.dq, d.hw, d.HW2, d.HW, D, b.counts);
     SV_LAUNCH_CHECK();
     // ---- forward: FeatureNet on 2B images
     if ((rc = conv2d_go<1, C, C, 2, 1, 1, false, 16>(b.img, 2 * B, d.H, d.W, d.h1, d.w1, 1,
@@ -1419,7 +1438,7 @@ int train_impl(sv_trainer *t, const float *left, const float *right, const float
                                            P + t->off_fb[3], b.f4, nullptr, 0, st)))
         return rc;
     count_launch();
-    k_tcostvol<<<dim3(B * C, (D * d.h + 63) / 64), 256, 0, st>>>(b.f4, B, C, D, d.h, d.w, b.vol);
+    pdl(k_tcostvol, dim3(B * C, (D * d.h + 63) / 64), 256, 0, st)(b.f4, B, C, D, d.h, d.w, b.vol);
     SV_LAUNCH_CHECK();
     if ((rc = conv3d_go<C, CM, CM, CH, 1, false>(b.vol, B, D, d.h, d.w, P + t->off_cw[0],
                                                  P + t->off_cb[0], b.b1, nullptr, st)))
@@ -1431,7 +1450,7 @@ int train_impl(sv_trainer *t, const float *left, const float *right, const float
                                                  P + t->off_cb[2], b.cost, nullptr, st)))
         return rc;
     count_launch();
-    k_tsoftargmin<<<nblocks(B * d.hw), 256, 0, st>>>(b.cost, B, D, d.h, d.w, b.probs, b.d0);
+    pdl(k_tsoftargmin, nblocks(B * d.hw), 256, 0, st)(b.cost, B, D, d.h, d.w, b.probs, b.d0);
     SV_LAUNCH_CHECK();
     // ---- refinement levels
     const int Hs[2] = {d.H2, d.H}, Ws[2] = {d.W2, d.W};
@@ -1442,7 +1461,7 @@ int train_impl(sv_trainer *t, const float *left, const float *right, const float
     for (int lv = 0; lv < 2; ++lv) {
         const int Hl = Hs[lv], Wl = Ws[lv];
         count_launch();
-        k_tupcat<<<nblocks(B * HWl[lv]), 256, 0, st>>>(prev, B, ph, pw, Hl, Wl, guides[lv],
+        pdl(k_tupcat, nblocks(B * HWl[lv]), 256, 0, st)(prev, B, ph, pw, Hl, Wl, guides[lv],
                                                        b.rin[lv]);
         const float *cur = b.rin[lv];
         for (int i = 0; i < nd; ++i) {
@@ -1466,20 +1485,20 @@ int train_impl(sv_trainer *t, const float *left, const float *right, const float
     }
     // ---- losses
     count_launch();
-    k_thuber<<<nblocks(B * d.hw), 256, 0, st>>>(b.d0, b.dq, b.vq, B, d.hw, b.counts, 0, 0.5f,
+    pdl(k_thuber, nblocks(B * d.hw), 256, 0, st)(b.d0, b.dq, b.vq, B, d.hw, b.counts, 0, 0.5f,
                                                 invB, b.gl0, b.t0);
     count_launch();
-    k_thuber<<<nblocks(B * d.HW2), 256, 0, st>>>(b.out[0], b.dh, b.vh, B, d.HW2, b.counts, 1,
+    pdl(k_thuber, nblocks(B * d.HW2), 256, 0, st)(b.out[0], b.dh, b.vh, B, d.HW2, b.counts, 1,
                                                  0.7f, invB, b.gl1, b.t1);
     count_launch();
-    k_thuber<<<nblocks(B * d.HW), 256, 0, st>>>(b.out[1], disp, valid, B, d.HW, b.counts, 2,
+    pdl(k_thuber, nblocks(B * d.HW), 256, 0, st)(b.out[1], disp, valid, B, d.HW, b.counts, 2,
                                                 1.0f, invB, b.gl2, b.t2);
     SV_LAUNCH_CHECK();
     // ---- backward: refinement levels, fine to coarse.  gsl[lv] is the
     // gradient on level lv's output after its ReLU (Refinement.backward's g).
     float *gsl[2] = {b.gs0, b.gs};
     count_launch();
-    k_tmask0<<<nblocks(B * d.HW), 256, 0, st>>>(b.gl2, b.out[1], B * d.HW, gsl[1]);
+    pdl(k_tmask0, nblocks(B * d.HW), 256, 0, st)(b.gl2, b.out[1], B * d.HW, gsl[1]);
     for (int lv = 1; lv >= 0; --lv) {
         const int Hl = Hs[lv], Wl = Ws[lv];
         const float *gs = gsl[lv];
@@ -1515,14 +1534,14 @@ int train_impl(sv_trainer *t, const float *left, const float *right, const float
         const int sh = lv ? d.H2 : d.h, sw = lv ? d.W2 : d.w;
         const int ry = (int)ceil(2.0 * Hl / sh) + 2, rx = (int)ceil(2.0 * Wl / sw) + 2;
         count_launch();
-        k_tup_bwd<<<nblocks((long)B * sh * sw), 256, 0, st>>>(
+        pdl(k_tup_bwd, nblocks((long)B * sh * sw), 256, 0, st)(
             b.grin, HWl[lv], gs, B, Hl, Wl, sh, sw, ry, rx, lv ? b.gl1 : b.gl0,
             lv ? b.out[0] : nullptr, lv ? gsl[0] : b.gd0);
         SV_LAUNCH_CHECK();
     }
     // ---- soft-argmin + cross-entropy, cost filter, cost volume
     count_launch();
-    k_tsoft_bwd<<<nblocks(B * d.hw), 256, 0, st>>>(b.probs, b.d0, b.gd0, b.dq, b.vq, b.counts, B,
+    pdl(k_tsoft_bwd, nblocks(B * d.hw), 256, 0, st)(b.probs, b.d0, b.gd0, b.dq, b.vq, b.counts, B,
                                                    D, d.hw, 2.0f, invB, b.gcost, b.tce);
     if ((rc = wgrad3d<CM, 1>(b.b2, b.gcost, B, D, d.h, d.w, wg, t->off_cw[2], t->off_cb[2], st)))
         return rc;
@@ -1540,7 +1559,7 @@ int train_impl(sv_trainer *t, const float *left, const float *right, const float
                                                 b.gvol, nullptr, st)))
         return rc;
     count_launch();
-    k_tcostvol_bwd<<<nblocks((long)B * C * d.hw), 256, 0, st>>>(b.gvol, b.f4, B, C, D, d.h, d.w,
+    pdl(k_tcostvol_bwd, nblocks((long)B * C * d.hw), 256, 0, st)(b.gvol, b.f4, B, C, D, d.h, d.w,
                                                                 b.gf);
     SV_LAUNCH_CHECK();
     // ---- FeatureNet, both towers as one batch of 2B images
@@ -1560,18 +1579,18 @@ int train_impl(sv_trainer *t, const float *left, const float *right, const float
                                t->off_fb[1], st)))
         return rc;
     count_launch();
-    k_tdgrad2d_s2<C, C><<<nblocks(2L * B * ((d.h1 + 1) / 2) * ((d.w1 + 1) / 2), 128), 128, 0, st>>>(
+    pdl(k_tdgrad2d_s2<C, C>, nblocks(2L * B * ((d.h1 + 1) / 2) * ((d.w1 + 1) / 2), 128), 128, 0, st)(
         b.gf, 2 * B, d.h1, d.w1, d.h, d.w, P + t->off_fw[1], b.a1, b.gF3);
     SV_LAUNCH_CHECK();
     if ((rc = wgrad2d<1, C, 2>(b.img, b.gF3, 2 * B, d.H, d.W, d.h1, d.w1, 1, wg, t->off_fw[0],
                                t->off_fb[0], st)))
         return rc;
     count_launch();
-    k_treduce<<<wg.jobs.block[wg.jobs.n], dim3(32, 32), 0, st>>>(b.partial, wg.jobs, t->g64);
+    pdl(k_treduce, wg.jobs.block[wg.jobs.n], dim3(32, 32), 0, st)(b.partial, wg.jobs, t->g64);
     SV_LAUNCH_CHECK();
     // ---- per-sample loss and the prediction
     count_launch();
-    k_tloss<<<B, 256, 0, st>>>(b.t0, b.t1, b.t2, b.tce, d.hw, d.HW2, d.HW, b.counts,
+    pdl(k_tloss, B, 256, 0, st)(b.t0, b.t1, b.t2, b.tce, d.hw, d.HW2, d.HW, b.counts,
                                loss ? loss : b.loss);
     SV_LAUNCH_CHECK();
     if (pred && cudaMemcpyAsync(pred, b.out[1], sizeof(float) * B * d.HW,
@@ -1748,7 +1767,7 @@ int sv_train_adam(sv_trainer *t, double lr, double clip, void *stream) {
     t->b2t *= 0.999;
     const double c1 = 1.0 / (1.0 - t->b1t), c2 = 1.0 / (1.0 - t->b2t);
     count_launch();
-    k_tadam<<<nblocks(t->np), 256, 0, (cudaStream_t)stream>>>(t->p64, t->g64, t->m, t->v, t->np,
+    pdl(k_tadam, nblocks(t->np), 256, 0, (cudaStream_t)stream)(t->p64, t->g64, t->m, t->v, t->np,
                                                                 lr, c1, c2, clip, t->p32);
     SV_LAUNCH_CHECK();
     return SV_OK;
