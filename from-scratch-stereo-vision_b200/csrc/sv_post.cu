@@ -124,25 +124,26 @@ __global__ void k_slic_init(const double *__restrict__ rgb, int W, int step, int
 }
 
 __global__ void k_slic_reset(long N, unsigned long long *__restrict__ dist,
-                             int *__restrict__ labtmp, int *__restrict__ flag) {
+                             int *__restrict__ labtmp) {
     pdl_sync();
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (i == 0) *flag = 0;
     if (i >= N) return;
     dist[i] = (unsigned long long)__double_as_longlong(1.0e30);
     labtmp[i] = INT_MAX;
 }
 
-// pass 0: atomicMin of the distance bits; pass 1: cluster index at the minimum
+// pass 0: atomicMin of the distance bits, and the cluster's window; pass 1: cluster
+// index at the minimum
 __global__ void __launch_bounds__(256)
     k_slic_assign(const double *__restrict__ rgb, int W, int H, int step, double m2,
                   const SlicCenter *__restrict__ cs, int pass, unsigned long long *__restrict__ dist,
-                  int *__restrict__ labtmp) {
+                  int *__restrict__ labtmp, int4 *__restrict__ win) {
     pdl_sync();
     const int ci = blockIdx.x;
     const SlicCenter c = cs[ci];
     const int4 w = slic_window(c, step, W, H);
     const int ww = w.y - w.x + 1, n = ww * (w.w - w.z + 1);
+    if (pass == 0 && threadIdx.x == 0) win[ci] = w;
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
         const int yy = w.z + t / ww, xx = w.x + t % ww;
         const long i = (long)yy * W + xx;
@@ -153,143 +154,125 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-__global__ void k_slic_commit(long N, const int *__restrict__ labtmp, int *__restrict__ lab,
-                              int *__restrict__ flag) {
+// Labels of the iteration.  A pixel that no window covers keeps its label, and its
+// cluster's window grows to hold it: then the cluster's pixels in index order are
+// again those with its label in row order of the window.  Resets the scratch for the
+// next iteration.
+__global__ void k_slic_commit(long N, int W, int *__restrict__ labtmp, int *__restrict__ lab,
+                              unsigned long long *__restrict__ dist, int4 *__restrict__ win) {
     pdl_sync();
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i >= N) return;
-    const int l = labtmp[i];
-    if (l != INT_MAX) lab[i] = l;
-    else atomicExch(flag, 1);                          // not covered: keeps its label
-}
-
-// One warp per cluster (window order == index order): the lanes stage 32
-// pixels of a window row at a time in shared memory and lane 0 adds the
-// cluster's ones in order -- or one thread for everything when some pixel
-// was not covered.  win[] keeps the windows of the assignment for the
-// segment lists.
-constexpr int kUpdWarps = 4;
-
-__global__ void __launch_bounds__(32 * kUpdWarps)
-    k_slic_update(const double *__restrict__ rgb, int W, int H, int step, int nc,
-                  SlicCenter *__restrict__ cs, const int *__restrict__ lab,
-                  const int *__restrict__ flag, int4 *__restrict__ win,
-                  double *__restrict__ acc, int cap) {
-    pdl_sync();
-    __shared__ double sv[kUpdWarps][32][3];
-    extern __shared__ __align__(16) unsigned char upd_smem[];   // [warps][cap] staged pixels
-    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-    const int ci = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (*flag) {
-        if (blockIdx.x != 0 || threadIdx.x != 0) return;
-        for (int k = 0; k < nc; ++k) win[k] = slic_window(cs[k], step, W, H);
-        for (int k = 0; k < 6 * nc; ++k) acc[k] = 0.0;
-        const long N = (long)W * H;
-        for (long i = 0; i < N; ++i) {
-            const int l = lab[i];
-            if (l < 0) continue;
-            double *a = acc + 6 * l;
-            a[0] = __dadd_rn(a[0], rgb[3 * i]);
-            a[1] = __dadd_rn(a[1], rgb[3 * i + 1]);
-            a[2] = __dadd_rn(a[2], rgb[3 * i + 2]);
-            a[3] = __dadd_rn(a[3], (double)(i % W));
-            a[4] = __dadd_rn(a[4], (double)(i / W));
-            a[5] += 1.0;
-        }
-        for (int k = 0; k < nc; ++k) {
-            const double *a = acc + 6 * k;
-            if (a[5] != 0.0) {
-                const double n = a[5];
-                cs[k] = {__dmul_rn(__ddiv_rn(a[0], n), 255.0), __dmul_rn(__ddiv_rn(a[1], n), 255.0),
-                         __dmul_rn(__ddiv_rn(a[2], n), 255.0), __ddiv_rn(a[3], n),
-                         __ddiv_rn(a[4], n)};
-            }
-        }
+    int l = labtmp[i];
+    labtmp[i] = INT_MAX;
+    dist[i] = (unsigned long long)__double_as_longlong(1.0e30);
+    if (l != INT_MAX) {
+        lab[i] = l;
         return;
     }
+    l = lab[i];
+    if (l < 0) return;
+    const int x = (int)(i % W), y = (int)(i / W);
+    atomicMin(&win[l].x, x);
+    atomicMax(&win[l].y, x);
+    atomicMin(&win[l].z, y);
+    atomicMax(&win[l].w, y);
+}
+
+// One warp per cluster (window order == index order).  The lanes gather the cluster's
+// pixels, in order, as five rows of doubles in shared memory; five lanes then add a
+// row each, in order (the sums' order is part of the result).  A full buffer is added
+// up before the gathering goes on, so any window fits.  What bounds it is the chain of
+// additions and the two dependent reads per pixel (label, colour), 8 at a time.  450 x
+// 375, step 12: 21 us with all five sums in one lane, now 12; with a pixel that no
+// window covered, 29 ms an iteration in one thread.
+// The last iteration's counts (and valid counts) are the segments'.
+constexpr int kUpdWarps = 2, kUpdCap = 512, kUpdLoads = 8;
+
+__global__ void __launch_bounds__(32 * kUpdWarps)
+    k_slic_update(const double *__restrict__ rgb, int W, int nc, SlicCenter *__restrict__ cs,
+                  const int *__restrict__ lab, const int4 *__restrict__ win,
+                  const uint8_t *__restrict__ valid, int *__restrict__ count,
+                  int *__restrict__ nvalid) {
+    pdl_sync();
+    __shared__ double sv[kUpdWarps][5][kUpdCap + 2];
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    const int ci = blockIdx.x * kUpdWarps + wi;
     if (ci >= nc) return;                              // whole warps leave together
-    const int4 w = slic_window(cs[ci], step, W, H);
-    if (lane == 0) win[ci] = w;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0, s4 = 0.0;
-    long cnt = 0;
+    const int4 w = win[ci];
     const int ww = w.y - w.x + 1, wn = ww * (w.w - w.z + 1);
-    if (wn <= cap) {
-        // stage the cluster's pixels, compacted in window (= index) order
-        const int nw = blockDim.x >> 5;
-        double *cv = reinterpret_cast<double *>(upd_smem) + (size_t)wi * cap * 3;
-        int2 *cxy = reinterpret_cast<int2 *>(reinterpret_cast<double *>(upd_smem) +
-                                             (size_t)nw * cap * 3) + (size_t)wi * cap;
-        int base = 0;
-        for (int t0 = 0; t0 < wn; t0 += 4 * 32) {
-            int xx[4], yy[4];
-            bool ok[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int t = t0 + 32 * u + lane;
-                ok[u] = false;
-                xx[u] = yy[u] = 0;
-                if (t < wn) {
-                    yy[u] = w.z + t / ww;
-                    xx[u] = w.x + t % ww;
-                    ok[u] = lab[(long)yy[u] * W + xx[u]] == ci;
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const unsigned m = __ballot_sync(kFull, ok[u]);
-                if (ok[u]) {
-                    const int pos = base + __popc(m & ((1u << lane) - 1u));
-                    const long i = (long)yy[u] * W + xx[u];
-                    cv[3 * pos] = rgb[3 * i];
-                    cv[3 * pos + 1] = rgb[3 * i + 1];
-                    cv[3 * pos + 2] = rgb[3 * i + 2];
-                    cxy[pos] = make_int2(xx[u], yy[u]);
-                }
-                base += __popc(m);
-            }
-        }
+    double sum = 0.0;                                  // lanes 0..4: r, g, b, x, y
+    int base = 0, cnt = 0, nv = 0;
+    const int comp = lane < 5 ? lane : 4;
+    auto add_up = [&]() {
         __syncwarp();
-        if (lane == 0) {
-            for (int k = 0; k < base; ++k) {
-                s0 = __dadd_rn(s0, cv[3 * k]);
-                s1 = __dadd_rn(s1, cv[3 * k + 1]);
-                s2 = __dadd_rn(s2, cv[3 * k + 2]);
-                s3 = __dadd_rn(s3, (double)cxy[k].x);
-                s4 = __dadd_rn(s4, (double)cxy[k].y);
-            }
-            cnt = base;
+        const double *v = sv[wi][comp];
+        int k = 0;
+        for (; k + 8 <= base; k += 8) {
+            double e[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) e[u] = v[k + u];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) sum = __dadd_rn(sum, e[u]);
         }
-    } else for (int yy = w.z; yy <= w.w; ++yy) {
-        for (int xb = w.x; xb <= w.y; xb += 32) {
-            const int xx = xb + lane;
-            const long i = (long)yy * W + xx;
-            const bool ok = xx <= w.y && lab[i] == ci;
+        for (; k < base; ++k) sum = __dadd_rn(sum, v[k]);
+        __syncwarp();
+        cnt += base;
+        base = 0;
+    };
+    // the window 32 pixels at a time, without a branch around a read
+    const int sx = 32 % ww, sy = 32 / ww;
+    int xx = w.x + lane % ww, yy = w.z + lane / ww;
+    for (int t0 = 0; t0 < wn; t0 += 32 * kUpdLoads) {
+        if (base + 32 * kUpdLoads > kUpdCap) add_up();
+        int px[kUpdLoads], py[kUpdLoads], lb[kUpdLoads];
+#pragma unroll
+        for (int u = 0; u < kUpdLoads; ++u) {
+            px[u] = xx;
+            py[u] = yy;
+            lb[u] = lab[(long)min(yy, w.w) * W + xx];
+            xx += sx;
+            yy += sy;
+            const bool over = xx > w.y;
+            xx -= over ? ww : 0;
+            yy += over;
+        }
+        double c[kUpdLoads][3];
+#pragma unroll
+        for (int u = 0; u < kUpdLoads; ++u) {
+            if (py[u] > w.w) lb[u] = -1;
+            const bool ok = lb[u] == ci;
+            const long i = ok ? (long)py[u] * W + px[u] : 0;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) c[u][q] = ok ? rgb[3 * i + q] : 0.0;
+            if (valid) nv += ok && valid[i];
+        }
+#pragma unroll
+        for (int u = 0; u < kUpdLoads; ++u) {
+            const bool ok = lb[u] == ci;
+            const unsigned m = __ballot_sync(kFull, ok);
             if (ok) {
-                sv[wi][lane][0] = rgb[3 * i];
-                sv[wi][lane][1] = rgb[3 * i + 1];
-                sv[wi][lane][2] = rgb[3 * i + 2];
+                const int pos = base + __popc(m & ((1u << lane) - 1u));
+                sv[wi][0][pos] = c[u][0];
+                sv[wi][1][pos] = c[u][1];
+                sv[wi][2][pos] = c[u][2];
+                sv[wi][3][pos] = (double)px[u];
+                sv[wi][4][pos] = (double)py[u];
             }
-            unsigned m = __ballot_sync(kFull, ok);
-            __syncwarp();
-            if (lane == 0) {
-                while (m) {
-                    const int b = __ffs(m) - 1;
-                    m &= m - 1;
-                    s0 = __dadd_rn(s0, sv[wi][b][0]);
-                    s1 = __dadd_rn(s1, sv[wi][b][1]);
-                    s2 = __dadd_rn(s2, sv[wi][b][2]);
-                    s3 = __dadd_rn(s3, (double)(xb + b));
-                    s4 = __dadd_rn(s4, (double)yy);
-                    ++cnt;
-                }
-            }
-            __syncwarp();
+            base += __popc(m);
         }
     }
-    if (lane == 0 && cnt) {
-        const double n = (double)cnt;
-        cs[ci] = {__dmul_rn(__ddiv_rn(s0, n), 255.0), __dmul_rn(__ddiv_rn(s1, n), 255.0),
-                  __dmul_rn(__ddiv_rn(s2, n), 255.0), __ddiv_rn(s3, n), __ddiv_rn(s4, n)};
+    add_up();
+    if (count) {
+        for (int m = 16; m > 0; m >>= 1) nv += __shfl_xor_sync(kFull, nv, m);
+        if (lane == 0) {
+            count[ci] = cnt;
+            nvalid[ci] = valid ? nv : cnt;
+        }
+    }
+    if (lane < 5 && cnt) {
+        const double q = __ddiv_rn(sum, (double)cnt);
+        reinterpret_cast<double *>(cs + ci)[lane] = lane < 3 ? __dmul_rn(q, 255.0) : q;
     }
 }
 
@@ -321,78 +304,6 @@ __device__ __forceinline__ int block_excl_sum(int v, int *total, int *sbuf) {
     return pre + x - v;
 }
 
-// Segment sizes (pass 0), then ordered pixel lists and valid counts
-// (pass 1), from the windows of the last assignment; the exact single-thread
-// path when some pixel was not covered in that assignment.
-__global__ void __launch_bounds__(256)
-    k_seg_lists(int W, int H, int nseg, const int *__restrict__ lab, const int4 *__restrict__ win,
-                const int *__restrict__ flag, int pass, int *__restrict__ count,
-                const int *__restrict__ start, int *__restrict__ list,
-                const uint8_t *__restrict__ valid, int *__restrict__ nvalid) {
-    pdl_sync();
-    __shared__ int sbuf[32];
-    if (*flag) {
-        if (blockIdx.x != 0 || threadIdx.x != 0) return;
-        const long N = (long)W * H;
-        if (pass == 0) {
-            for (int g = 0; g < nseg; ++g) count[g] = 0;
-            for (long i = 0; i < N; ++i)
-                if (lab[i] >= 0) ++count[lab[i]];
-        } else {
-            for (int g = 0; g < nseg; ++g) count[g] = nvalid[g] = 0;   // count: fill cursors
-            for (long i = 0; i < N; ++i) {
-                const int l = lab[i];
-                if (l < 0) continue;
-                list[start[l] + count[l]++] = (int)i;
-                nvalid[l] += valid ? (int)valid[i] : 1;
-            }
-        }
-        return;
-    }
-    const int g = blockIdx.x;
-    const int4 w = win[g];
-    const int ww = w.y - w.x + 1, n = ww * (w.w - w.z + 1);
-    int base = 0, nv = 0;
-    for (int t0 = 0; t0 < n; t0 += blockDim.x) {
-        const int t = t0 + threadIdx.x;
-        int i = -1;
-        if (t < n) {
-            i = (w.z + t / ww) * W + w.x + t % ww;
-            if (lab[i] != g) i = -1;
-        }
-        int tot;
-        const int pos = block_excl_sum(i >= 0, &tot, sbuf);
-        if (pass == 1) {
-            if (i >= 0) list[start[g] + base + pos] = i;
-            int vt;
-            block_excl_sum(i >= 0 && (!valid || valid[i]), &vt, sbuf);
-            nv += vt;
-        }
-        base += tot;
-    }
-    if (threadIdx.x == 0) {
-        if (pass == 0) count[g] = base;
-        else nvalid[g] = nv;
-    }
-}
-
-// Exclusive scan of count[] into start[] (one CTA of 1024 threads).
-__global__ void __launch_bounds__(1024)
-    k_seg_scan(int nseg, const int *__restrict__ count, int *__restrict__ start) {
-    pdl_sync();
-    __shared__ int sbuf[32];
-    int base = 0;
-    for (int g0 = 0; g0 < nseg; g0 += blockDim.x) {
-        const int g = g0 + threadIdx.x;
-        const int v = g < nseg ? count[g] : 0;
-        int tot;
-        const int pos = block_excl_sum(v, &tot, sbuf);
-        if (g < nseg) start[g] = base + pos;
-        base += tot;
-    }
-    if (threadIdx.x == 0) start[nseg] = base;
-}
-
 __device__ __forceinline__ uint32_t xorshift32(uint32_t s) {
     s ^= s << 13;
     s ^= s >> 17;
@@ -409,48 +320,66 @@ __device__ __forceinline__ uint32_t gf2_apply(const uint32_t *A, uint32_t x) {
     return y;
 }
 
-constexpr int kJumpBits = 24;                // up to 2^24 segments
+// The same from a table per 4 bits of x: tab[16 * i + e] = A (e << 4 i).
+constexpr int kGfTab = 8 * 16;
+__device__ __forceinline__ uint32_t gf2_entry(const uint32_t *A, int k) {
+    const uint32_t *c = A + 4 * (k >> 4);
+    return (k & 1 ? c[0] : 0u) ^ (k & 2 ? c[1] : 0u) ^ (k & 4 ? c[2] : 0u) ^ (k & 8 ? c[3] : 0u);
+}
+__device__ __forceinline__ uint32_t gf2_lookup(const uint32_t *tab, uint32_t x) {
+    uint32_t y = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) y ^= tab[16 * i + ((x >> (4 * i)) & 15u)];
+    return y;
+}
 
-// Starting xorshift32 state of every segment: seed advanced by 3*trials
-// draws for each earlier segment with at least 12 valid pixels.  One CTA:
-// the jump matrices J_j = M^(3*trials*2^j) by squaring, then a scan of the
-// eligibility and one matrix product per set bit of each segment's count.
+constexpr int kJumpBits = 24;                // up to 2^24 segments
+constexpr int kDrawBits = 7;                 // up to 64 trials
+
+// Offsets of the segments' pixels, and the starting xorshift32 state of every
+// segment: seed advanced by 3*trials draws for each earlier segment with at
+// least 12 valid pixels.  One CTA: the jump matrices J_j = M^(3*trials*2^j) by
+// squaring (as many as nseg has bits), their tables, then a scan of the
+// eligibility and one table look-up per set bit of each segment's count (by
+// columns, four times the instructions: 16 us for 1,147 segments, now 13).
+// draw[j] is the table of M^(3*2^j): the segments jump to their trials' draws.
 __global__ void __launch_bounds__(1024)
-    k_seg_rng(int nseg, const int *__restrict__ nvalid, int trials, uint32_t seed,
-              uint32_t *__restrict__ state) {
+    k_seg_rng(int nseg, const int *__restrict__ count, const int *__restrict__ nvalid, int trials,
+              uint32_t seed, int *__restrict__ start, uint32_t *__restrict__ state,
+              uint32_t *__restrict__ draw) {
     pdl_sync();
-    __shared__ uint32_t J[kJumpBits][32];
-    __shared__ uint32_t T[2][32];
+    __shared__ uint32_t J[kJumpBits][32], JT[kJumpBits][kGfTab];
+    __shared__ uint32_t T[2][32], DJ[kDrawBits][32];
     __shared__ int sbuf[32];
     const int t = threadIdx.x;
     // M^(3*trials): square-and-multiply on columns (warp 0)
     if (t < 32) {
-        T[0][t] = xorshift32(1u << t);                 // M
+        T[0][t] = xorshift32(xorshift32(xorshift32(1u << t)));     // M^3
         T[1][t] = 1u << t;                             // identity (accumulator)
-    }
-    __syncthreads();
-    int e = 3 * trials;
-    while (e > 0) {
-        uint32_t acc = 0, sq = 0;
-        if (t < 32) {
-            acc = (e & 1) ? gf2_apply(T[0], T[1][t]) : T[1][t];
-            sq = gf2_apply(T[0], T[0][t]);
-        }
-        __syncthreads();
-        if (t < 32) {
+        __syncwarp();
+        for (int j = 0; j < kDrawBits; ++j) {
+            const uint32_t acc = (trials >> j) & 1 ? gf2_apply(T[0], T[1][t]) : T[1][t];
+            const uint32_t sq = gf2_apply(T[0], T[0][t]);
+            DJ[j][t] = T[0][t];
+            __syncwarp();
             T[1][t] = acc;
             T[0][t] = sq;
+            __syncwarp();
         }
-        __syncthreads();
-        e >>= 1;
+        J[0][t] = T[1][t];
+        __syncwarp();
+        for (int j = 1; j < kJumpBits && (nseg >> j); ++j) {
+            J[j][t] = gf2_apply(J[j - 1], J[j - 1][t]);
+            __syncwarp();
+        }
     }
-    if (t < 32) J[0][t] = T[1][t];
     __syncthreads();
-    for (int j = 1; j < kJumpBits; ++j) {
-        if (t < 32) J[j][t] = gf2_apply(J[j - 1], J[j - 1][t]);
-        __syncthreads();
-    }
-    int base = 0;
+    for (int k = t; k < kDrawBits * kGfTab; k += blockDim.x)
+        draw[k] = gf2_entry(DJ[k / kGfTab], k % kGfTab);
+    for (int k = t; k < kJumpBits * kGfTab && (nseg >> (k / kGfTab)); k += blockDim.x)
+        JT[k / kGfTab][k % kGfTab] = gf2_entry(J[k / kGfTab], k % kGfTab);
+    __syncthreads();
+    int base = 0, first = 0;
     for (int g0 = 0; g0 < nseg; g0 += blockDim.x) {
         const int g = g0 + t;
         const int nv = g < nseg ? nvalid[g] : 0;
@@ -458,11 +387,14 @@ __global__ void __launch_bounds__(1024)
         const int c = base + block_excl_sum(g < nseg && nv >= 12, &tot, sbuf);
         if (g < nseg) {
             uint32_t s = seed;
-            for (int j = 0; j < kJumpBits; ++j)
-                if ((c >> j) & 1) s = gf2_apply(J[j], s);
+            for (int j = 0; j < kJumpBits && (c >> j); ++j)
+                if ((c >> j) & 1) s = gf2_lookup(JT[j], s);
             state[g] = s;
         }
         base += tot;
+        const int pos = first + block_excl_sum(g < nseg ? count[g] : 0, &tot, sbuf);
+        if (g < nseg) start[g] = pos;
+        first += tot;
     }
 }
 
@@ -496,167 +428,231 @@ __device__ __forceinline__ double plane_at(const double *pl, int i, int W) {
 }
 
 constexpr int kMaxTrials = 64;
-constexpr int kSnapCap = 2048;          // segment points staged in shared memory
+constexpr int kSnapCap = 2048;          // most points of a segment in shared memory
+constexpr int kSnapThreads = 128, kSnapScan = 5;
 
-// One CTA per segment: RANSAC, least squares over the inliers, snap.  The
-// segment's valid points (x, y, d) are staged in shared memory so the
-// sequential parts (the draws and planes of thread 0, the ordered
-// least-squares sums) read shared memory; segments larger than kSnapCap
-// read global memory instead (same values, same order).
-__global__ void __launch_bounds__(256)
+// The points of a segment: rows of x, y and d in shared memory, or pixel indices.
+struct SnapRows {
+    const double *rows;
+    int cap;
+    __device__ __forceinline__ double operator()(int c, int j) const { return rows[c * cap + j]; }
+};
+struct SnapList {
+    const int *list;
+    const double *disp;
+    int W;
+    __device__ __forceinline__ double operator()(int c, int j) const {
+        const int i = list[j];
+        return c == 0 ? (double)(i % W) : c == 1 ? (double)(i / W) : disp[i];
+    }
+};
+
+template <typename P>
+__device__ __forceinline__ int snap_ok(const P &p, const double *pl, double thr, int j) {
+    const double v = __dadd_rn(__dadd_rn(__dmul_rn(pl[0], p(0, j)), __dmul_rn(pl[1], p(1, j))), pl[2]);
+    return fabs(__dsub_rn(v, p(2, j))) <= thr;
+}
+
+// the points within thr of a plane, counted by a warp
+template <typename P>
+__device__ __forceinline__ int snap_count(const P &p, const double *pl, double thr, int n, int lane) {
+    int c = 0, j = lane;
+    for (; j + 96 < n; j += 128) {
+        int e[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) e[u] = snap_ok(p, pl, thr, j + 32 * u);
+        c += (e[0] + e[1]) + (e[2] + e[3]);
+    }
+    for (; j < n; j += 32) c += snap_ok(p, pl, thr, j);
+    for (int m = 16; m > 0; m >>= 1) c += __shfl_xor_sync(kFull, c, m);
+    return c;
+}
+
+// s plus f(0), f(1), ..., f(n - 1) in order, the terms 8 at a time ahead of the chain
+template <typename F>
+__device__ __forceinline__ double chain_sum(double s, int n, F f) {
+    int k = 0;
+    for (; k + 8 <= n; k += 8) {
+        double e[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) e[u] = f(k + u);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s = __dadd_rn(s, e[u]);
+    }
+    for (; k < n; ++k) s = __dadd_rn(s, f(k));
+    return s;
+}
+
+// _lsq_plane, stereonet.py:5472-5502, by one warp: sums in the points' order
+template <typename P>
+__device__ __forceinline__ void snap_fit(const P &p, int n, int lane, double *fit) {
+    const int c3 = lane < 3 ? lane : 2;                    // lanes 0..2: x, y, d
+    const double mean = __ddiv_rn(chain_sum(0.0, n, [&](int k) { return p(c3, k); }), (double)n);
+    const double mx = __shfl_sync(kFull, mean, 0), my = __shfl_sync(kFull, mean, 1),
+                 md = __shfl_sync(kFull, mean, 2);
+    // lanes 0..4: xx, xy, yy, xd, yd
+    const int ca = lane == 2 || lane == 4 ? 1 : 0;
+    const int cb = lane == 0 ? 0 : lane <= 2 ? 1 : 2;
+    const double ma = ca ? my : mx, mb = cb == 0 ? mx : cb == 1 ? my : md;
+    const double s = chain_sum(0.0, n, [&](int k) {
+        return __dmul_rn(__dsub_rn(p(ca, k), ma), __dsub_rn(p(cb, k), mb));
+    });
+    const double sxx = __shfl_sync(kFull, s, 0), sxy = __shfl_sync(kFull, s, 1),
+                 syy = __shfl_sync(kFull, s, 2), sxd = __shfl_sync(kFull, s, 3),
+                 syd = __shfl_sync(kFull, s, 4);
+    if (lane != 0) return;
+    const double det = __dsub_rn(__dmul_rn(sxx, syy), __dmul_rn(sxy, sxy));
+    if (fabs(det) < 1.0e-9) {
+        fit[0] = 0.0;
+        fit[1] = 0.0;
+        fit[2] = md;
+    } else {
+        const double a = __ddiv_rn(__dsub_rn(__dmul_rn(sxd, syy), __dmul_rn(syd, sxy)), det);
+        const double b = __ddiv_rn(__dsub_rn(__dmul_rn(syd, sxx), __dmul_rn(sxd, sxy)), det);
+        fit[0] = a;
+        fit[1] = b;
+        fit[2] = __dsub_rn(__dsub_rn(md, __dmul_rn(a, mx)), __dmul_rn(b, my));
+    }
+}
+
+// One CTA per segment: RANSAC, least squares over the inliers, snap.  The segment's
+// valid points are gathered from its window, in index order, as rows of x, y and d in
+// shared memory (cap of them; a larger segment keeps their indices in pts and inl:
+// same values, same order).  The draws are one stream, so a trial's thread jumps to
+// its own three; a warp counts a trial's inliers; the least-squares sums, whose order
+// is part of the result, are one chain each, so a lane each adds them up.  What bounds
+// it is those chains and the scan of the window.  450 x 375, step 12, 40 trials: 125
+// us with draws and sums in one thread and a list made by kernels ahead (18 us), now
+// 33.
+__global__ void __launch_bounds__(kSnapThreads)
     k_seg_snap(const double *__restrict__ disp, int W, const uint8_t *__restrict__ valid,
-               const int *__restrict__ start, const int *__restrict__ list,
-               const int *__restrict__ nvalid, const uint32_t *__restrict__ state, int trials,
-               double thr, double min_inl, int *__restrict__ pts, int *__restrict__ inl,
+               const int *__restrict__ lab, const int4 *__restrict__ win,
+               const int *__restrict__ start, const int *__restrict__ nvalid,
+               const uint32_t *__restrict__ state, const uint32_t *__restrict__ draw, int trials,
+               double thr, double min_inl, int cap, int *__restrict__ pts, int *__restrict__ inl,
                double *__restrict__ out) {
     pdl_sync();
     __shared__ double planes[kMaxTrials][3];
     __shared__ int ok[kMaxTrials], cnt[kMaxTrials];
-    __shared__ int sbuf[32];
-    __shared__ int s_best;
+    __shared__ int sbuf[32], wcnt[kSnapScan][kSnapThreads / 32];
     __shared__ double fit[3];
-    __shared__ int2 sxy[kSnapCap];
-    __shared__ double sdv[kSnapCap];
-    __shared__ int sinl[kSnapCap];
-    __shared__ int sbuf_draw[3 * kMaxTrials];
-    const int g = blockIdx.x, t = threadIdx.x;
-    const int s0 = start[g], gn = start[g + 1] - s0;
-    if (nvalid[g] < 12) return;
-    // valid pixels in index order
+    extern __shared__ __align__(16) double rows[];     // [3][cap]
+    const int g = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int n = nvalid[g];
+    if (n < 12) return;
+    const int4 w = win[g];
+    const int ww = w.y - w.x + 1, wn = ww * (w.w - w.z + 1);
+    const bool staged = n <= cap;
+    int *const gp = pts + start[g], *const gi = inl + start[g];
+    // valid pixels in index order, kSnapScan x kSnapThreads of the window at a time
     int base = 0;
-    for (int k0 = 0; k0 < gn; k0 += blockDim.x) {
-        const int k = k0 + t;
-        const int i = k < gn ? list[s0 + k] : -1;
-        const int take = i >= 0 && (!valid || valid[i]);
-        int tot;
-        const int pos = block_excl_sum(take, &tot, sbuf);
-        if (take) pts[s0 + base + pos] = i;
-        base += tot;
-    }
-    const int n = base;
-    const bool staged = n <= kSnapCap;
-    __syncthreads();
-    if (staged) {
-        for (int j = t; j < n; j += blockDim.x) {
-            const int i = pts[s0 + j];
-            sxy[j] = make_int2(i % W, i / W);
-            sdv[j] = disp[i];
+    for (int k0 = 0; k0 < wn; k0 += kSnapScan * kSnapThreads) {
+        long i[kSnapScan];
+        unsigned m[kSnapScan];
+        double d[kSnapScan];
+        bool take[kSnapScan];
+#pragma unroll
+        for (int u = 0; u < kSnapScan; ++u) {
+            const int k = k0 + u * kSnapThreads + t;
+            i[u] = (long)(w.z + k / ww) * W + w.x + k % ww;
+            take[u] = k < wn && lab[i[u]] == g;
         }
-    }
-    __syncthreads();
-    auto P = [&](int j, double &x, double &y, double &d) {
-        if (staged) {
-            const int2 q = sxy[j];
-            x = (double)q.x;
-            y = (double)q.y;
-            d = sdv[j];
-        } else {
-            const int i = pts[s0 + j];
-            x = (double)(i % W);
-            y = (double)(i / W);
-            d = disp[i];
+#pragma unroll
+        for (int u = 0; u < kSnapScan; ++u) {
+            take[u] = take[u] && (!valid || valid[i[u]]);
+            d[u] = take[u] ? disp[i[u]] : 0.0;
+            m[u] = __ballot_sync(kFull, take[u]);
+            if (lane == 0) wcnt[u][warp] = __popc(m[u]);
         }
-    };
-    auto resid_ok = [&](const double *pl, int j) {
-        double x, y, d;
-        P(j, x, y, d);
-        const double v = __dadd_rn(__dadd_rn(__dmul_rn(pl[0], x), __dmul_rn(pl[1], y)), pl[2]);
-        return fabs(__dsub_rn(v, d)) <= thr;
-    };
-    // the draws are one sequential stream (thread 0); the planes are not
-    if (t == 0) {
-        uint32_t s = state[g];
-        for (int k = 0; k < 3 * trials; ++k) {
-            s = xorshift32(s);
-            sbuf_draw[k] = (int)(s % (uint32_t)n);
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kSnapScan; ++u) {
+            int pos = base + __popc(m[u] & ((1u << lane) - 1u));
+#pragma unroll
+            for (int q = 0; q < kSnapThreads / 32; ++q) {
+                if (q < warp) pos += wcnt[u][q];
+                base += wcnt[u][q];
+            }
+            if (!take[u]) continue;
+            if (staged) {
+                const int y = (int)(i[u] / W);
+                rows[pos] = (double)((int)i[u] - y * W);
+                rows[cap + pos] = (double)y;
+                rows[2 * cap + pos] = d[u];
+            } else {
+                gp[pos] = (int)i[u];
+            }
         }
+        __syncthreads();
     }
-    __syncthreads();
+    const SnapRows pr{rows, cap};
+    const SnapList pp{gp, disp, W}, pi{gi, disp, W};
+    auto at = [&](int c, int j) { return staged ? pr(c, j) : pp(c, j); };
     if (t < trials) {
+        uint32_t s = state[g];
+        for (int j = 0; j < kDrawBits; ++j)
+            if ((t >> j) & 1) s = gf2_lookup(draw + kGfTab * j, s);
         double A[3][3], bv[3];
         for (int u = 0; u < 3; ++u) {
-            P(sbuf_draw[3 * t + u], A[u][0], A[u][1], bv[u]);
+            s = xorshift32(s);
+            const int j = (int)(s % (uint32_t)n);
+            A[u][0] = at(0, j);
+            A[u][1] = at(1, j);
             A[u][2] = 1.0;
+            bv[u] = at(2, j);
         }
         ok[t] = solve3_dev(A, bv, planes[t]);
-        cnt[t] = 0;
     }
     __syncthreads();
-    for (long q = t; q < (long)trials * n; q += blockDim.x) {
-        const int tr = (int)(q / n), j = (int)(q - (long)tr * n);
-        if (ok[tr] && resid_ok(planes[tr], j)) atomicAdd(&cnt[tr], 1);
+    for (int tr = warp; tr < trials; tr += kSnapThreads / 32) {
+        if (!ok[tr]) continue;
+        const double pl[3] = {planes[tr][0], planes[tr][1], planes[tr][2]};
+        const int c = staged ? snap_count(pr, pl, thr, n, lane) : snap_count(pp, pl, thr, n, lane);
+        if (lane == 0) cnt[tr] = c;
     }
     __syncthreads();
-    if (t == 0) {
-        int best = -1, bestc = -1;
-        for (int tr = 0; tr < trials; ++tr)
-            if (ok[tr] && cnt[tr] > bestc) {
-                bestc = cnt[tr];
-                best = tr;
-            }
-        s_best = (best < 0 || (double)bestc < __dmul_rn(min_inl, (double)n)) ? -1 : best;
-    }
-    __syncthreads();
-    const int best = s_best;
-    if (best < 0) return;
+    int best = -1, bestc = -1;
+    for (int tr = 0; tr < trials; ++tr)
+        if (ok[tr] && cnt[tr] > bestc) {
+            bestc = cnt[tr];
+            best = tr;
+        }
+    if (best < 0 || (double)bestc < __dmul_rn(min_inl, (double)n)) return;
+    // the inliers, in order, over the points (an inlier moves down or stays)
+    const double pl[3] = {planes[best][0], planes[best][1], planes[best][2]};
     base = 0;
-    for (int k0 = 0; k0 < n; k0 += blockDim.x) {
+    for (int k0 = 0; k0 < n; k0 += kSnapThreads) {
         const int k = k0 + t;
-        const int take = k < n && resid_ok(planes[best], k);
+        const int take = k < n && (staged ? snap_ok(pr, pl, thr, k) : snap_ok(pp, pl, thr, k));
+        double x = 0.0, y = 0.0, d = 0.0;
+        if (take && staged) {
+            x = rows[k];
+            y = rows[cap + k];
+            d = rows[2 * cap + k];
+        }
         int tot;
-        const int pos = block_excl_sum(take, &tot, sbuf);
+        const int pos = base + block_excl_sum(take, &tot, sbuf);
         if (take) {
-            if (staged) sinl[base + pos] = k;
-            else inl[s0 + base + pos] = k;
+            if (staged) {
+                rows[pos] = x;
+                rows[cap + pos] = y;
+                rows[2 * cap + pos] = d;
+            } else {
+                gi[pos] = gp[k];
+            }
         }
         base += tot;
     }
     __syncthreads();
-    if (t == 0) {
-        // _lsq_plane, stereonet.py:5472-5502: sums in inlier order
-        const int ni = base;
-        const double nn = (double)ni;
-        double sx = 0.0, sy = 0.0, sd = 0.0, x, y, d;
-        for (int k = 0; k < ni; ++k) {
-            P(staged ? sinl[k] : inl[s0 + k], x, y, d);
-            sx = __dadd_rn(sx, x);
-        }
-        for (int k = 0; k < ni; ++k) {
-            P(staged ? sinl[k] : inl[s0 + k], x, y, d);
-            sy = __dadd_rn(sy, y);
-        }
-        for (int k = 0; k < ni; ++k) {
-            P(staged ? sinl[k] : inl[s0 + k], x, y, d);
-            sd = __dadd_rn(sd, d);
-        }
-        const double mx = __ddiv_rn(sx, nn), my = __ddiv_rn(sy, nn), md = __ddiv_rn(sd, nn);
-        double sxx = 0.0, sxy_ = 0.0, syy = 0.0, sxd = 0.0, syd = 0.0;
-        for (int k = 0; k < ni; ++k) {
-            P(staged ? sinl[k] : inl[s0 + k], x, y, d);
-            const double u = __dsub_rn(x, mx), v = __dsub_rn(y, my), w = __dsub_rn(d, md);
-            sxx = __dadd_rn(sxx, __dmul_rn(u, u));
-            sxy_ = __dadd_rn(sxy_, __dmul_rn(u, v));
-            syy = __dadd_rn(syy, __dmul_rn(v, v));
-            sxd = __dadd_rn(sxd, __dmul_rn(u, w));
-            syd = __dadd_rn(syd, __dmul_rn(v, w));
-        }
-        const double det = __dsub_rn(__dmul_rn(sxx, syy), __dmul_rn(sxy_, sxy_));
-        if (fabs(det) < 1.0e-9) {
-            fit[0] = 0.0;
-            fit[1] = 0.0;
-            fit[2] = md;
-        } else {
-            const double a = __ddiv_rn(__dsub_rn(__dmul_rn(sxd, syy), __dmul_rn(syd, sxy_)), det);
-            const double b = __ddiv_rn(__dsub_rn(__dmul_rn(syd, sxx), __dmul_rn(sxd, sxy_)), det);
-            fit[0] = a;
-            fit[1] = b;
-            fit[2] = __dsub_rn(__dsub_rn(md, __dmul_rn(a, mx)), __dmul_rn(b, my));
-        }
+    if (warp == 0) {
+        if (staged) snap_fit(pr, base, lane, fit);
+        else snap_fit(pi, base, lane, fit);
     }
     __syncthreads();
-    for (int k = t; k < gn; k += blockDim.x) {
-        const int i = list[s0 + k];
-        const double v = plane_at(fit, i, W);
+    for (int k = t; k < wn; k += kSnapThreads) {
+        const long i = (long)(w.z + k / ww) * W + w.x + k % ww;
+        if (lab[i] != g) continue;
+        const double v = plane_at(fit, (int)i, W);
         if (fabs(__dsub_rn(v, disp[i])) <= thr || (valid && !valid[i])) out[i] = v > 0.0 ? v : 0.0;
     }
 #undef M_
@@ -699,18 +695,16 @@ size_t carve_post(void *ws, int W, int H, int step, PostWs *o) {
     p.flags = cv.take<DevFlags>(1);
     p.cs = cv.take<unsigned char>(sizeof(SlicCenter) * nca);
     p.win = cv.take<int4>(nca);
-    p.acc = cv.take<double>(6 * (size_t)nca);
     p.dist = cv.take<unsigned long long>(N);
     p.labtmp = cv.take<int>(N);
     p.lab = cv.take<int>(N);
-    p.flag = cv.take<int>(4);
     p.count = cv.take<int>(nca);
-    p.start = cv.take<int>(nca + 1);
-    p.list = cv.take<int>(N);
+    p.start = cv.take<int>(nca);
     p.pts = cv.take<int>(N);
     p.inl = cv.take<int>(N);
     p.nvalid = cv.take<int>(nca);
     p.state = cv.take<uint32_t>(nca);
+    p.draw = cv.take<uint32_t>(kGfTab * kDrawBits);
     p.valid = cv.take<uint8_t>(N);
     p.tmp = cv.take<double>(N);
     if (o) *o = p;
@@ -718,7 +712,7 @@ size_t carve_post(void *ws, int W, int H, int step, PostWs *o) {
 }
 
 int launch_slic(const double *rgb, int W, int H, int step, double compactness, int iters,
-                const PostWs &w, cudaStream_t st) {
+                const PostWs &w, cudaStream_t st, const uint8_t *valid) {
     if (W < 1 || H < 1 || step < 1 || iters < 0) {
         set_error("slic: bad shape or step");
         return SV_ERR_PARAM;
@@ -729,29 +723,26 @@ int launch_slic(const double *rgb, int W, int H, int step, double compactness, i
     const double m2 = slic_m2(compactness, step);
     SlicCenter *cs = reinterpret_cast<SlicCenter *>(w.cs);
     SV_CUDA_TRY(cudaMemsetAsync(w.lab, 0xFF, sizeof(int) * N, st));       // -1
-    SV_CUDA_TRY(cudaMemsetAsync(w.flag, 0, sizeof(int) * 4, st));
     if (nc == 0) return SV_OK;
     count_launch();
     pdl(k_slic_init, (nc + 127) / 128, 128, 0, st)(rgb, W, step, ncx, nc, cs);
     const int nb = grid_for(N, 256, 1 << 30);
-    // SLIC update staging: (2 step + 1)^2 pixels of 32 bytes per warp
-    const long wmax = (long)(2 * step + 1) * (2 * step + 1);
-    // within the 48 KB default, next to the kernel's 3 KB of static shared memory
-    const int wpb0 = (int)((44l * 1024) / (wmax * 32));
-    const int wpb = wpb0 < 1 ? kUpdWarps : (wpb0 > kUpdWarps ? kUpdWarps : wpb0);
-    const int cap = wpb0 < 1 ? 0 : (int)wmax;
+    if (iters > 0) {
+        count_launch();
+        pdl(k_slic_reset, nb, 256, 0, st)(N, w.dist, w.labtmp);
+    }
     for (int it = 0; it < iters; ++it) {
+        const bool last = it + 1 == iters;
         count_launch();
-        pdl(k_slic_reset, nb, 256, 0, st)(N, w.dist, w.labtmp, w.flag);
+        pdl(k_slic_assign, nc, 256, 0, st)(rgb, W, H, step, m2, cs, 0, w.dist, w.labtmp, w.win);
         count_launch();
-        pdl(k_slic_assign, nc, 256, 0, st)(rgb, W, H, step, m2, cs, 0, w.dist, w.labtmp);
+        pdl(k_slic_assign, nc, 256, 0, st)(rgb, W, H, step, m2, cs, 1, w.dist, w.labtmp, w.win);
         count_launch();
-        pdl(k_slic_assign, nc, 256, 0, st)(rgb, W, H, step, m2, cs, 1, w.dist, w.labtmp);
+        pdl(k_slic_commit, nb, 256, 0, st)(N, W, w.labtmp, w.lab, w.dist, w.win);
         count_launch();
-        pdl(k_slic_commit, nb, 256, 0, st)(N, w.labtmp, w.lab, w.flag);
-        count_launch();
-        pdl(k_slic_update, (nc + wpb - 1) / wpb, 32 * wpb, (size_t)wpb * cap * 32, st)(
-            rgb, W, H, step, nc, cs, w.lab, w.flag, w.win, w.acc, cap);
+        pdl(k_slic_update, (nc + kUpdWarps - 1) / kUpdWarps, 32 * kUpdWarps, 0, st)(
+            rgb, W, nc, cs, w.lab, w.win, valid, last ? w.count : nullptr,
+            last ? w.nvalid : nullptr);
     }
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -768,21 +759,21 @@ int launch_plane_snap(const double *disp, const double *rgb, int W, int H, const
     SV_CUDA_TRY(cudaMemcpyAsync(out, disp, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
     int ncx, ncy;
     const int nc = slic_grid(W, H, step, &ncx, &ncy);
-    SV_TRY_POST(launch_slic(rgb, W, H, step, 10.0, 5, w, st));
+    SV_TRY_POST(launch_slic(rgb, W, H, step, 10.0, 5, w, st, valid));
     if (nc == 0 || trials == 0) return SV_OK;
     count_launch();
-    pdl(k_seg_lists, nc, 256, 0, st)(W, H, nc, w.lab, w.win, w.flag, 0, w.count, w.start, w.list,
-                                    valid, w.nvalid);
+    pdl(k_seg_rng, 1, 1024, 0, st)(nc, w.count, w.nvalid, trials, seed, w.start, w.state, w.draw);
+    // shared memory for a whole window's points, at most kSnapCap
+    const long wmax = (long)(2 * step + 1) * (2 * step + 1);
+    const int cap = wmax < kSnapCap ? (int)wmax : kSnapCap;
+    const size_t smem = (size_t)cap * 3 * sizeof(double);
+    if (smem > 40 * 1024)
+        SV_CUDA_TRY(cudaFuncSetAttribute(k_seg_snap, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem));
     count_launch();
-    pdl(k_seg_scan, 1, 1024, 0, st)(nc, w.count, w.start);
-    count_launch();
-    pdl(k_seg_lists, nc, 256, 0, st)(W, H, nc, w.lab, w.win, w.flag, 1, w.count, w.start, w.list,
-                                    valid, w.nvalid);
-    count_launch();
-    pdl(k_seg_rng, 1, 1024, 0, st)(nc, w.nvalid, trials, seed, w.state);
-    count_launch();
-    pdl(k_seg_snap, nc, 256, 0, st)(disp, W, valid, w.start, w.list, w.nvalid, w.state, trials,
-                                   thr, min_inl, w.pts, w.inl, out);
+    pdl(k_seg_snap, nc, kSnapThreads, smem, st)(disp, W, valid, w.lab, w.win, w.start, w.nvalid,
+                                               w.state, w.draw, trials, thr, min_inl, cap, w.pts,
+                                               w.inl, out);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }

@@ -13,15 +13,15 @@ struct DevFlags;
 struct PostWs {
     DevFlags *flags;
     unsigned char *cs;          // SLIC centres
-    int4 *win;                  // each cluster's window of the last assignment
-    double *acc;                // exact single-thread update path
+    int4 *win;                  // each cluster's window of the last assignment, grown to
+                                // hold the pixels it kept outside
     unsigned long long *dist;   // per-pixel minimum distance bits
     int *labtmp, *lab;          // assignment scratch, labels
-    int *flag;                  // "a pixel was not covered" in the current iteration
-    int *count, *start, *list;  // segment sizes, offsets, pixel lists in index order
+    int *count, *start;         // segment sizes, offsets
     int *pts, *inl;             // per segment: valid pixels, inliers (same offsets)
     int *nvalid;
     uint32_t *state;            // per segment: xorshift32 state at its first draw
+    uint32_t *draw;             // jumps over 3 * 2^j draws
     uint8_t *valid;             // status == 0 (refine_disparity)
     double *tmp;                // intermediate disparity
 };
@@ -38,7 +38,7 @@ size_t carve_post(void *ws, int W, int H, int step, PostWs *o);
 int launch_median(const double *in, int W, int H, int radius, int passes, double *out,
                   double *tmp, cudaStream_t st);
 int launch_slic(const double *rgb, int W, int H, int step, double compactness, int iters,
-                const PostWs &w, cudaStream_t st);
+                const PostWs &w, cudaStream_t st, const uint8_t *valid = nullptr);
 int launch_plane_snap(const double *disp, const double *rgb, int W, int H, const uint8_t *valid,
                       int step, double thr, double min_inl, int trials, uint32_t seed,
                       double *out, const PostWs &w, cudaStream_t st);
