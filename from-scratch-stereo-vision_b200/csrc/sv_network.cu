@@ -411,29 +411,6 @@ __device__ __forceinline__ void conv_level(int lv, int Hw, int Ww, int &H, int &
     }
 }
 
-template <int IC, int OC, int OCG, int ACT, int CS>
-__global__ void __launch_bounds__(CT2_TW *CT2_TH *CS)
-    k_b_conv2d_tiled(NetLaunch L, int lv, int Z, const float *x0, const float *x1, int stride,
-                     int pad, int dil, const float *__restrict__ w, const float *__restrict__ b,
-                     float *y0, float *y1, const float *resid) {
-    pdl_sync();
-    long long c;
-    const int p = net_pair(L, c);
-    const NetPair &P = L.pairs[p];
-    if (!P.active) return;
-    int H, W, OH, OW;
-    conv_level(lv, P.Hw, P.Ww, H, W, OH, OW);
-    const int tx = (OW + CT2_TW - 1) / CT2_TW, ty = (OH + CT2_TH - 1) / CT2_TH;
-    const int bz = (int)(c % Z);
-    const long long t = c / Z;
-    const int bx = (int)(t % tx), by = (int)(t / tx);
-    if (by >= ty) return;
-    conv2d_tiled_body<IC, OC, OCG, ACT, CS>(bx, by, bz, net_slab(x0, L, p), net_slab(x1, L, p),
-                                            H, W, OH, OW, stride, pad, dil, w, b,
-                                            net_slab(y0, L, p), net_slab(y1, L, p),
-                                            net_slab(resid, L, p));
-}
-
 // 3x3 convolutions (padding = dilation; stride S = 1, or 2 with dilation 1)
 // with every output channel in one thread and PX pixels per thread, CTB_TW /
 // PX columns apart: the register-blocked form of k_conv2d_tiled<IC, OC, *,
@@ -604,6 +581,244 @@ static void b_conv2d_wide(const NetLaunch &L, unsigned ctas, int lv, int Z, cons
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     pdl(k_b_conv2d_wide<IC, OC, ACT, CS, PX, S>, ctas, CTB_TW / PX * CTB_TH, smem, st)(
         L, lv, Z, x0, x1, dil, w, b, y0, y1, resid);
+}
+
+// The Refinement levels' 3x3 convolutions, stride 1, padding = dilation: a CTA
+// computes 32 columns x 16 rows, a thread 4 columns of every output channel, so a
+// 16-byte read of the tile or of the weights (a broadcast) feeds 8 to 16 FMAs, and
+// what bounds it is the FMAs.  The arithmetic is k_conv2d_tiled<IC, OC, *, ACT, CS>'s:
+// each of the CS channel groups is its own fmaf chain over (channel, ky, kx), the
+// sums combined as the butterfly combines them, then the bias and the activation --
+// so the results are bit-identical to that kernel's.  DIL: the dilation, 0 to read it
+// (up to 8), -1 to read the taps from memory without a tile (any dilation).
+// 8 -> 8 channels, dilations 2 and 4: 640 x 480 36 and 46 us with k_conv2d_tiled, now
+// 16; 20 pairs of 77,000 pixels 95 and 125 us with 2 columns, 32 x 4 tiles and one
+// element per copy, now 53 and 55.
+constexpr int CTR_TW = 32, CTR_TH = 16;         // output tile of a CTA
+
+template <int DIL>
+struct ConvRows {
+    static constexpr int PAD = DIL > 0 && DIL <= 4 ? 4 : 8;    // columns staged ahead of the tile
+    static constexpr int NCH = (CTR_TW + 2 * PAD) / 4;         // 16-byte chunks of a row
+    static constexpr int RW = 4 * NCH + 4 * (1 - NCH % 2);     // an odd number: spreads banks
+};
+
+template <int BYTES>
+__device__ __forceinline__ void conv_copy(float *dst, const float *src, bool on) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if constexpr (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src),
+                     "r"(on ? 16 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src),
+                     "r"(on ? 4 : 0) : "memory");
+}
+
+template <int IC, int OC, int ACT, int CS, int DIL>
+__device__ __forceinline__ void conv2d_rows_body(int bx, int by, const float *__restrict__ x, int H,
+                                                 int W, int dil_, const float *__restrict__ w,
+                                                 const float *__restrict__ b, float *y,
+                                                 const float *__restrict__ resid) {
+    using R = ConvRows<DIL>;
+    constexpr int CPS = IC / CS, NT = 8 * CTR_TH, OCP = OC >= 4 ? (OC + 3) / 4 * 4 : OC;
+    static_assert(IC % CS == 0 && (CS == 1 || CS == 2 || CS == 4) && DIL <= 4, "shape");
+    extern __shared__ __align__(16) float tile[];      // [IC][TH + 2 dil][RW]
+    __shared__ __align__(16) float sw[IC * 9 * OCP];
+    __shared__ float sb[OC];
+    const int dil = DIL > 0 ? DIL : dil_, th = CTR_TH + 2 * dil;
+    const int tid = threadIdx.x, ox0 = bx * CTR_TW, oy0 = by * CTR_TH;
+    const long HW = (long)H * W;
+    const bool vec = (W & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    const int nrows = IC * th, xs = ox0 - R::PAD;
+    auto row_of = [&](int r) -> const float * {
+        const int c = r / th, gy = oy0 - dil + r - c * th;
+        return gy >= 0 && gy < H ? x + c * HW + (long)gy * W : nullptr;
+    };
+    if (DIL < 0) {
+    } else if (vec) {
+        for (int i = tid; i < nrows * R::NCH; i += NT) {
+            const int r = i / R::NCH, ch = i - r * R::NCH, xx = xs + 4 * ch;
+            const float *p = row_of(r);
+            const bool on = p && xx >= 0 && xx < W;    // a chunk is inside the row or outside
+            conv_copy<16>(tile + r * R::RW + 4 * ch, on ? p + xx : x, on);
+        }
+    } else {
+        for (int i = tid; i < nrows * R::NCH * 4; i += NT) {
+            const int r = i / (R::NCH * 4), j = i - r * (R::NCH * 4), xx = xs + j;
+            const float *p = row_of(r);
+            const bool on = p && xx >= 0 && xx < W;
+            conv_copy<4>(tile + r * R::RW + j, on ? p + xx : x, on);
+        }
+    }
+    for (int i = tid; i < IC * 9 * OCP; i += NT) {
+        const int o = i % OCP, ct = i / OCP;           // ct = c * 9 + tap
+        sw[i] = o < OC ? __ldg(w + o * IC * 9 + ct) : 0.f;
+    }
+    if (tid < OC) sb[tid] = __ldg(b + tid);
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const int xg = tid & 7, ly = tid >> 3;
+    float tot[4][OC], half[4][OC];
+#pragma unroll
+    for (int g = 0; g < CS; ++g) {
+        float acc[4][OC];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int o = 0; o < OC; ++o) acc[q][o] = 0.f;
+#pragma unroll
+        for (int j = 0; j < CPS; ++j) {
+            const int c = g * CPS + j;
+#pragma unroll 1
+            for (int ky = 0; ky < 3; ++ky) {
+                const float *row = tile + (c * th + ly + ky * dil) * R::RW + 4 * xg;
+                float v[12];
+                if constexpr (DIL > 0) {
+#pragma unroll
+                    for (int e = 0; e < 12; e += 4) {
+                        const float4 f = *reinterpret_cast<const float4 *>(row + e);
+                        v[e] = f.x; v[e + 1] = f.y; v[e + 2] = f.z; v[e + 3] = f.w;
+                    }
+                } else if constexpr (DIL == 0) {
+#pragma unroll
+                    for (int e = 0; e < 12; ++e)
+                        v[e] = row[R::PAD + (e >> 2) * dil - dil + (e & 3)];
+                } else {
+                    const long yy = (long)oy0 + ly + (ky - 1l) * dil;
+#pragma unroll
+                    for (int e = 0; e < 12; ++e) {
+                        const long xx = (long)ox0 + 4 * xg + ((e >> 2) - 1l) * dil + (e & 3);
+                        v[e] = yy >= 0 && yy < H && xx >= 0 && xx < W ? __ldg(x + c * HW + yy * W + xx)
+                                                                    : 0.f;
+                    }
+                }
+#pragma unroll
+                for (int kx = 0; kx < 3; ++kx) {
+                    constexpr int V0 = DIL > 0 ? 4 - DIL : 0, VS = DIL > 0 ? DIL : 4;
+                    const float *wt = sw + (c * 9 + ky * 3 + kx) * OCP;
+                    float wv[OCP];
+                    if constexpr (OCP % 4 == 0) {
+#pragma unroll
+                        for (int o = 0; o < OCP; o += 4) {
+                            const float4 f = *reinterpret_cast<const float4 *>(wt + o);
+                            wv[o] = f.x; wv[o + 1] = f.y; wv[o + 2] = f.z; wv[o + 3] = f.w;
+                        }
+                    } else {
+#pragma unroll
+                        for (int o = 0; o < OCP; ++o) wv[o] = wt[o];
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+#pragma unroll
+                        for (int o = 0; o < OC; ++o)
+                            acc[q][o] = fmaf(v[V0 + kx * VS + q], wv[o], acc[q][o]);
+                }
+            }
+        }
+        // (s0 + s1) + (s2 + s3)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int o = 0; o < OC; ++o) {
+                if (g == 0) tot[q][o] = acc[q][o];
+                else if (g == 1) tot[q][o] = tot[q][o] + acc[q][o];
+                else if (g == 2) half[q][o] = acc[q][o];
+                else tot[q][o] = tot[q][o] + (half[q][o] + acc[q][o]);
+            }
+    }
+    const int ox = ox0 + 4 * xg, oy = oy0 + ly;
+    if (ox >= W || oy >= H) return;
+    const long oi = (long)oy * W + ox;
+    const bool out16 = (W & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+#pragma unroll
+    for (int o = 0; o < OC; ++o) {
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            v[q] = tot[q][o] + sb[o];
+            if (ACT == 1) v[q] = v[q] > 0.f ? v[q] : v[q] * 0.2f;
+            if (ACT == 2 && ox + q < W) {
+                v[q] = resid[oi + q] + v[q];
+                v[q] = v[q] > 0.f ? v[q] : v[q] * 0.f;
+            }
+        }
+        float *yo = y + o * HW + oi;
+        if (out16) {
+            *reinterpret_cast<float4 *>(yo) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (ox + q < W) yo[q] = v[q];
+        }
+    }
+}
+
+template <int IC, int OC, int ACT, int CS, int DIL>
+__global__ void __launch_bounds__(8 * CTR_TH, 4)
+    k_conv2d_rows(const float *__restrict__ x, int H, int W, int dil, const float *__restrict__ w,
+                  const float *__restrict__ b, float *y, const float *__restrict__ resid) {
+    pdl_sync();
+    conv2d_rows_body<IC, OC, ACT, CS, DIL>(blockIdx.x, blockIdx.y, x, H, W, dil, w, b, y, resid);
+}
+
+// The batched form: Refinement level lv - 3 of conv_level.
+template <int IC, int OC, int ACT, int CS, int DIL>
+__global__ void __launch_bounds__(8 * CTR_TH, 4)
+    k_b_conv2d_rows(NetLaunch L, int lv, const float *x, int dil, const float *__restrict__ w,
+                    const float *__restrict__ b, float *y, const float *resid) {
+    pdl_sync();
+    long long c;
+    const int p = net_pair(L, c);
+    const NetPair &P = L.pairs[p];
+    if (!P.active) return;
+    int H, W, OH, OW;
+    conv_level(lv, P.Hw, P.Ww, H, W, OH, OW);
+    const int tx = (W + CTR_TW - 1) / CTR_TW, ty = (H + CTR_TH - 1) / CTR_TH;
+    const int bx = (int)(c % tx), by = (int)(c / tx);
+    if (by >= ty) return;
+    conv2d_rows_body<IC, OC, ACT, CS, DIL>(bx, by, net_slab(x, L, p), H, W, dil, w, b,
+                                           net_slab(y, L, p), net_slab(resid, L, p));
+}
+
+template <int DIL>
+static size_t conv2d_rows_bytes(int IC, int dil) {
+    return DIL < 0 ? 0 : (size_t)IC * (CTR_TH + 2 * dil) * ConvRows<DIL>::RW * sizeof(float);
+}
+
+// One such convolution of a whole image (L NULL) or of a batch's pairs.
+template <int IC, int OC, int ACT, int CS, int DIL>
+static void conv2d_rows_go(const NetLaunch *L, unsigned ctas, int lv, int H, int W, const float *x,
+                           int dil, const float *w, const float *b, float *y, const float *resid,
+                           cudaStream_t st) {
+    const size_t smem = conv2d_rows_bytes<DIL>(IC, dil);
+    const size_t fixed = (size_t)(IC * 9 + 1) * ((OC + 3) / 4 * 4) * sizeof(float);
+    if (L) {
+        if (smem + fixed > 48 * 1024)
+            cudaFuncSetAttribute(k_b_conv2d_rows<IC, OC, ACT, CS, DIL>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        pdl(k_b_conv2d_rows<IC, OC, ACT, CS, DIL>, ctas, 8 * CTR_TH, smem, st)(*L, lv, x, dil, w, b,
+                                                                              y, resid);
+    } else {
+        if (smem + fixed > 48 * 1024)
+            cudaFuncSetAttribute(k_conv2d_rows<IC, OC, ACT, CS, DIL>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const dim3 g((W + CTR_TW - 1) / CTR_TW, (H + CTR_TH - 1) / CTR_TH);
+        pdl(k_conv2d_rows<IC, OC, ACT, CS, DIL>, g, 8 * CTR_TH, smem, st)(x, H, W, dil, w, b, y,
+                                                                         resid);
+    }
+}
+
+// dilations 1, 2 and 4 (the shipped nets') compiled in
+template <int IC, int OC, int ACT, int CS>
+static void conv2d_rows(const NetLaunch *L, unsigned ctas, int lv, int H, int W, const float *x,
+                        int dil, const float *w, const float *b, float *y, const float *resid,
+                        cudaStream_t st) {
+    if (dil == 1) conv2d_rows_go<IC, OC, ACT, CS, 1>(L, ctas, lv, H, W, x, dil, w, b, y, resid, st);
+    else if (dil == 2) conv2d_rows_go<IC, OC, ACT, CS, 2>(L, ctas, lv, H, W, x, dil, w, b, y, resid, st);
+    else if (dil == 4) conv2d_rows_go<IC, OC, ACT, CS, 4>(L, ctas, lv, H, W, x, dil, w, b, y, resid, st);
+    else if (dil >= 0 && dil <= 8)
+        conv2d_rows_go<IC, OC, ACT, CS, 0>(L, ctas, lv, H, W, x, dil, w, b, y, resid, st);
+    else conv2d_rows_go<IC, OC, ACT, CS, -1>(L, ctas, lv, H, W, x, dil, w, b, y, resid, st);
 }
 
 // A Refinement level's first convolution (2 -> RC, stride 1, dilation dil,
@@ -1405,6 +1620,12 @@ static int forward_bf16_front(const NetView &n, const float *left, const float *
     return launch_conv_tc(v, st);
 }
 
+// Refinement levels of at least so many pixels take k_conv2d_rows; below, its blocks
+// are fewer than the SMs and k_conv2d_tiled's shorter chains win (a 450 x 375 pair,
+// levels up to 38,000 pixels: 399 us, 407 with k_conv2d_rows from 12,000 on; a 320 x
+// 266 forward: 246 us without it at 85,000, 224 with).
+constexpr long kRowsMin = 40000;
+
 // The network shapes this build instantiates: the reference's shipped
 // architectures (feat_C, cost_C, refine_C) = (12, 6, 8), (8, 4, 8), (8, 4, 4),
 // (16, 8, 8) with D <= 16.
@@ -1473,6 +1694,7 @@ static int forward_impl(const NetView &n, const float *left, const float *right,
     for (int lv = 0; lv < 2; ++lv) {
         const int Hl = Hs[lv], Wl = Ws[lv];
         const float *cur = nullptr;
+        const bool rows = (long)Hl * Wl >= kRowsMin;
         float *bufs[2] = {b.ra, b.rb};
         constexpr int RG = RC % 4 == 0 ? 4 : RC;
         constexpr int RS = RC % 4 == 0 ? 4 : 2;     // lanes per output of the dilated convs
@@ -1484,6 +1706,9 @@ static int forward_impl(const NetView &n, const float *left, const float *right,
                 pdl(k_conv2d_up<RC, RG>, tgrid(Wl, Hl, RC / RG), tb, conv2d_tile_bytes(2, 1, dl),
                                       st)(prev, ph, pw, guides[lv], Hl, Wl, dl, n.rw[lv][i],
                                             n.rb[lv][i], dst, b.rin);
+            else if (rows && dl >= 0 && dl <= 8)
+                conv2d_rows<RC, RC, 1, RS>(nullptr, 0, 0, Hl, Wl, cur, dl, n.rw[lv][i], n.rb[lv][i],
+                                           dst, nullptr, st);
             else            // every output channel per thread (measured faster)
                 pdl(k_conv2d_tiled<RC, RC, RC, 1, RS>, tgrid(Wl, Hl, 1), RS * tb1,
                                                     conv2d_tile_bytes(RC, 1, dl, RS), st)(
@@ -1498,6 +1723,9 @@ static int forward_impl(const NetView &n, const float *left, const float *right,
                                             outs[lv], b.rin, *b.decide->width,
                                             b.decide->state, b.decide->hist,
                                             b.decide->mirror);
+        else if (rows)
+            conv2d_rows<RC, 1, 2, 4>(nullptr, 0, 0, Hl, Wl, cur, 1, n.rw[lv][n.ndil],
+                                     n.rb[lv][n.ndil], outs[lv], b.rin, st);
         else
             pdl(k_conv2d_tiled<RC, 1, 1, 2, 4>, tgrid(Wl, Hl, 1), tb4,
                                              conv2d_tile_bytes(RC, 1, 1, 4), st)(
@@ -1573,9 +1801,12 @@ static void stage_ctas_impl(const NetView &n, int Hm, int Wm, long long *o) {
     o[NK_V2] = (long long)((w + G2::TX - 1) / G2::TX) * h * ((D + G2::TD - 1) / G2::TD);
     o[NK_SA] = (long long)cx * h;
     o[NK_R0] = (long long)(RC / RG) * t2(Wm / 2, Hm / 2);
-    o[NK_R0F] = t2(Wm / 2, Hm / 2);
+    auto tr = [](int OW, int OH) {
+        return (long long)((OW + CTR_TW - 1) / CTR_TW) * ((OH + CTR_TH - 1) / CTR_TH);
+    };
+    o[NK_R0F] = tr(Wm / 2, Hm / 2);
     o[NK_R1] = (long long)(RC / RG) * t2(Wm, Hm);
-    o[NK_R1F] = t2(Wm, Hm);
+    o[NK_R1F] = tr(Wm, Hm);
     o[NK_C1W] = 2LL * t2(w1, h1);            // k_b_conv2d_wide: both images, all channels
     o[NK_C2W] = 2LL * t2(w, h);
 }
@@ -1603,7 +1834,6 @@ static int b_forward_impl(const NetView &n, const NetStageLaunch &g, const NetSl
     const int D = n.D;
     auto L = [&](int k) { return NetLaunch{g.pre[k], g.pairs, g.n, g.slab}; };
     auto B = [&](int k) { return ctas_of(g.total[k]); };
-    const int tb1 = CT2_TW * CT2_TH;
     const dim3 tb(CT2_TW, CT2_TH);
     // FeatureNet, both images: every output channel and 2 pixels per thread
     // (the arithmetic of k_conv2d_tiled<.., FG, .., 1 or 2>)
@@ -1637,7 +1867,7 @@ static int b_forward_impl(const NetView &n, const NetStageLaunch &g, const NetSl
     const float *guides[2] = {s.gh, s.lw};
     const float *prevs[2] = {s.d0, s.d1};
     float *outs[2] = {s.d1, s.d2};
-    const bool tiled = RC > 8;     // the register-blocked form holds at most 8 channels
+    static_assert(RC <= 8, "k_b_conv2d_rows holds at most 8 channels");
     for (int lv = 0; lv < 2; ++lv) {
         const int kk = lv ? NK_R1 : NK_R0, kf = lv ? NK_R1F : NK_R0F;
         float *bufs[2] = {s.f.ra, s.f.rb};
@@ -1649,27 +1879,17 @@ static int b_forward_impl(const NetView &n, const NetStageLaunch &g, const NetSl
             if (i == 0)
                 pdl(k_b_conv2d_up<RC, RG>, B(kk), tb, conv2d_tile_bytes(2, 1, dl), st)(
                     L(kk), lv, prevs[lv], guides[lv], dl, n.rw[lv][i], n.rb[lv][i], dst, s.f.rin);
-            else if (!tiled)
-                b_conv2d_wide<RC, RC, 1, RS, 2, 1>(L(kf), B(kf), lv + 3, 1, cur, cur, dl,
-                                                   n.rw[lv][i], n.rb[lv][i], dst, dst, nullptr,
-                                                   st);
-            else
-                pdl(k_b_conv2d_tiled<RC, RC, RG, 1, RS>, B(kk), RS * tb1,
-                                                      conv2d_tile_bytes(RC, 1, dl, RS), st)(
-                    L(kk), 3 + lv, RC / RG, cur, cur, 1, dl, dl, n.rw[lv][i], n.rb[lv][i], dst,
-                    dst, nullptr);
+            else {
+                const NetLaunch l = L(kf);
+                conv2d_rows<RC, RC, 1, RS>(&l, B(kf), lv + 3, 0, 0, cur, dl, n.rw[lv][i],
+                                           n.rb[lv][i], dst, nullptr, st);
+            }
             cur = dst;
         }
         count_launch();
-        if (!tiled)
-            b_conv2d_wide<RC, 1, 2, 4, 2, 1>(L(kf), B(kf), lv + 3, 1, cur, cur, 1,
-                                             n.rw[lv][n.ndil], n.rb[lv][n.ndil], outs[lv],
-                                             outs[lv], s.f.rin, st);
-        else
-            pdl(k_b_conv2d_tiled<RC, 1, 1, 2, 4>, B(kf), 4 * tb1, conv2d_tile_bytes(RC, 1, 1, 4),
-                                               st)(L(kf), 3 + lv, 1, cur, cur, 1, 1, 1,
-                                                     n.rw[lv][n.ndil], n.rb[lv][n.ndil],
-                                                     outs[lv], outs[lv], s.f.rin);
+        const NetLaunch l = L(kf);
+        conv2d_rows<RC, 1, 2, 4>(&l, B(kf), lv + 3, 0, 0, cur, 1, n.rw[lv][n.ndil],
+                                 n.rb[lv][n.ndil], outs[lv], s.f.rin, st);
         SV_LAUNCH_CHECK();
     }
     return SV_OK;
