@@ -106,6 +106,93 @@ __device__ __forceinline__ void census_tile(const T *__restrict__ img, int W, in
     out[(long)y * W + x] = s;
 }
 
+// The same tile of an 8-bit image and the 9 x 7 window by 64 threads, 4 pixels each,
+// a byte of every register per pixel.  lt's top bits are x < c: with d = (x | 0x80) -
+// (c & 0x7F) in each byte (no borrow leaves it), the top bit of d says x >= c where
+// the top bits of x and c agree, and c's own says x < c where they differ.  The
+// neighbours come in ascending bit order and are shifted in at the top, so 8 of them
+// leave a finished byte of each pixel's word.  What bounds it is the integer pipe: 6
+// instructions per neighbour for 4 pixels instead of 4 for one (20 pairs, 20 million
+// pixels of both views: 433 us, now 175).
+constexpr int kCen8Threads = 64;
+__device__ __forceinline__ void census_tile_u8(const uint8_t *__restrict__ img, int W, int H,
+                                               uint64_t *__restrict__ out, int tx0, int ty0,
+                                               unsigned *tile) {
+    constexpr int RX = 4, RY = 3, SW = (CT_W + 2 * RX) / 4, SH = CT_H + 2 * RY;
+    constexpr unsigned TOP = 0x80808080u;
+    const int tid = threadIdx.x;
+    const bool vec = (W & 3) == 0 && (reinterpret_cast<uintptr_t>(img) & 3) == 0;
+    unsigned v[(SW * SH + kCen8Threads - 1) / kCen8Threads];
+#pragma unroll
+    for (int u = 0; u < (SW * SH + kCen8Threads - 1) / kCen8Threads; ++u) {
+        const int i = tid + u * kCen8Threads, sy = i / SW, gx = tx0 - RX + 4 * (i - sy * SW);
+        const uint8_t *row = img + (long)min(max(ty0 + sy - RY, 0), H - 1) * W;
+        if (vec && gx >= 0 && gx + 3 < W) {
+            v[u] = __ldg(reinterpret_cast<const unsigned *>(row + gx));
+        } else {
+            v[u] = 0u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                v[u] |= (unsigned)__ldg(row + min(max(gx + j, 0), W - 1)) << (8 * j);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < (SW * SH + kCen8Threads - 1) / kCen8Threads; ++u)
+        if (tid + u * kCen8Threads < SW * SH) tile[tid + u * kCen8Threads] = v[u];
+    __syncthreads();
+    const int xg = tid & 7, ly = tid >> 3;
+    const unsigned *t = tile + ly * SW + xg;               // the window's first row
+    const unsigned c = t[RY * SW + 1], c7 = c & ~TOP;
+    unsigned bytes[8], acc = 0u;
+    int b = 0;
+#pragma unroll
+    for (int dy = 2 * RY; dy >= 0; --dy) {
+        const unsigned w[3] = {t[dy * SW], t[dy * SW + 1], t[dy * SW + 2]};
+#pragma unroll
+        for (int dx = 2 * RX; dx >= 0; --dx) {
+            if (dy == RY && dx == RX) continue;
+            const unsigned x = dx % 4 == 0 ? w[dx / 4]
+                                           : __funnelshift_r(w[dx / 4], w[dx / 4 + (dx < 8)], 8 * (dx % 4));
+            const unsigned d = (x | TOP) - c7;
+            const unsigned lt = (~x & c) | (~(x ^ c) & ~d);
+            acc = ((acc >> 1) & ~TOP) | (lt & TOP);
+            if ((++b & 7) == 0) bytes[b / 8 - 1] = acc;
+        }
+    }
+    bytes[7] = (acc >> 2) & 0x3F3F3F3Fu;                   // 62 neighbours
+    const int x = tx0 + 4 * xg, y = ty0 + ly;
+    if (x >= W || y >= H) return;
+    uint64_t r[4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {                          // 4 x 4 bytes transposed
+        const unsigned *q = bytes + 4 * h;
+        const unsigned a0 = __byte_perm(q[0], q[1], 0x5140), a1 = __byte_perm(q[2], q[3], 0x5140),
+                       a2 = __byte_perm(q[0], q[1], 0x7362), a3 = __byte_perm(q[2], q[3], 0x7362);
+        const unsigned o[4] = {__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632),
+                               __byte_perm(a2, a3, 0x5410), __byte_perm(a2, a3, 0x7632)};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r[j] = h ? r[j] | (uint64_t)o[j] << 32 : (uint64_t)o[j];
+    }
+    uint64_t *p = out + (long)y * W + x;
+    if ((W & 1) == 0 && x + 3 < W && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+        *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(r[0], r[1]);
+        *reinterpret_cast<ulonglong2 *>(p + 2) = make_ulonglong2(r[2], r[3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (x + j < W) p[j] = r[j];
+    }
+}
+
+__global__ void __launch_bounds__(kCen8Threads)
+    k_census_u8(const uint8_t *__restrict__ img0, const uint8_t *__restrict__ img1, int W, int H,
+                uint64_t *__restrict__ out0, uint64_t *__restrict__ out1) {
+    pdl_sync();
+    __shared__ unsigned tile[(CT_W + 8) / 4 * (CT_H + 6)];
+    census_tile_u8(blockIdx.z ? img1 : img0, W, H, blockIdx.z ? out1 : out0, blockIdx.x * CT_W,
+                   blockIdx.y * CT_H, tile);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(CT_W *CT_H)
     k_census(const T *__restrict__ img0, const T *__restrict__ img1, int W, int H,
@@ -508,6 +595,12 @@ int launch_census(const void *img0, const void *img1, int dtype, int W, int H,
     size_t cells = (size_t)(CT_W + 2 * rx) * (CT_H + 2 * ry);
     switch (dtype) {
     case SV_U8:
+        if (rx == 4 && ry == 3) {
+            count_launch();
+            pdl(k_census_u8, grd, kCen8Threads, 0, st)((const uint8_t *)img0, (const uint8_t *)img1,
+                                                       W, H, out0, out1);
+            break;
+        }
         count_launch(); pdl(k_census<uint8_t>, grd, blk, cells * 1, st)(
             (const uint8_t *)img0, (const uint8_t *)img1, W, H, rx, ry, out0, out1);
         break;
@@ -647,6 +740,18 @@ __global__ void __launch_bounds__(CT_W *CT_H) k_b_census(BatchTables t) {
                    reinterpret_cast<T *>(smem_raw));
 }
 
+__global__ void __launch_bounds__(kCen8Threads) k_b_census_u8(BatchTables t) {
+    pdl_sync();
+    __shared__ unsigned tile[(CT_W + 8) / 4 * (CT_H + 6)];
+    const int i = batch_find(t.tile_blk, t.n, blockIdx.x);
+    const BatchPair &P = t.pairs[i];
+    const int tiles_x = (P.W + CT_W - 1) / CT_W;
+    const int tl = (int)(blockIdx.x - t.tile_blk[i]);
+    const int ty = tl / tiles_x, tx = tl - ty * tiles_x;
+    census_tile_u8(reinterpret_cast<const uint8_t *>(blockIdx.z ? P.right : P.left), P.W, P.H,
+                   blockIdx.z ? P.cen1 : P.cen0, tx * CT_W, ty * CT_H, tile);
+}
+
 __global__ void __launch_bounds__(256) k_b_lr_check(BatchTables t) {
     pdl_sync();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -672,7 +777,10 @@ int launch_batch_front(const BatchTables &t, long long px_blocks, long long rows
     const dim3 g((unsigned)tiles, 1, 2), blk(CT_W, CT_H);
     count_launch();
     switch (t.dtype) {
-    case SV_U8: pdl(k_b_census<uint8_t>, g, blk, cells, st)(t); break;
+    case SV_U8:
+        if (t.rx == 4 && t.ry == 3) pdl(k_b_census_u8, g, kCen8Threads, 0, st)(t);
+        else pdl(k_b_census<uint8_t>, g, blk, cells, st)(t);
+        break;
     case SV_F32: pdl(k_b_census<float>, g, blk, cells * 4, st)(t); break;
     case SV_F64: pdl(k_b_census<double>, g, blk, cells * 8, st)(t); break;
     default: set_error("unknown image dtype %d", t.dtype); return SV_ERR_PARAM;
