@@ -176,7 +176,7 @@ extern "C" int sv_refine_fullres_noalloc(const void *left, const void *right, in
     // the sum above take 16 bytes per pixel
     const size_t o_base = 256;
     const size_t o_c = o_base + up256(N * 4);
-    const size_t o_l = o_c + up256(N * cost_row_bytes(K));
+    const size_t o_l = o_c + up256(N * cost_row_bytes(K, false));
     const size_t o_cl = o_l;
     const size_t o_cr = o_cl + up256(N * 8);
     char *s = nullptr;
@@ -193,7 +193,7 @@ extern "C" int sv_refine_fullres_noalloc(const void *left, const void *right, in
     if ((rc = launch_base(disp0, (long)N, base, flag, st))) return rc;
     if ((rc = launch_census(left, right, dtype, W, H, p->rx, p->ry, cl, cr, st))) return rc;
     if ((rc = launch_band_costs_slot(cl, cr, base, nullptr, W, H, p->R, invalid, C, nullptr, 1,
-                                    st)))
+                                    st, nullptr, false)))
         return rc;
     if ((rc = launch_sgm_packed(C, nullptr, base, nullptr, W, H, K, P1, P2, L, l16, false, 1,
                                npaths, st)))

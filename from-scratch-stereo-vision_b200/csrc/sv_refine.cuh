@@ -49,8 +49,8 @@ inline SgmTasks make_sgm_tasks(int W, int H, int nviews, int npaths, const int *
 // Slots per pixel of the fused refinement's layout (K + 2 rounded up to a
 // table width) and the bytes of a pixel's cost and path-cost rows (sv_sgm.cu).
 // pad: path-cost rows of the 24-slot layout padded to 32 bytes.
-int slot_width(int K);
-size_t cost_row_bytes(int K);
+int slot_width(int K, bool pad = true);
+size_t cost_row_bytes(int K, bool pad = true);
 size_t path_row_bytes(int K, bool l16, bool pad);
 
 // Validated refinement parameters (sv_api.cu).
@@ -145,7 +145,7 @@ int launch_sgm_add_path(const uint8_t *C, const int32_t *base, int W, int H, int
 int launch_band_costs_slot(const uint64_t *cl, const uint64_t *cr, const int32_t *base0,
                            const int32_t *base1, int W, int H, int R, int invalid, uint8_t *C0,
                            uint8_t *C1, int nviews, cudaStream_t st,
-                           const uint8_t *rad0 = nullptr);
+                           const uint8_t *rad0 = nullptr, bool pad = true);
 int launch_sgm_packed(const uint8_t *C0, const uint8_t *C1, const int32_t *b0,
                       const int32_t *b1, int W, int H, int K, int P1, int P2, void *Lout,
                       bool l16, bool pad, int nviews, int npaths, cudaStream_t st);

@@ -321,7 +321,9 @@ struct SgmRing {
     static constexpr int Kp = 2 * NR * GL, NW = NR / 2;
     static constexpr bool INROW = Kp == 24;         // the band centre is in the cost row
     static constexpr int LB = INROW ? 16 : 2 * NR;  // cost bytes a lane copies per pixel
-    static constexpr int PB = LB % 16 == 0 ? 16 : 8, NP = LB / PB;
+    // the widest copy that every lane's share of a row is aligned to
+    static constexpr int PB = LB % 16 == 0 ? 16 : LB % 8 == 0 ? 8 : 4, NP = LB / PB;
+    static_assert(LB % PB == 0, "a lane's share in whole copies");
     static constexpr int SLOT = 32 * (LB + (INROW ? 0 : 4));     // bytes per pixel of a warp
     static constexpr int PF = NR > 8 ? 8 : 16;      // pixels
     static constexpr int WARP = PF * SLOT;
@@ -382,10 +384,12 @@ __device__ __forceinline__ void sgm_scan(const uint8_t *__restrict__ C,
                     c[4 * i + 1] = v.y;
                     c[4 * i + 2] = v.z;
                     c[4 * i + 3] = v.w;
-                } else {
+                } else if constexpr (Rg::PB == 8) {
                     const uint2 v = lds64(q);
                     c[2 * i] = v.x;
                     c[2 * i + 1] = v.y;
+                } else {
+                    c[i] = (unsigned)lds32(q);
                 }
             }
             b = lds32(mineb + off);
@@ -818,23 +822,26 @@ __global__ void __launch_bounds__(256)
 // Host
 // ====================================================================
 
-int slot_width(int K) {
+// Slots of a pixel.  Without padding (the static scratch) also 48: a lane's share of
+// such a row is no 16-byte copy, and 64 slots are faster although they are more (500 x
+// 150, K = 31: 271 us a pass, 328 with 48).
+int slot_width(int K, bool pad) {
     static const int widths[] = {8, 16, 24, 32, 48, 64, 96, 128, 160, 192, 224, 256};
     for (int w : widths)
-        if (w >= K + 2) return w;
+        if (w >= K + 2 && (w != 48 || !pad)) return w;
     return 256;
 }
 
-size_t cost_row_bytes(int K) { return cost_row(slot_width(K)); }
+size_t cost_row_bytes(int K, bool pad) { return cost_row(slot_width(K, pad)); }
 size_t path_row_bytes(int K, bool l16, bool pad) {
-    return l16 ? 2 * slot_width(K) : path_row(slot_width(K), pad);
+    return l16 ? 2 * slot_width(K, pad) : path_row(slot_width(K, pad), pad);
 }
 
 int launch_band_costs_slot(const uint64_t *cl, const uint64_t *cr, const int32_t *base0,
                            const int32_t *base1, int W, int H, int R, int invalid, uint8_t *C0,
-                           uint8_t *C1, int nviews, cudaStream_t st, const uint8_t *rad0) {
+                           uint8_t *C1, int nviews, cudaStream_t st, const uint8_t *rad0, bool pad) {
     const long N = (long)W * H;
-    const int K = 2 * R + 1, Kp = slot_width(K);
+    const int K = 2 * R + 1, Kp = slot_width(K, pad);
     const dim3 px(grid_for(N, Kp == 24 ? 256 : 256 / (Kp / 8), 148 * 8), nviews);
     count_launch();
     if (K == 21)    // R = 10, the refine_disparity default
@@ -872,19 +879,23 @@ static int sgm_go(const uint8_t *C0, const uint8_t *C1, const int32_t *b0, const
 
 template <typename LT, bool PAD>
 static int sgm_dispatch(const uint8_t *C0, const uint8_t *C1, const int32_t *b0,
-                        const int32_t *b1, int W, int H, int K, int P1, int P2, void *Lout,
+                        const int32_t *b1, int W, int H, int K, int Kp, int P1, int P2, void *Lout,
                         int nviews, int npaths, cudaStream_t st) {
+    // More lanes shorten a step, whose latency a warp alone on its scheduler pays; the
+    // fewest registers per lane that leave 16-byte copies (640 x 480, a pass: K = 49 2
+    // lanes 460 us, 4 414; K = 101 4 lanes 660, 8 634; K = 25 2 lanes 311, 4 and 8-byte
+    // copies 326).
 #define SV_SGM(NR, GL) \
     return sgm_go<NR, GL, LT, PAD>(C0, C1, b0, b1, W, H, K, P1, P2, Lout, nviews, npaths, st)
-    switch (slot_width(K)) {
+    switch (Kp) {
     case 8: SV_SGM(4, 1);
     case 16: SV_SGM(4, 2);
     case 24: SV_SGM(6, 2);
     case 32: SV_SGM(8, 2);
-    case 48: SV_SGM(12, 2);
-    case 64: SV_SGM(16, 2);
+    case 48: SV_SGM(6, 4);
+    case 64: SV_SGM(8, 4);
     case 96: SV_SGM(12, 4);
-    case 128: SV_SGM(16, 4);
+    case 128: SV_SGM(8, 8);
     case 160: SV_SGM(20, 4);
     case 192: SV_SGM(24, 4);
     case 224: SV_SGM(28, 4);
@@ -899,11 +910,12 @@ static int sgm_dispatch(const uint8_t *C0, const uint8_t *C1, const int32_t *b0,
 int launch_sgm_packed(const uint8_t *C0, const uint8_t *C1, const int32_t *b0,
                       const int32_t *b1, int W, int H, int K, int P1, int P2, void *Lout,
                       bool l16, bool pad, int nviews, int npaths, cudaStream_t st) {
+    const int Kp = slot_width(K, pad);
     if (l16)
-        return sgm_dispatch<uint16_t, false>(C0, C1, b0, b1, W, H, K, P1, P2, Lout, nviews, npaths, st);
+        return sgm_dispatch<uint16_t, false>(C0, C1, b0, b1, W, H, K, Kp, P1, P2, Lout, nviews, npaths, st);
     if (pad)
-        return sgm_dispatch<uint8_t, true>(C0, C1, b0, b1, W, H, K, P1, P2, Lout, nviews, npaths, st);
-    return sgm_dispatch<uint8_t, false>(C0, C1, b0, b1, W, H, K, P1, P2, Lout, nviews, npaths, st);
+        return sgm_dispatch<uint8_t, true>(C0, C1, b0, b1, W, H, K, Kp, P1, P2, Lout, nviews, npaths, st);
+    return sgm_dispatch<uint8_t, false>(C0, C1, b0, b1, W, H, K, Kp, P1, P2, Lout, nviews, npaths, st);
 }
 
 int launch_wta_slot(const void *L, bool l16, bool pad, int npaths, int nviews, int W, int H, int R,
@@ -911,7 +923,7 @@ int launch_wta_slot(const void *L, bool l16, bool pad, int npaths, int nviews, i
                     double uniq, double *out0, double *out1, double *conf0, cudaStream_t st) {
     const long N = (long)W * H;
     const int K = 2 * R + 1;
-    const int Kp = slot_width(K);
+    const int Kp = slot_width(K, pad);
     count_launch();
     if (nviews < 1 || nviews > 2) {
         set_error("wta: nviews=%d", nviews);
