@@ -141,7 +141,12 @@ const int kClOrder[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11, 4, 12, 3, 13, 2,
 // all that a symbol needs: bits 0-3 the code's length, 4-7 the extra bits', 8-9 the
 // kind, 16-31 the literal or the base of the length or distance.  A code longer
 // than the table, an unused one and the end of the block have the kind kOther.
-constexpr int kLitBits = 12, kDistBits = 11;
+// Building the tables costs what some 200 symbols save, so a block decodes symbol by
+// symbol until it has taken kFastAfter bytes (640 x 480 gray in blocks of 128 symbols:
+// 7.1 ms with 12- and 11-bit tables for every block, 4.6 so and without a fast loop;
+// blocks of 16,000 symbols: 1.09, 1.08 and 1.76 ms).
+constexpr int kLitBits = 10, kDistBits = 9;
+constexpr size_t kFastAfter = 512;
 constexpr uint32_t kLiteral = 0u << 8, kCopy = 1u << 8, kOther = 2u << 8;
 struct FastTables {
     uint32_t lit[1 << kLitBits], dist[1 << kDistBits];
@@ -220,8 +225,11 @@ struct Out {
 // bounds it is the chain from one symbol's length to the next one's bits and the
 // branch between literals and copies; so a word of input serves three literals, a
 // copy's length and distance each take one table entry, and copies go 8 bytes at a
-// time.  A 450 x 375 RGB image of 260,000 symbols inflates in 2.1 ms (3.0 symbol by
-// symbol through codes(); 3.1 with one branch-free path for literals and copies).
+// time.  (The refill -- whole words ORed in above the bits held, the position moved by
+// the whole bytes taken -- is the published branch-free one; see Fabian Giesen's
+// "Reading bits in far too many ways", part 2, variant 4.)  A 450 x 375 RGB image of
+// 260,000 symbols inflates in 2.1 ms (3.0 symbol by symbol through codes(); 3.1 with
+// one branch-free path for literals and copies).
 void codes_fast(BitIn &b, const FastTables &f, Out &out) {
     uint64_t buf = b.buf;
     unsigned cnt = (unsigned)b.cnt;
@@ -260,7 +268,7 @@ void codes_fast(BitIn &b, const FastTables &f, Out &out) {
             cnt |= 56;
         }
         if (e & kOther) break;
-        // length (12 + 5 bits at most), distance (11 + 13): 41 of at least 56 bits
+        // length (10 + 5 bits at most), distance (9 + 13): 37 of at least 56 bits
         const unsigned lc = e & 15, le = (e >> 4) & 15;
         const uint64_t b1 = buf >> lc, b2 = b1 >> le;
         const uint32_t ed = f.dist[b2 & DM];
@@ -295,11 +303,14 @@ void codes_fast(BitIn &b, const FastTables &f, Out &out) {
 // The symbols of one Huffman block.  The bit buffer and the output cursor
 // live in locals for the loop (stores of output bytes may alias anything
 // reachable through a pointer); the slow bit-at-a-time decode and buffer
-// growth write them back first.
-bool codes(BitIn &b, const Code &lit, const Code &dist, const FastTables &fast, Out &out) {
+// growth write them back first.  fast: the block's tables, or NULL to have make()
+// build them when the block has taken kFastAfter bytes of input.
+template <typename M>
+bool codes(BitIn &b, const Code &lit, const Code &dist, const FastTables *fast, M make, Out &out) {
     uint64_t buf = b.buf;
     int cnt = b.cnt;
     size_t pos = b.pos, size = out.size;
+    const size_t fast_at = pos + kFastAfter;
     const uint8_t *const p = b.p;
     const size_t n = b.n;
     uint8_t *o = out.v.data();
@@ -345,10 +356,11 @@ bool codes(BitIn &b, const Code &lit, const Code &dist, const FastTables &fast, 
         return v;
     };
     for (;;) {
-        if (pos + 8 <= n && size + 3 + 258 + 8 <= cap) {    // up to the next special symbol
+        if (!fast && pos >= fast_at) fast = make();
+        if (fast && pos + 8 <= n && size + 3 + 258 + 8 <= cap) {   // up to the next special symbol
             sync_out();
             out.size = size;
-            codes_fast(b, fast, out);
+            codes_fast(b, *fast, out);
             sync_in();
             size = out.size;
         }
@@ -406,8 +418,8 @@ bool inflate_raw(const uint8_t *p, size_t n, Out &out) {
             out.size += rest;
             b.pos += rest;
         } else if (type == 1) {
-            if (!codes(b, fixed_codes().lit, fixed_codes().dist, fixed_codes().fast, out))
-                return false;
+            const FixedCodes &f = fixed_codes();
+            if (!codes(b, f.lit, f.dist, &f.fast, [&] { return &f.fast; }, out)) return false;
         } else if (type == 2) {
             const int nlen = (int)b.get(5) + 257, ndist = (int)b.get(5) + 1,
                       ncode = (int)b.get(4) + 4;
@@ -443,8 +455,11 @@ bool inflate_raw(const uint8_t *p, size_t n, Out &out) {
             }
             Code lit, dist;
             if (!build(lit, lens, nlen) || !build(dist, lens + nlen, ndist)) return false;
-            build_fast(fast, lit, lens, nlen, dist, lens + nlen, ndist);
-            if (!codes(b, lit, dist, fast, out)) return false;
+            const auto make = [&]() -> const FastTables * {
+                build_fast(fast, lit, lens, nlen, dist, lens + nlen, ndist);
+                return &fast;
+            };
+            if (!codes(b, lit, dist, nullptr, make, out)) return false;
         } else {
             return false;
         }
