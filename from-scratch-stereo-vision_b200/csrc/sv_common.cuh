@@ -67,6 +67,19 @@ struct DevFlags {
         }                                                                        \
     } while (0)
 
+// Ahead of a launch with `bytes` of dynamic shared memory: lifts the kernel's limit over
+// the default 48 KB (less the static shared memory, below 10 KB in every kernel here).
+// The limit belongs to the kernel, not to the launch, so it is always set to `most`, the
+// same for every call: a call's own size would take away what another host thread, between
+// its own setting and its launch, has asked for, and that launch would be refused.
+template <typename... P>
+inline int allow_smem(void (*kernel)(P...), size_t bytes, size_t most) {
+    if (bytes > 38 * 1024)
+        SV_CUDA_TRY(cudaFuncSetAttribute((const void *)kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    return SV_OK;
+}
+
 // Launch of a kernel that may be set up before the kernel ahead of it in the stream
 // has ended (programmatic stream serialization): pdl(kernel, grid, block, shared
 // bytes, stream)(arguments...).  The kernel starts with pdl_sync().  Most launches

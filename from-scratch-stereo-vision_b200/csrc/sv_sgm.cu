@@ -867,9 +867,8 @@ static int sgm_go(const uint8_t *C0, const uint8_t *C1, const int32_t *b0, const
     int warps = (plan.total + blocks - 1) / blocks;
     if (warps > MAXW) warps = MAXW;
     const size_t smem = (size_t)warps * SgmRing<NR, GL>::WARP;
-    if (smem > 48 * 1024)
-        SV_CUDA_TRY(cudaFuncSetAttribute(k_sgm_scan<NR, GL, LT, PAD>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int rc = allow_smem(k_sgm_scan<NR, GL, LT, PAD>, smem, MAXW * SgmRing<NR, GL>::WARP);
+    if (rc) return rc;
     count_launch();
     pdl(k_sgm_scan<NR, GL, LT, PAD>, blocks, warps * 32, smem, st)(
         C0, C1, b0, b1, plan, (K - 1) / 2, K, P1, P2, (LT *)Lout);
@@ -1054,9 +1053,8 @@ static int batch_sgm_go(const BatchTables &t, long long tasks, int threads, int 
     const long long cap = (long long)sms * (ctas_per_sm < 4 ? 1 : ctas_per_sm / 4);
     const unsigned blocks = (unsigned)(want < cap ? (want < 1 ? 1 : want) : cap);
     const size_t smem = (size_t)(threads / 32) * SgmRing<NR, GL>::WARP;
-    if (smem > 48 * 1024)
-        SV_CUDA_TRY(cudaFuncSetAttribute(k_b_sgm<NR, GL, LT, PAD>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int rc = allow_smem(k_b_sgm<NR, GL, LT, PAD>, smem, 256 / 32 * SgmRing<NR, GL>::WARP);
+    if (rc) return rc;
     count_launch();
     pdl(k_b_sgm<NR, GL, LT, PAD>, blocks, threads, smem, st)(t, tasks);
     SV_LAUNCH_CHECK();

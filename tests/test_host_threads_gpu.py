@@ -1,0 +1,77 @@
+"""Calls of several host threads, each with its own stream, workspace and sizes.
+
+A kernel's dynamic shared-memory limit belongs to the kernel, not to the call, so two
+calls that need different amounts must not lower it for each other: every call returns
+without an error, with the bits of the same call made alone.  The sizes are the ones
+whose kernels ask for different amounts above the default 48 KB; most are small
+images, so that the host's part of a call (where the threads meet) is most of it."""
+
+import threading
+from importlib import import_module
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _together(jobs, n):
+    """jobs: [(call(stream), outputs)]; each call once alone, then n times in a thread
+    of its own beside the others."""
+    streams = [torch.cuda.Stream() for _ in jobs]
+    want = []
+    torch.cuda.synchronize()
+    for (call, outs), s in zip(jobs, streams):
+        call(s.cuda_stream)
+        s.synchronize()
+        want.append([o.clone() for o in outs])
+    torch.cuda.synchronize()
+    errors = []
+    gate = threading.Barrier(len(jobs))
+
+    def work(call, stream):
+        gate.wait()
+        for _ in range(n):
+            try:
+                call(stream.cuda_stream)
+            except Exception as e:                       # every refused call counts
+                errors.append(str(e))
+        stream.synchronize()
+
+    threads = [threading.Thread(target=work, args=(j[0], s)) for j, s in zip(jobs, streams)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors, (len(errors), errors[0])
+    for (_, outs), w in zip(jobs, want):
+        for a, b in zip(outs, w):
+            assert torch.equal(a, b)
+
+
+def _images(seed, W, H):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    left = torch.randint(0, 256, (H, W), dtype=torch.uint8, device="cuda", generator=g)
+    right = torch.roll(left, -3, 1)
+    d0 = 3.0 + torch.rand(H * W, dtype=torch.float64, device="cuda", generator=g)
+    return left.ravel(), right.ravel().contiguous(), d0
+
+
+def _refine_job(svb, W, H, **kw):
+    refine = import_module(svb.__name__ + ".refine")
+    r = refine.LRRefiner(W, H, **kw)
+    left, right, d0 = _images(W, W, H)
+    out = torch.empty(W * H, dtype=torch.float64, device="cuda")
+    st = torch.empty(W * H, dtype=torch.uint8, device="cuda")
+    return (lambda s: r.run(left, right, d0, out, st, stream=s)), [out, st]
+
+
+@pytest.mark.parametrize("sizes,R,n", [
+    (((1300, 4), (2000, 4)) * 2, 10, 3000),     # SGM rings of 7 and 8 warps
+    (((720, 576), (1397, 1101)), 10, 200),
+    (((450, 375), (640, 480)), 12, 200),
+    (((600, 4), (2000, 4)) * 2, 40, 2000),
+])
+def test_refiners_of_two_sizes(svb, sizes, R, n):
+    _together([_refine_job(svb, W, H, R=R) for W, H in sizes], n)
