@@ -665,13 +665,14 @@ int launch_sgm_add_path(const uint8_t *C, const int32_t *base, int W, int H, int
     return sgm_dispatch<uint16_t, true>(C, C, base, base, W, H, K, P1, P2, S, 1, t, st);
 }
 
+// Shared memory of a row kernel: a row of doubles, integers and bytes.
+static size_t row_smem(int W) { return (size_t)W * (8 + 4 + 1) + 16; }
+
 int launch_left_to_right(const double *dl, int W, int H, double *dr, int32_t *base_r,
                          cudaStream_t st, int32_t *base_l, int *flag) {
-    size_t smem = (size_t)W * (8 + 4 + 1) + 16;
-    if (smem > 48 * 1024)
-        SV_CUDA_TRY(cudaFuncSetAttribute(k_left_to_right,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
+    const size_t smem = row_smem(W);
+    const int rc = allow_smem(k_left_to_right, smem, row_smem(kMaxRowW));
+    if (rc) return rc;
     count_launch(); pdl(k_left_to_right, H, 256, smem, st)(dl, W, dr, base_r, base_l, flag);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -679,11 +680,9 @@ int launch_left_to_right(const double *dl, int W, int H, double *dr, int32_t *ba
 
 int launch_lr_check(const double *dl, const double *dr, const double *disp0, int W,
                     int H, double tol, double *out, uint8_t *status, cudaStream_t st) {
-    size_t smem = (size_t)W * (8 + 4 + 1) + 16;
-    if (smem > 48 * 1024)
-        SV_CUDA_TRY(cudaFuncSetAttribute(k_lr_check,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
+    const size_t smem = row_smem(W);
+    const int rc = allow_smem(k_lr_check, smem, row_smem(kMaxRowW));
+    if (rc) return rc;
     count_launch(); pdl(k_lr_check, H, 256, smem, st)(dl, dr, disp0, W, tol, out, status);
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -766,13 +765,11 @@ int launch_batch_front(const BatchTables &t, long long px_blocks, long long rows
                        long long tiles, cudaStream_t st) {
     count_launch();
     pdl(k_b_base, (unsigned)px_blocks, 256, 0, st)(t);
-    const size_t row_smem = (size_t)t.maxW * (8 + 4 + 1) + 16;
-    if (row_smem > 48 * 1024)
-        SV_CUDA_TRY(cudaFuncSetAttribute(k_b_left_to_right,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)row_smem));
+    const size_t smem = row_smem(t.maxW);
+    const int rc = allow_smem(k_b_left_to_right, smem, row_smem(kMaxRowW));
+    if (rc) return rc;
     count_launch();
-    pdl(k_b_left_to_right, (unsigned)rows, 256, row_smem, st)(t);
+    pdl(k_b_left_to_right, (unsigned)rows, 256, smem, st)(t);
     const size_t cells = (size_t)(CT_W + 2 * t.rx) * (CT_H + 2 * t.ry);
     const dim3 g((unsigned)tiles, 1, 2), blk(CT_W, CT_H);
     count_launch();
@@ -790,12 +787,11 @@ int launch_batch_front(const BatchTables &t, long long px_blocks, long long rows
 }
 
 int launch_batch_back(const BatchTables &t, long long rows, cudaStream_t st) {
-    const size_t row_smem = (size_t)t.maxW * (8 + 4 + 1) + 16;
-    if (row_smem > 48 * 1024)
-        SV_CUDA_TRY(cudaFuncSetAttribute(k_b_lr_check, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)row_smem));
+    const size_t smem = row_smem(t.maxW);
+    const int rc = allow_smem(k_b_lr_check, smem, row_smem(kMaxRowW));
+    if (rc) return rc;
     count_launch();
-    pdl(k_b_lr_check, (unsigned)rows, 256, row_smem, st)(t);
+    pdl(k_b_lr_check, (unsigned)rows, 256, smem, st)(t);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }

@@ -72,6 +72,18 @@ def _refine_job(svb, W, H, **kw):
     (((720, 576), (1397, 1101)), 10, 200),
     (((450, 375), (640, 480)), 12, 200),
     (((600, 4), (2000, 4)) * 2, 40, 2000),
+    (((4000, 2), (8000, 2)) * 2, 10, 2000),     # row kernels: a row in shared memory
 ])
 def test_refiners_of_two_sizes(svb, sizes, R, n):
     _together([_refine_job(svb, W, H, R=R) for W, H in sizes], n)
+
+
+def test_batches_of_two_widths(svb):
+    jobs = []
+    for W in (4000, 8000) * 2:
+        b = svb.batch.BatchRefiner([(W, 2)] * 2)
+        for i in range(2):
+            for dst, src in zip((b.left[i], b.right[i], b.disp0[i]), _images(W + i, W, 2)):
+                dst.copy_(src)
+        jobs.append((lambda s, b=b: b.run(stream=s), b.out + b.status))
+    _together(jobs, 1000)
