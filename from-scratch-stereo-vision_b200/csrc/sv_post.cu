@@ -767,9 +767,7 @@ int launch_plane_snap(const double *disp, const double *rgb, int W, int H, const
     const long wmax = (long)(2 * step + 1) * (2 * step + 1);
     const int cap = wmax < kSnapCap ? (int)wmax : kSnapCap;
     const size_t smem = (size_t)cap * 3 * sizeof(double);
-    if (smem > 40 * 1024)
-        SV_CUDA_TRY(cudaFuncSetAttribute(k_seg_snap, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
+    SV_TRY_POST(allow_smem(k_seg_snap, smem, (size_t)kSnapCap * 3 * sizeof(double)));
     count_launch();
     pdl(k_seg_snap, nc, kSnapThreads, smem, st)(disp, W, valid, w.lab, w.win, w.start, w.nvalid,
                                                w.state, w.draw, trials, thr, min_inl, cap, w.pts,

@@ -6,6 +6,7 @@ without an error, with the bits of the same call made alone.  The sizes are the 
 whose kernels ask for different amounts above the default 48 KB; most are small
 images, so that the host's part of a call (where the threads meet) is most of it."""
 
+import ctypes
 import threading
 from importlib import import_module
 
@@ -86,4 +87,24 @@ def test_batches_of_two_widths(svb):
             for dst, src in zip((b.left[i], b.right[i], b.disp0[i]), _images(W + i, W, 2)):
                 dst.copy_(src)
         jobs.append((lambda s, b=b: b.run(stream=s), b.out + b.status))
+    _together(jobs, 1000)
+
+
+def test_plane_snaps_of_two_steps(svb):
+    lib = svb._lib.load()
+    jobs = []
+    for step in (21, 24) * 2:
+        W, H = 96, 64
+        g = torch.Generator(device="cuda").manual_seed(step)
+        rgb = torch.rand(3 * W * H, dtype=torch.float64, device="cuda", generator=g)
+        d = 5.0 + torch.rand(W * H, dtype=torch.float64, device="cuda", generator=g)
+        out = torch.empty_like(d)
+        need = lib.sv_postproc_workspace_size(W, H, step)
+        ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+
+        def call(s, d=d, rgb=rgb, out=out, ws=ws, need=need, step=step):
+            p = lambda t: ctypes.c_void_p(t.data_ptr())
+            svb._lib.check(lib.sv_plane_snap(p(d), p(rgb), 96, 64, None, step, 1.0, 0.3, 40,
+                                             ctypes.c_uint32(7), p(out), p(ws), need, s), "snap")
+        jobs.append((call, [out]))
     _together(jobs, 1000)
