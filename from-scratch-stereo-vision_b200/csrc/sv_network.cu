@@ -571,16 +571,16 @@ static size_t conv2d_wide_bytes(int IC, int S, int dil) {
 }
 
 template <int IC, int OC, int ACT, int CS, int PX, int S>
-static void b_conv2d_wide(const NetLaunch &L, unsigned ctas, int lv, int Z, const float *x0,
-                          const float *x1, int dil, const float *w, const float *b, float *y0,
-                          float *y1, const float *resid, cudaStream_t st) {
+static int b_conv2d_wide(const NetLaunch &L, unsigned ctas, int lv, int Z, const float *x0,
+                         const float *x1, int dil, const float *w, const float *b, float *y0,
+                         float *y1, const float *resid, cudaStream_t st) {
     const size_t smem = conv2d_wide_bytes(IC, S, dil);
-    constexpr size_t kStatic = (size_t)(IC * 9 + 1) * ((OC + 3) / 4 * 4) * sizeof(float);
-    if (smem + kStatic > 48 * 1024)
-        cudaFuncSetAttribute(k_b_conv2d_wide<IC, OC, ACT, CS, PX, S>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int rc = allow_smem(k_b_conv2d_wide<IC, OC, ACT, CS, PX, S>, smem,
+                              conv2d_wide_bytes(IC, S, 1));      // the feature net: dilation 1
+    if (rc) return rc;
     pdl(k_b_conv2d_wide<IC, OC, ACT, CS, PX, S>, ctas, CTB_TW / PX * CTB_TH, smem, st)(
         L, lv, Z, x0, x1, dil, w, b, y0, y1, resid);
+    return SV_OK;
 }
 
 // The Refinement levels' 3x3 convolutions, stride 1, padding = dilation: a CTA
@@ -787,38 +787,38 @@ static size_t conv2d_rows_bytes(int IC, int dil) {
 
 // One such convolution of a whole image (L NULL) or of a batch's pairs.
 template <int IC, int OC, int ACT, int CS, int DIL>
-static void conv2d_rows_go(const NetLaunch *L, unsigned ctas, int lv, int H, int W, const float *x,
-                           int dil, const float *w, const float *b, float *y, const float *resid,
-                           cudaStream_t st) {
+static int conv2d_rows_go(const NetLaunch *L, unsigned ctas, int lv, int H, int W, const float *x,
+                          int dil, const float *w, const float *b, float *y, const float *resid,
+                          cudaStream_t st) {
     const size_t smem = conv2d_rows_bytes<DIL>(IC, dil);
-    const size_t fixed = (size_t)(IC * 9 + 1) * ((OC + 3) / 4 * 4) * sizeof(float);
+    const size_t most = conv2d_rows_bytes<DIL>(IC, DIL > 0 ? DIL : 8);
+    int rc;
     if (L) {
-        if (smem + fixed > 48 * 1024)
-            cudaFuncSetAttribute(k_b_conv2d_rows<IC, OC, ACT, CS, DIL>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if ((rc = allow_smem(k_b_conv2d_rows<IC, OC, ACT, CS, DIL>, smem, most))) return rc;
         pdl(k_b_conv2d_rows<IC, OC, ACT, CS, DIL>, ctas, 8 * CTR_TH, smem, st)(*L, lv, x, dil, w, b,
                                                                               y, resid);
     } else {
-        if (smem + fixed > 48 * 1024)
-            cudaFuncSetAttribute(k_conv2d_rows<IC, OC, ACT, CS, DIL>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if ((rc = allow_smem(k_conv2d_rows<IC, OC, ACT, CS, DIL>, smem, most))) return rc;
         const dim3 g((W + CTR_TW - 1) / CTR_TW, (H + CTR_TH - 1) / CTR_TH);
         pdl(k_conv2d_rows<IC, OC, ACT, CS, DIL>, g, 8 * CTR_TH, smem, st)(x, H, W, dil, w, b, y,
                                                                          resid);
     }
+    return SV_OK;
 }
 
 // dilations 1, 2 and 4 (the shipped nets') compiled in
 template <int IC, int OC, int ACT, int CS>
-static void conv2d_rows(const NetLaunch *L, unsigned ctas, int lv, int H, int W, const float *x,
-                        int dil, const float *w, const float *b, float *y, const float *resid,
-                        cudaStream_t st) {
-    if (dil == 1) conv2d_rows_go<IC, OC, ACT, CS, 1>(L, ctas, lv, H, W, x, dil, w, b, y, resid, st);
-    else if (dil == 2) conv2d_rows_go<IC, OC, ACT, CS, 2>(L, ctas, lv, H, W, x, dil, w, b, y, resid, st);
-    else if (dil == 4) conv2d_rows_go<IC, OC, ACT, CS, 4>(L, ctas, lv, H, W, x, dil, w, b, y, resid, st);
-    else if (dil >= 0 && dil <= 8)
-        conv2d_rows_go<IC, OC, ACT, CS, 0>(L, ctas, lv, H, W, x, dil, w, b, y, resid, st);
-    else conv2d_rows_go<IC, OC, ACT, CS, -1>(L, ctas, lv, H, W, x, dil, w, b, y, resid, st);
+static int conv2d_rows(const NetLaunch *L, unsigned ctas, int lv, int H, int W, const float *x,
+                       int dil, const float *w, const float *b, float *y, const float *resid,
+                       cudaStream_t st) {
+#define SV_ROWS(DIL) \
+    return conv2d_rows_go<IC, OC, ACT, CS, DIL>(L, ctas, lv, H, W, x, dil, w, b, y, resid, st)
+    if (dil == 1) SV_ROWS(1);
+    if (dil == 2) SV_ROWS(2);
+    if (dil == 4) SV_ROWS(4);
+    if (dil >= 0 && dil <= 8) SV_ROWS(0);
+    SV_ROWS(-1);
+#undef SV_ROWS
 }
 
 // A Refinement level's first convolution (2 -> RC, stride 1, dilation dil,
@@ -1706,10 +1706,12 @@ static int forward_impl(const NetView &n, const float *left, const float *right,
                 pdl(k_conv2d_up<RC, RG>, tgrid(Wl, Hl, RC / RG), tb, conv2d_tile_bytes(2, 1, dl),
                                       st)(prev, ph, pw, guides[lv], Hl, Wl, dl, n.rw[lv][i],
                                             n.rb[lv][i], dst, b.rin);
-            else if (rows && dl >= 0 && dl <= 8)
-                conv2d_rows<RC, RC, 1, RS>(nullptr, 0, 0, Hl, Wl, cur, dl, n.rw[lv][i], n.rb[lv][i],
-                                           dst, nullptr, st);
-            else            // every output channel per thread (measured faster)
+            else if (rows && dl >= 0 && dl <= 8) {
+                const int rc = conv2d_rows<RC, RC, 1, RS>(nullptr, 0, 0, Hl, Wl, cur, dl,
+                                                          n.rw[lv][i], n.rb[lv][i], dst, nullptr,
+                                                          st);
+                if (rc) return rc;
+            } else            // every output channel per thread (measured faster)
                 pdl(k_conv2d_tiled<RC, RC, RC, 1, RS>, tgrid(Wl, Hl, 1), RS * tb1,
                                                     conv2d_tile_bytes(RC, 1, dl, RS), st)(
                     cur, cur, Hl, Wl, Hl, Wl, 1, dl, dl, n.rw[lv][i], n.rb[lv][i], dst, dst,
@@ -1723,10 +1725,12 @@ static int forward_impl(const NetView &n, const float *left, const float *right,
                                             outs[lv], b.rin, *b.decide->width,
                                             b.decide->state, b.decide->hist,
                                             b.decide->mirror);
-        else if (rows)
-            conv2d_rows<RC, 1, 2, 4>(nullptr, 0, 0, Hl, Wl, cur, 1, n.rw[lv][n.ndil],
-                                     n.rb[lv][n.ndil], outs[lv], b.rin, st);
-        else
+        else if (rows) {
+            const int rc = conv2d_rows<RC, 1, 2, 4>(nullptr, 0, 0, Hl, Wl, cur, 1,
+                                                    n.rw[lv][n.ndil], n.rb[lv][n.ndil], outs[lv],
+                                                    b.rin, st);
+            if (rc) return rc;
+        } else
             pdl(k_conv2d_tiled<RC, 1, 1, 2, 4>, tgrid(Wl, Hl, 1), tb4,
                                              conv2d_tile_bytes(RC, 1, 1, 4), st)(
                 cur, cur, Hl, Wl, Hl, Wl, 1, 1, 1, n.rw[lv][n.ndil], n.rb[lv][n.ndil], outs[lv],
@@ -1835,20 +1839,25 @@ static int b_forward_impl(const NetView &n, const NetStageLaunch &g, const NetSl
     auto L = [&](int k) { return NetLaunch{g.pre[k], g.pairs, g.n, g.slab}; };
     auto B = [&](int k) { return ctas_of(g.total[k]); };
     const dim3 tb(CT2_TW, CT2_TH);
+    int rc;
     // FeatureNet, both images: every output channel and 2 pixels per thread
     // (the arithmetic of k_conv2d_tiled<.., FG, .., 1 or 2>)
     count_launch();
-    b_conv2d_wide<1, C, 1, 1, 2, 2>(L(NK_C1W), B(NK_C1W), 0, 2, s.lw, s.rw, 1, n.fw[0], n.fb[0],
-                                    s.f.fa[0], s.f.fa[1], nullptr, st);
+    if ((rc = b_conv2d_wide<1, C, 1, 1, 2, 2>(L(NK_C1W), B(NK_C1W), 0, 2, s.lw, s.rw, 1, n.fw[0], n.fb[0],
+                                              s.f.fa[0], s.f.fa[1], nullptr, st)))
+        return rc;
     count_launch();
-    b_conv2d_wide<C, C, 1, 2, 2, 2>(L(NK_C2W), B(NK_C2W), 1, 2, s.f.fa[0], s.f.fa[1], 1,
-                                    n.fw[1], n.fb[1], s.f.fb[0], s.f.fb[1], nullptr, st);
+    if ((rc = b_conv2d_wide<C, C, 1, 2, 2, 2>(L(NK_C2W), B(NK_C2W), 1, 2, s.f.fa[0], s.f.fa[1], 1,
+                                              n.fw[1], n.fb[1], s.f.fb[0], s.f.fb[1], nullptr, st)))
+        return rc;
     count_launch();
-    b_conv2d_wide<C, C, 1, 2, 2, 1>(L(NK_C2W), B(NK_C2W), 2, 2, s.f.fb[0], s.f.fb[1], 1,
-                                    n.fw[2], n.fb[2], s.f.fa[0], s.f.fa[1], nullptr, st);
+    if ((rc = b_conv2d_wide<C, C, 1, 2, 2, 1>(L(NK_C2W), B(NK_C2W), 2, 2, s.f.fb[0], s.f.fb[1], 1,
+                                              n.fw[2], n.fb[2], s.f.fa[0], s.f.fa[1], nullptr, st)))
+        return rc;
     count_launch();
-    b_conv2d_wide<C, C, 0, 2, 2, 1>(L(NK_C2W), B(NK_C2W), 2, 2, s.f.fa[0], s.f.fa[1], 1,
-                                    n.fw[3], n.fb[3], s.f.fb[0], s.f.fb[1], nullptr, st);
+    if ((rc = b_conv2d_wide<C, C, 0, 2, 2, 1>(L(NK_C2W), B(NK_C2W), 2, 2, s.f.fa[0], s.f.fa[1], 1,
+                                              n.fw[3], n.fb[3], s.f.fb[0], s.f.fb[1], nullptr, st)))
+        return rc;
     SV_LAUNCH_CHECK();
     constexpr int S1 = C % 4 == 0 ? 4 : 2, S2 = CM % 4 == 0 && CM > 4 ? 4 : 2;
     count_launch();
@@ -1881,15 +1890,17 @@ static int b_forward_impl(const NetView &n, const NetStageLaunch &g, const NetSl
                     L(kk), lv, prevs[lv], guides[lv], dl, n.rw[lv][i], n.rb[lv][i], dst, s.f.rin);
             else {
                 const NetLaunch l = L(kf);
-                conv2d_rows<RC, RC, 1, RS>(&l, B(kf), lv + 3, 0, 0, cur, dl, n.rw[lv][i],
-                                           n.rb[lv][i], dst, nullptr, st);
+                if ((rc = conv2d_rows<RC, RC, 1, RS>(&l, B(kf), lv + 3, 0, 0, cur, dl, n.rw[lv][i],
+                                                     n.rb[lv][i], dst, nullptr, st)))
+                    return rc;
             }
             cur = dst;
         }
         count_launch();
         const NetLaunch l = L(kf);
-        conv2d_rows<RC, 1, 2, 4>(&l, B(kf), lv + 3, 0, 0, cur, 1, n.rw[lv][n.ndil],
-                                 n.rb[lv][n.ndil], outs[lv], s.f.rin, st);
+        if ((rc = conv2d_rows<RC, 1, 2, 4>(&l, B(kf), lv + 3, 0, 0, cur, 1, n.rw[lv][n.ndil],
+                                           n.rb[lv][n.ndil], outs[lv], s.f.rin, st)))
+            return rc;
         SV_LAUNCH_CHECK();
     }
     return SV_OK;

@@ -13,6 +13,8 @@ from importlib import import_module
 import pytest
 import torch
 
+from test_refinement_sizes_gpu import _net as _forward_net
+
 pytestmark = pytest.mark.gpu
 
 
@@ -107,4 +109,27 @@ def test_plane_snaps_of_two_steps(svb):
             svb._lib.check(lib.sv_plane_snap(p(d), p(rgb), 96, 64, None, step, 1.0, 0.3, 40,
                                              ctypes.c_uint32(7), p(out), p(ws), need, s), "snap")
         jobs.append((call, [out]))
+    _together(jobs, 1000)
+
+
+def test_forwards_of_two_dilations(svb):
+    network = import_module(svb.__name__ + ".network")
+    lib = svb._lib.load()
+    jobs = []
+    for dil in ((1, 7), (1, 8)) * 2:
+        g = network.gpu_net(_forward_net(svb, dil, dil[1]))
+        H = W = 200
+        gen = torch.Generator(device="cuda").manual_seed(dil[1])
+        new = lambda n: torch.rand(n, device="cuda", generator=gen)
+        ins = [new(H * W), new(H * W), new(H * W // 4), new(H * W)]
+        outs = [torch.empty(n, device="cuda") for n in (H * W // 16, H * W // 4, H * W)]
+        need = lib.sv_forward_workspace_size(g.handle, H, W)
+        ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+
+        def call(s, g=g, ins=ins, outs=outs, ws=ws, need=need):
+            p = lambda t: ctypes.c_void_p(t.data_ptr())
+            svb._lib.check(lib.sv_stereonet_forward(
+                g.handle, p(ins[0]), p(ins[1]), 200, 200, p(ins[2]), p(ins[3]), p(outs[0]),
+                p(outs[1]), p(outs[2]), svb._lib.SV_FP32, p(ws), need, s), "forward")
+        jobs.append((call, outs))
     _together(jobs, 1000)
