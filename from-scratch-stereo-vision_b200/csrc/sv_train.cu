@@ -1270,23 +1270,25 @@ void carve(const sv_trainer *t, const Dims &d, Carver &cv, TrainBufs &b) {
     b.loss = cv.take<double>(B);
 }
 
-// Raised limit of a kernel that stages more than the default 48 KB.
+constexpr int kMaxDil = 8, kMaxD = 16;     // of a trainable architecture
+
+// Raised limit of a kernel that stages more than the default 48 KB; most: the largest
+// that any architecture asks of it.
 template <typename F>
-int big_smem(F *f, size_t sm, const char *what) {
+int big_smem(F *f, size_t sm, size_t most, const char *what) {
     if (sm > 200 * 1024) {
         set_error("%s needs %zu bytes of shared memory", what, sm);
         return SV_ERR_SHAPE;
     }
-    if (sm > 40 * 1024)
-        SV_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    return SV_OK;
+    return allow_smem(f, sm, most);
 }
 
 template <int IC, int OC, int WC, int S, int DIL, int MODE, bool FLIP, int TR>
 int conv2d_go(const float *x, int nimg, int H, int W, int OH, int OW, int dil, const float *w,
               const float *b, float *y, const float *aux, long stride, cudaStream_t st) {
     const size_t sm = tconv2d_smem(IC, S, dil, TR);
-    const int rc = big_smem(k_tconv2d<IC, OC, WC, S, DIL, MODE, FLIP, TR>, sm, "convolution tile");
+    const int rc = big_smem(k_tconv2d<IC, OC, WC, S, DIL, MODE, FLIP, TR>, sm,
+                            tconv2d_smem(IC, S, DIL > 0 ? DIL : kMaxDil, TR), "convolution tile");
     if (rc) return rc;
     const dim3 g((OW + 31) / 32, (OH + TR - 1) / TR, nimg);
     count_launch();
@@ -1316,8 +1318,10 @@ int conv3d_go(const float *x, int B, int D, int h, int w, const float *wt, const
               const float *xin, cudaStream_t st) {
     if (nxg == 8 && w <= 24)                               // groups of 4 columns
         return conv3d_go<IC, OC, WC, CCH, MODE, FLIP, 6>(x, B, D, h, w, wt, b, y, xin, st);
-    const size_t sm = sizeof(float) * CCH * (D + 2) * 3 * (4 * nxg + 4);
-    const int rc = big_smem(k_tconv3d<IC, OC, WC, CCH, MODE, FLIP, nxg>, sm, "3-D convolution tile");
+    auto tile = [](int d) { return sizeof(float) * CCH * (d + 2) * 3 * (4 * nxg + 4); };
+    const size_t sm = tile(D);
+    const int rc = big_smem(k_tconv3d<IC, OC, WC, CCH, MODE, FLIP, nxg>, sm, tile(kMaxD),
+                            "3-D convolution tile");
     if (rc) return rc;
     const dim3 g((w + 4 * nxg - 1) / (4 * nxg), h, B);
     count_launch();
@@ -1351,7 +1355,9 @@ template <int IC, int OC, int S, int DIL>
 int wgrad2d_go(const float *x, const float *gy, int nimg, int H, int W, int OH, int OW, int dil,
                WGrads &g, long gw, long gb, cudaStream_t st) {
     const size_t sm = twgrad2d_smem<IC, OC, S, DIL>(dil);
-    const int rc = big_smem(k_twgrad2d<IC, OC, S, DIL>, sm, "weight-gradient tile");
+    const int rc = big_smem(k_twgrad2d<IC, OC, S, DIL>, sm,
+                            twgrad2d_smem<IC, OC, S, DIL>(DIL > 0 ? DIL : kMaxDil),
+                            "weight-gradient tile");
     if (rc) return rc;
     const long ntiles = tiles2d(nimg, OH, OW);
     const int nblk = (int)(ntiles < kWgCtas ? ntiles : kWgCtas);
@@ -1382,7 +1388,7 @@ template <int IC, int OC>
 int wgrad3d(const float *x, const float *gy, int B, int D, int h, int w, WGrads &g, long gw, long gb,
             cudaStream_t st) {
     using Gm = Wg3<IC, OC>;
-    const int rc = big_smem(k_twgrad3d<IC, OC>, Gm::SMEM, "weight-gradient tile");
+    const int rc = big_smem(k_twgrad3d<IC, OC>, Gm::SMEM, Gm::SMEM, "weight-gradient tile");
     if (rc) return rc;
     const long ntiles = (long)B * h * ((D + 3) / 4) * ((w + 31) / 32);
     const int nblk = (int)(ntiles < kWgCtas ? ntiles : kWgCtas);
@@ -1616,8 +1622,8 @@ int check_dims(const sv_trainer *t, int B, int W, int H) {
         return SV_ERR_SHAPE;
     }
     for (int i = 0; i < t->nd; ++i)
-        if (t->dil[i] < 1 || t->dil[i] > 8) {
-            set_error("dilation %d outside 1..8", t->dil[i]);
+        if (t->dil[i] < 1 || t->dil[i] > kMaxDil) {
+            set_error("dilation %d outside 1..%d", t->dil[i], kMaxDil);
             return SV_ERR_NET;
         }
     return SV_OK;
@@ -1636,7 +1642,7 @@ int sv_trainer_create(const int *arch, int n_arch, const double *params, long n_
     }
     const bool ok_arch = (arch[0] == 12 && arch[1] == 6 && arch[3] == 8) ||
                          (arch[0] == 8 && arch[1] == 4 && arch[3] == 8);
-    if (!ok_arch || arch[2] < 2 || arch[2] > 16) {
+    if (!ok_arch || arch[2] < 2 || arch[2] > kMaxD) {
         set_error("trainable architectures: feat_C/cost_C/refine_C 12/6/8 or 8/4/8, D 2..16");
         return SV_ERR_NET;
     }

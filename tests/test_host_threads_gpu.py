@@ -13,6 +13,7 @@ from importlib import import_module
 import pytest
 import torch
 
+from test_train_sizes_gpu import _net as _train_net
 from test_refinement_sizes_gpu import _net as _forward_net
 
 pytestmark = pytest.mark.gpu
@@ -133,3 +134,26 @@ def test_forwards_of_two_dilations(svb):
                 p(outs[1]), p(outs[2]), svb._lib.SV_FP32, p(ws), need, s), "forward")
         jobs.append((call, outs))
     _together(jobs, 1000)
+
+
+def test_trainers_of_two_dilations(svb):
+    train = import_module(svb.__name__ + ".train")
+    lib = svb._lib.load()
+    jobs = []
+    for dil in ((6, 1), (8, 1)) * 2:
+        t = train.Trainer(_train_net(svb, 8, 4, 4, dil, dil[0]))
+        B, W, H = 1, 32, 32
+        g = torch.Generator(device="cuda").manual_seed(dil[0])
+        left, right, disp = (torch.rand(B * W * H, device="cuda", generator=g) for _ in range(3))
+        valid = torch.ones(B * W * H, dtype=torch.uint8, device="cuda")
+        loss = torch.empty(B, dtype=torch.float64, device="cuda")
+        pred = torch.empty(B * W * H, device="cuda")
+        need = lib.sv_train_workspace_size(t.handle, B, W, H)
+        ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+
+        def call(s, t=t, a=(left, right, disp, valid), loss=loss, pred=pred, ws=ws, need=need):
+            p = lambda x: ctypes.c_void_p(x.data_ptr())
+            svb._lib.check(lib.sv_train_grads(t.handle, p(a[0]), p(a[1]), p(a[2]), p(a[3]), 1, 32,
+                                              32, p(loss), p(pred), p(ws), need, s), "grads")
+        jobs.append((call, [loss, pred]))
+    _together(jobs, 300)
