@@ -826,7 +826,7 @@ __global__ void __launch_bounds__(256)
 // such a row is no 16-byte copy, and 64 slots are faster although they are more (500 x
 // 150, K = 31: 271 us a pass, 328 with 48).
 int slot_width(int K, bool pad) {
-    static const int widths[] = {8, 16, 24, 32, 48, 64, 96, 128, 160, 192, 224, 256};
+    static const int widths[] = {8, 16, 24, 32, 48, 64, 96, 128, 160, 192, 256};
     for (int w : widths)
         if (w >= K + 2 && (w != 48 || !pad)) return w;
     return 256;
@@ -883,7 +883,12 @@ static int sgm_dispatch(const uint8_t *C0, const uint8_t *C1, const int32_t *b0,
     // More lanes shorten a step, whose latency a warp alone on its scheduler pays; the
     // fewest registers per lane that leave 16-byte copies (640 x 480, a pass: K = 49 2
     // lanes 460 us, 4 414; K = 101 4 lanes 660, 8 634; K = 25 2 lanes 311, 4 and 8-byte
-    // copies 326).
+    // copies 326).  From 160 slots on at most 12 registers whatever the copies: steps of
+    // 20 and more cost more than in proportion.  The SGM launch, 8- / 16-bit path costs:
+    // 640 x 480, K = 155: 4 lanes of 20 375 / 903 us, 8 of 10 364 / 547; K = 159: 4 of 24
+    // 963 / 1600, 8 of 12 344 / 672; K = 253: 4 of 32 1567 / 2695, 8 of 16 561 / 1509, 16
+    // of 8 520 / 774; 160 x 120, K = 253: 229 / 301, 59 / 100 and 43 / 59.  K = 191 to 222
+    // take 256 slots too (640 x 480: 224 slots in 8 lanes of 14 551 / 991).
 #define SV_SGM(NR, GL) \
     return sgm_go<NR, GL, LT, PAD>(C0, C1, b0, b1, W, H, K, P1, P2, Lout, nviews, npaths, st)
     switch (Kp) {
@@ -895,10 +900,9 @@ static int sgm_dispatch(const uint8_t *C0, const uint8_t *C1, const int32_t *b0,
     case 64: SV_SGM(8, 4);
     case 96: SV_SGM(12, 4);
     case 128: SV_SGM(8, 8);
-    case 160: SV_SGM(20, 4);
-    case 192: SV_SGM(24, 4);
-    case 224: SV_SGM(28, 4);
-    case 256: SV_SGM(32, 4);
+    case 160: SV_SGM(10, 8);
+    case 192: SV_SGM(12, 8);
+    case 256: SV_SGM(8, 16);
     default: break;
     }
 #undef SV_SGM

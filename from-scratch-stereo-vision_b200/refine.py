@@ -40,7 +40,7 @@ def sgm_kernel_name(K: int = 21) -> str:
     """Name of the SGM kernel the library runs for a band of K, with its split
     of a scanline: registers of two 16-bit slots per lane x lanes."""
     split = {8: (4, 1), 16: (4, 2), 24: (6, 2), 32: (8, 2), 64: (8, 4), 96: (12, 4),
-             128: (8, 8), 160: (20, 4), 192: (24, 4), 224: (28, 4), 256: (32, 4)}
+             128: (8, 8), 160: (10, 8), 192: (12, 8), 256: (8, 16)}
     Kp = next((k for k in sorted(split) if k >= K + 2), 256)
     return "k_sgm_scan<%d registers x %d lanes>" % split[Kp]
 
