@@ -717,23 +717,23 @@ __device__ __forceinline__ void wta_pixel(const uint8_t *__restrict__ Lp, long s
     *outp = wta_value(bk, bv, va, vb, base_p, R);
 }
 
-// One pixel by 8 neighbouring lanes (any band, any path-cost width): lane l
-// takes the 8-slot chunks l, l + 8, ... of every path's row, so a warp reads
+// One pixel by LPP neighbouring lanes (any band, any path-cost width): lane l
+// takes the 8-slot chunks l, l + LPP, ... of every path's row, so a warp reads
 // whole rows (one thread per pixel read 8 bytes every Kp: 1,940 us at 640x480
-// with K = 155, against 0.94 GB of path costs).  All 8 lanes call it.
-template <typename LT>
+// with K = 155, against 0.94 GB of path costs).  All LPP lanes call it.
+template <typename LT, int LPP>
 __device__ __forceinline__ void wta_pixel_wide(const LT *__restrict__ Lp, long stride, int npaths,
                                                int K, int Kp, int R, int32_t base_p,
                                                const double *__restrict__ d0p, double uniq,
                                                bool want_conf, double *__restrict__ outp,
                                                double *__restrict__ confp) {
-    const int lane = threadIdx.x & 31, l = lane & 7;
-    const unsigned mask = 0xFFu << (lane & 24);
+    const int lane = threadIdx.x & 31, l = lane & (LPP - 1);
+    const unsigned mask = ((1u << LPP) - 1u) << (lane & ~(LPP - 1));
     const int am = first_slot(base_p - R, Kp);
     // smallest S * 256 + k over the band indices outside [x0, x1]
     auto scan = [&](int x0, int x1) {
         unsigned best = 0xFFFFFFFFu;
-        for (int c = 8 * l; c < Kp; c += 64) {
+        for (int c = 8 * l; c < Kp; c += 8 * LPP) {
             unsigned acc[4] = {0u, 0u, 0u, 0u};
             if (npaths == 8) {
 #pragma unroll
@@ -752,30 +752,34 @@ __device__ __forceinline__ void wta_pixel_wide(const LT *__restrict__ Lp, long s
             }
         }
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) best = min(best, __shfl_xor_sync(mask, best, o));
+        for (int o = 1; o < LPP; o <<= 1) best = min(best, __shfl_xor_sync(mask, best, o));
         return best;
     };
     const unsigned key = scan(1, 0);
     const int bk = (int)(key & 255u), bv = (int)(key >> 8);
-    if (bk == 0 || bk == K - 1) {                          // the same for the 8 lanes
+    if (bk == 0 || bk == K - 1) {                          // the same for the LPP lanes
         if (l == 0) {
             *outp = *d0p;
             if (want_conf) *confp = 0.0;
         }
         return;
     }
-    // the sums beside the winner, one path per lane (both fit 16 bits)
+    // the sums beside the winner, the paths dealt to the lanes (both fit 16 bits)
     unsigned ab = 0u;
-    if (l < npaths) {
+    {
         int ja = am + bk - 1, jb = am + bk + 1;
         ja -= ja >= Kp ? Kp : 0;
         jb -= jb >= Kp ? Kp : 0;
-        const LT *row = Lp + l * stride;
-        ab = (unsigned)row[elem_of_slot(ja, Kp, false)] |
-             (unsigned)row[elem_of_slot(jb, Kp, false)] << 16;
+        const int ea = elem_of_slot(ja, Kp, false), eb = elem_of_slot(jb, Kp, false);
+#pragma unroll
+        for (int d = 0; d < 8; d += LPP)
+            if (d + l < npaths) {
+                const LT *row = Lp + (d + l) * stride;
+                ab += (unsigned)row[ea] | (unsigned)row[eb] << 16;
+            }
     }
 #pragma unroll
-    for (int o = 1; o < 8; o <<= 1) ab += __shfl_xor_sync(mask, ab, o);
+    for (int o = 1; o < LPP; o <<= 1) ab += __shfl_xor_sync(mask, ab, o);
     bool use_d0 = false;
     double conf = 0.0;
     if (uniq > 0.0 || want_conf) {
@@ -788,8 +792,8 @@ __device__ __forceinline__ void wta_pixel_wide(const LT *__restrict__ Lp, long s
     *outp = use_d0 ? *d0p : wta_value(bk, bv, (int)(ab & 0xFFFFu), (int)(ab >> 16), base_p, R);
 }
 
-// nviews <= 2; KP > 0: one thread per pixel with Kp fixed, else 8 lanes.
-template <typename LT, int KP, bool PAD, int NPC>
+// nviews <= 2; KP > 0: one thread per pixel with Kp fixed, else LPP lanes.
+template <typename LT, int KP, bool PAD, int NPC, int LPP>
 __global__ void __launch_bounds__(256)
     k_wta_slot(const LT *__restrict__ Lall, int npaths, int nviews, long N, int K, int Kp, int R,
                const int32_t *__restrict__ base0, const int32_t *__restrict__ base1,
@@ -797,7 +801,6 @@ __global__ void __launch_bounds__(256)
                int want_conf, double *__restrict__ out0, double *__restrict__ out1,
                double *__restrict__ conf0) {
     pdl_sync();
-    constexpr int LPP = KP > 0 ? 1 : 8;                    // lanes per pixel
     const int row = path_row(KP > 0 ? KP : Kp, PAD);
     const long stride = N * row;                           // between path arrays
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nviews * N * LPP;
@@ -813,8 +816,8 @@ __global__ void __launch_bounds__(256)
             wta_pixel<KP, PAD, NPC>(Lp, stride, npaths, K, R, b, d0, uniq, want_conf && view == 0,
                                     out, conf);
         else
-            wta_pixel_wide<LT>(Lp, stride, npaths, K, Kp, R, b, d0, uniq, want_conf && view == 0,
-                               out, conf);
+            wta_pixel_wide<LT, LPP>(Lp, stride, npaths, K, Kp, R, b, d0, uniq,
+                                    want_conf && view == 0, out, conf);
     }
 }
 
@@ -932,20 +935,26 @@ int launch_wta_slot(const void *L, bool l16, bool pad, int npaths, int nviews, i
         set_error("wta: nviews=%d", nviews);
         return SV_ERR_PARAM;
     }
-#define SV_WTA(LT, KP, PAD, NP, BLOCKS)                                                          \
-    pdl(k_wta_slot<LT, KP, PAD, NP>, BLOCKS, 256, 0, st)((const LT *)L, npaths, nviews, N, K, Kp, \
-                                                        R, b0, b1, d00, d01, uniq,               \
-                                                        conf0 != nullptr, out0, out1, conf0)
+#define SV_WTA(LT, KP, PAD, NP, LPP, BLOCKS)                                                \
+    pdl(k_wta_slot<LT, KP, PAD, NP, LPP>, BLOCKS, 256, 0, st)(                               \
+        (const LT *)L, npaths, nviews, N, K, Kp, R, b0, b1, d00, d01, uniq, conf0 != nullptr, \
+        out0, out1, conf0)
     const int blocks = grid_for(nviews * N, 256, 148 * 16);
     const int wide = grid_for(nviews * N * 8, 256, 148 * 64);
-    if (l16) SV_WTA(uint16_t, 0, false, 0, wide);
-    else if (Kp == 24 && pad && npaths == 8) SV_WTA(uint8_t, 24, true, 8, blocks);
-    else if (Kp == 24 && pad) SV_WTA(uint8_t, 24, true, 0, blocks);
-    else if (Kp == 24) SV_WTA(uint8_t, 24, false, 0, blocks);
-    else if (Kp == 8) SV_WTA(uint8_t, 8, false, 0, blocks);
-    else if (Kp == 16) SV_WTA(uint8_t, 16, false, 0, blocks);
-    else if (Kp == 32) SV_WTA(uint8_t, 32, false, 0, blocks);
-    else SV_WTA(uint8_t, 0, false, 0, wide);
+    // 16-bit path costs of a narrow band: as many lanes as leave each a chunk or two, or
+    // most of them idle (1397 x 1101, both views, lanes 1 / 2 / 4 / 8: K = 11 160 / 175 /
+    // 299 / 516 us, K = 21 234 / 231 / 312 / 527, K = 25 321 / 280 / 336 / 547; with 64
+    // slots or more 8 lanes are the fastest, K = 95 at 160 x 120 45 / 24 / 20 / 18).
+    if (l16 && Kp <= 16) SV_WTA(uint16_t, 0, false, 0, 1, blocks);
+    else if (l16 && Kp <= 32) SV_WTA(uint16_t, 0, false, 0, 2, grid_for(nviews * N * 2, 256, 148 * 64));
+    else if (l16) SV_WTA(uint16_t, 0, false, 0, 8, wide);
+    else if (Kp == 24 && pad && npaths == 8) SV_WTA(uint8_t, 24, true, 8, 1, blocks);
+    else if (Kp == 24 && pad) SV_WTA(uint8_t, 24, true, 0, 1, blocks);
+    else if (Kp == 24) SV_WTA(uint8_t, 24, false, 0, 1, blocks);
+    else if (Kp == 8) SV_WTA(uint8_t, 8, false, 0, 1, blocks);
+    else if (Kp == 16) SV_WTA(uint8_t, 16, false, 0, 1, blocks);
+    else if (Kp == 32) SV_WTA(uint8_t, 32, false, 0, 1, blocks);
+    else SV_WTA(uint8_t, 0, false, 0, 8, wide);
 #undef SV_WTA
     SV_LAUNCH_CHECK();
     return SV_OK;
@@ -1012,10 +1021,9 @@ __global__ void __launch_bounds__(256) k_b_sgm(BatchTables t, long long total) {
     }
 }
 
-template <typename LT, int KP, bool PAD, int NPC>
+template <typename LT, int KP, bool PAD, int NPC, int LPP>
 __global__ void __launch_bounds__(256) k_b_wta(BatchTables t) {
     pdl_sync();
-    constexpr int LPP = KP > 0 ? 1 : 8;
     const int i = batch_find(t.px_blk, t.n, blockIdx.x);
     const BatchPair &P = t.pairs[i];
     const int view = blockIdx.y;
@@ -1034,8 +1042,8 @@ __global__ void __launch_bounds__(256) k_b_wta(BatchTables t) {
             wta_pixel<KP, PAD, NPC>(Lv + p * row, stride, t.npaths, t.K, t.R, b, d0, t.uniq, false,
                                     out, nullptr);
         else
-            wta_pixel_wide<LT>(Lv + p * row, stride, t.npaths, t.K, t.Kp, t.R, b, d0, t.uniq,
-                               false, out, nullptr);
+            wta_pixel_wide<LT, LPP>(Lv + p * row, stride, t.npaths, t.K, t.Kp, t.R, b, d0,
+                                    t.uniq, false, out, nullptr);
     }
 }
 
@@ -1095,12 +1103,13 @@ int launch_batch_refine(const BatchTables &t, long long px_blocks, long long row
 #undef SV_BGO
     if (rc) return rc;
     count_launch();
-    if (l16) pdl(k_b_wta<uint16_t, 0, false, 0>, px, 256, 0, st)(t);
-    else if (t.Kp == 24 && t.npaths == 8) pdl(k_b_wta<uint8_t, 24, true, 8>, px, 256, 0, st)(t);
-    else if (t.Kp == 24) pdl(k_b_wta<uint8_t, 24, true, 0>, px, 256, 0, st)(t);
-    else if (t.Kp == 8) pdl(k_b_wta<uint8_t, 8, true, 0>, px, 256, 0, st)(t);
-    else if (t.Kp == 16) pdl(k_b_wta<uint8_t, 16, true, 0>, px, 256, 0, st)(t);
-    else pdl(k_b_wta<uint8_t, 32, true, 0>, px, 256, 0, st)(t);
+    if (l16 && t.Kp <= 16) pdl(k_b_wta<uint16_t, 0, false, 0, 1>, px, 256, 0, st)(t);
+    else if (l16) pdl(k_b_wta<uint16_t, 0, false, 0, 2>, px, 256, 0, st)(t);
+    else if (t.Kp == 24 && t.npaths == 8) pdl(k_b_wta<uint8_t, 24, true, 8, 1>, px, 256, 0, st)(t);
+    else if (t.Kp == 24) pdl(k_b_wta<uint8_t, 24, true, 0, 1>, px, 256, 0, st)(t);
+    else if (t.Kp == 8) pdl(k_b_wta<uint8_t, 8, true, 0, 1>, px, 256, 0, st)(t);
+    else if (t.Kp == 16) pdl(k_b_wta<uint8_t, 16, true, 0, 1>, px, 256, 0, st)(t);
+    else pdl(k_b_wta<uint8_t, 32, true, 0, 1>, px, 256, 0, st)(t);
     SV_LAUNCH_CHECK();
     return launch_batch_back(t, rows, st);
 }
