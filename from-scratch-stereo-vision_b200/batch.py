@@ -63,8 +63,11 @@ def default_config() -> BatchConfig:
 # candidate values per knob, tried one knob at a time
 TUNE_SPACE = {"px_per_block": (512, 1024, 2048, 4096),
               "sgm_threads": (64, 128, 256),
-              "sgm_ctas_per_sm": (4, 8, 16),
+              "sgm_ctas_per_sm": (1, 2, 4, 8),       # 8 warps per SM at most
               "sgm_fetch": (32, 64)}
+# raised when the kernels or a knob's meaning change: a cached choice holds for the
+# kernels it was timed with
+TUNE_VERSION = 2
 
 
 def _cache_path() -> str:
@@ -118,8 +121,9 @@ class BatchRefiner:
         props = torch.cuda.get_device_properties(torch.cuda.current_device())
         mpix = self.pixels / 1e6
         bucket = 1 << max(0, int(np.ceil(np.log2(max(mpix, 1e-6)))) + 20)   # pixels, next 2^k
-        return "%s|sm%d|R%d|paths%d|n%d|px%d" % (props.name, props.multi_processor_count,
-                                                 self.p.R, self.p.paths, len(self.sizes), bucket)
+        return "v%d|%s|sm%d|R%d|paths%d|n%d|px%d" % (TUNE_VERSION, props.name,
+                                                     props.multi_processor_count, self.p.R,
+                                                     self.p.paths, len(self.sizes), bucket)
 
     def time_config(self, cfg: BatchConfig, reps: int = 3) -> float:
         """Median device milliseconds of one batched call with `cfg`."""

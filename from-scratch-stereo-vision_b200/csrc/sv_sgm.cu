@@ -1058,14 +1058,15 @@ static int batch_sgm_go(const BatchTables &t, long long tasks, int threads, int 
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     long long want = (tasks * GL + threads - 1) / threads;
-    // persistent: a quarter of ctas_per_sm CTAs on each SM (the default 8: 8
-    // warps, 128 scanlines).  More of them read and write more rows at once
-    // than the caches hold: 20 uneven pairs took 1.8 ms with 8 warps per SM,
+    // persistent: ctas_per_sm CTAs on each SM, but no more than SGM_WARPS warps
+    // (128 scanlines at 2 lanes each).  More of them read and write more rows at
+    // once than the caches hold: 20 uneven pairs took 1.8 ms with 8 warps per SM,
     // 2.0 with 12, 2.7 with 28, and 2.3 with 4.
-    const long long cap = (long long)sms * (ctas_per_sm < 4 ? 1 : ctas_per_sm / 4);
+    const int most = threads / 32 < SGM_WARPS ? SGM_WARPS / (threads / 32) : 1;
+    const long long cap = (long long)sms * (ctas_per_sm < most ? ctas_per_sm : most);
     const unsigned blocks = (unsigned)(want < cap ? (want < 1 ? 1 : want) : cap);
     const size_t smem = (size_t)(threads / 32) * SgmRing<NR, GL>::WARP;
-    const int rc = allow_smem(k_b_sgm<NR, GL, LT, PAD>, smem, 256 / 32 * SgmRing<NR, GL>::WARP);
+    const int rc = allow_smem(k_b_sgm<NR, GL, LT, PAD>, smem, SGM_WARPS * SgmRing<NR, GL>::WARP);
     if (rc) return rc;
     count_launch();
     pdl(k_b_sgm<NR, GL, LT, PAD>, blocks, threads, smem, st)(t, tasks);

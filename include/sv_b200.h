@@ -153,9 +153,9 @@ int sv_batch_lr_refine(const sv_pair_desc *pairs, int n, int dtype, double tol,
 /* Scheduling of sv_batch_lr_refine_ex (results do not depend on it): pixels
  * per CTA of the per-pixel stages (base, band costs, WTA, left-right check;
  * a power of 2 in 256..8192), threads per CTA of the persistent SGM kernel
- * (32/64/128/256), four times its CTAs per SM (1..32: a quarter, at least one,
- * is launched), and the lanes' tasks a warp claims per fetch from the queue
- * (32/64/128, over the lanes of a scanline).  batch.autotune picks them by
+ * (32/64/128/256), its CTAs per SM (1..32, of which as many are launched as make
+ * up 8 warps: more only thrash the caches), and the lanes' tasks a warp claims per
+ * fetch from the queue (32/64/128, over the lanes of a scanline).  batch.autotune picks them by
  * timing the caller's batch.  No reference counterpart. */
 typedef struct sv_batch_config {
     int px_per_block;
