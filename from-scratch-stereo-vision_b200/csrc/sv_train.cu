@@ -27,6 +27,7 @@
 // siamese towers run as one batch of 2B images (the B left views, then the
 // B right views).
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -1188,6 +1189,7 @@ struct TrainBufs {
     float *t0, *t1, *t2, *tce, *gl0, *gl1, *gl2;
     float *gs, *gs0, *gA, *gB, *grin, *gd0, *gcost, *gq2, *gq1, *gvol, *gf, *gF3, *gF4;
     float *partial;
+    long partial_n;
     double *loss;
 };
 
@@ -1211,16 +1213,22 @@ long tiles2d(int nimg, int OH, int OW) {
     return (long)nimg * ((OH + 3) / 4) * ((OW + 31) / 32);
 }
 
-// every layer's partial sums, at most kWgCtas CTAs each
-long partial_floats(const sv_trainer *t) {
+// Partial sums, at most kWgCtas CTAs a layer: of every layer, so that one launch adds
+// them all up, or (all false) of the widest one, the least a step can do with.
+long partial_floats(const sv_trainer *t, bool all) {
     const int C = t->C, Cm = t->Cm, Rc = t->Rc;
+    if (!all) {
+        const long layers[3] = {(long)C * (C * 9 + 1), (long)Cm * (C * 27 + 1),
+                                (long)Rc * (Rc * 9 + 1)};
+        return *std::max_element(layers, layers + 3) * kWgCtas;
+    }
     long n = (long)C * (9 + 1) + 3L * C * (C * 9 + 1);
     n += (long)Cm * (C * 27 + 1) + (long)Cm * (Cm * 27 + 1) + (Cm * 27 + 1);
     n += 2L * (Rc * (2 * 9 + 1) + (long)(t->nd - 1) * Rc * (Rc * 9 + 1) + (Rc * 9 + 1));
     return n * kWgCtas;
 }
 
-void carve(const sv_trainer *t, const Dims &d, Carver &cv, TrainBufs &b) {
+void carve(const sv_trainer *t, const Dims &d, Carver &cv, TrainBufs &b, bool all) {
     const int B = d.B, C = t->C, Cm = t->Cm, D = t->D, Rc = t->Rc;
     const long DHW = (long)D * d.hw;
     b.img = cv.take<float>(2 * B * d.HW);
@@ -1266,7 +1274,8 @@ void carve(const sv_trainer *t, const Dims &d, Carver &cv, TrainBufs &b) {
     b.gf = cv.take<float>(2L * B * C * d.hw);
     b.gF3 = cv.take<float>(2L * B * C * d.h1w1);
     b.gF4 = cv.take<float>(2L * B * C * d.hw);
-    b.partial = cv.take<float>(partial_floats(t));
+    b.partial_n = partial_floats(t, all);
+    b.partial = cv.take<float>(b.partial_n);
     b.loss = cv.take<double>(B);
 }
 
@@ -1331,13 +1340,23 @@ int conv3d_go(const float *x, int B, int D, int h, int w, const float *wt, const
     return SV_OK;
 }
 
-// The weight gradients leave their partial sums in b.partial and a job each;
-// reduce_all adds them up.
+// The weight gradients leave their partial sums in b.partial and a job each; reduce
+// adds up the ones there: at the end, or before a layer whose sums no longer fit.
 struct WGrads {
     float *partial;
+    long cap;
+    double *grads;
+    cudaStream_t st;
     long used = 0;
     ReduceJobs jobs{};
+    void reduce() {
+        count_launch();
+        pdl(k_treduce, jobs.block[jobs.n], dim3(32, 32), 0, st)(partial, jobs, grads);
+        jobs = ReduceJobs{};
+        used = 0;
+    }
     int add(int nblk, int OC, int K, long gw, long gb) {
+        if (used + (long)nblk * OC * K > cap) reduce();
         const int l = jobs.n++;
         jobs.nblk[l] = nblk;
         jobs.OC[l] = OC;
@@ -1408,8 +1427,7 @@ int train_impl(sv_trainer *t, const float *left, const float *right, const float
     const float *P = t->p32;
     const float invB = 1.0f / (float)B;
     constexpr int CH = C % 4 == 0 ? 4 : C, CMH = CM % 3 == 0 ? 3 : 2;   // staged channels in 3-D
-    WGrads wg;
-    wg.partial = b.partial;
+    WGrads wg{b.partial, b.partial_n, t->g64, st};
     int rc;
     // inputs: the B left views, then the B right views
     if (cudaMemcpyAsync(b.img, left, sizeof(float) * B * d.HW, cudaMemcpyDeviceToDevice, st) !=
@@ -1591,8 +1609,7 @@ int train_impl(sv_trainer *t, const float *left, const float *right, const float
     if ((rc = wgrad2d<1, C, 2>(b.img, b.gF3, 2 * B, d.H, d.W, d.h1, d.w1, 1, wg, t->off_fw[0],
                                t->off_fb[0], st)))
         return rc;
-    count_launch();
-    pdl(k_treduce, wg.jobs.block[wg.jobs.n], dim3(32, 32), 0, st)(b.partial, wg.jobs, t->g64);
+    wg.reduce();
     SV_LAUNCH_CHECK();
     // ---- per-sample loss and the prediction
     count_launch();
@@ -1741,7 +1758,7 @@ size_t sv_train_workspace_size(const sv_trainer *t, int B, int W, int H) {
     if (check_dims(t, B, W, H) != SV_OK) return 0;
     Carver cv(nullptr);
     TrainBufs b;
-    carve(t, dims(B, W, H), cv, b);
+    carve(t, dims(B, W, H), cv, b, true);
     return cv.off + 256;
 }
 
@@ -1751,15 +1768,20 @@ int sv_train_grads(sv_trainer *t, const float *left, const float *right, const f
     if (!t || !left || !right || !disp || !valid) { set_error("NULL argument"); return SV_ERR_NULL; }
     int rc = check_dims(t, B, W, H);
     if (rc) return rc;
+    // a smaller workspace does too: the partial sums are then added up more often
     const size_t need = sv_train_workspace_size(t, B, W, H);
-    if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255)) {
-        set_error("workspace must be 256-byte aligned and hold %zu bytes", need);
+    const bool all = workspace_bytes >= need;
+    const Dims d = dims(B, W, H);
+    TrainBufs b;
+    Carver least(nullptr);
+    carve(t, d, least, b, false);
+    if (!workspace || workspace_bytes < least.off + 256 || ((uintptr_t)workspace & 255)) {
+        set_error("workspace must be 256-byte aligned and hold %zu bytes (%zu for the fewest "
+                  "launches)", least.off + 256, need);
         return SV_ERR_WORKSPACE;
     }
     Carver cv(workspace);
-    TrainBufs b;
-    const Dims d = dims(B, W, H);
-    carve(t, d, cv, b);
+    carve(t, d, cv, b, all);
     cudaStream_t st = (cudaStream_t)stream;
     if (t->C == 12)
         return train_impl<12, 6, 8>(t, left, right, disp, valid, d, b, pred, loss, st);

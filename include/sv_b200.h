@@ -547,6 +547,10 @@ int sv_trainer_get_params(const sv_trainer *t, double *out, long n);
 int sv_trainer_get_grads(const sv_trainer *t, double *out, long n);
 int sv_trainer_set_params(sv_trainer *t, const double *params, long n);
 int sv_trainer_set_grads(sv_trainer *t, const double *grads, long n);
+/* The weight gradients' partial sums are most of what does not grow with the batch;
+ * sv_train_grads also takes a workspace with room for the widest layer's only (592 *
+ * max(C (9 C + 1), Cm (27 C + 1), Rc (9 Rc + 1)) floats in the place of 592 * all
+ * layers' OC (taps * IC + 1)), with a launch more for each time they fill it. */
 size_t sv_train_workspace_size(const sv_trainer *t, int B, int W, int H);
 /* left, right, disp: FP32 [B][H][W] (gray in [0, 1], ground-truth
  * disparity); valid: [B][H][W] (nonzero = known).  Leaves the batch
