@@ -342,7 +342,7 @@ constexpr int kDrawBits = 7;                 // up to 64 trials
 // squaring (as many as nseg has bits), their tables, then a scan of the
 // eligibility and one table look-up per set bit of each segment's count (by
 // columns, four times the instructions: 16 us for 1,147 segments, now 13).
-// draw[j] is the table of M^(3*2^j): the segments jump to their trials' draws.
+// draw[j] is M^(3*2^j): the segments jump to their trials' draws.
 __global__ void __launch_bounds__(1024)
     k_seg_rng(int nseg, const int *__restrict__ count, const int *__restrict__ nvalid, int trials,
               uint32_t seed, int *__restrict__ start, uint32_t *__restrict__ state,
@@ -374,8 +374,7 @@ __global__ void __launch_bounds__(1024)
         }
     }
     __syncthreads();
-    for (int k = t; k < kDrawBits * kGfTab; k += blockDim.x)
-        draw[k] = gf2_entry(DJ[k / kGfTab], k % kGfTab);
+    if (t < kDrawBits * 32) draw[t] = DJ[t / 32][t % 32];
     for (int k = t; k < kJumpBits * kGfTab && (nseg >> (k / kGfTab)); k += blockDim.x)
         JT[k / kGfTab][k % kGfTab] = gf2_entry(J[k / kGfTab], k % kGfTab);
     __syncthreads();
@@ -536,6 +535,7 @@ __global__ void __launch_bounds__(kSnapThreads)
     __shared__ int ok[kMaxTrials], cnt[kMaxTrials];
     __shared__ int sbuf[32], wcnt[kSnapScan][kSnapThreads / 32];
     __shared__ double fit[3];
+    __shared__ uint32_t jump[kDrawBits * kGfTab];      // tables of the jumps over draws
     extern __shared__ __align__(16) double rows[];     // [3][cap]
     const int g = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int n = nvalid[g];
@@ -544,6 +544,8 @@ __global__ void __launch_bounds__(kSnapThreads)
     const int ww = w.y - w.x + 1, wn = ww * (w.w - w.z + 1);
     const bool staged = n <= cap;
     int *const gp = pts + start[g], *const gi = inl + start[g];
+    for (int k = t; k < kDrawBits * kGfTab; k += kSnapThreads)
+        jump[k] = gf2_entry(draw + k / kGfTab * 32, k % kGfTab);
     // valid pixels in index order, kSnapScan x kSnapThreads of the window at a time
     int base = 0;
     for (int k0 = 0; k0 < wn; k0 += kSnapScan * kSnapThreads) {
@@ -591,7 +593,7 @@ __global__ void __launch_bounds__(kSnapThreads)
     if (t < trials) {
         uint32_t s = state[g];
         for (int j = 0; j < kDrawBits; ++j)
-            if ((t >> j) & 1) s = gf2_lookup(draw + kGfTab * j, s);
+            if ((t >> j) & 1) s = gf2_lookup(jump + kGfTab * j, s);
         double A[3][3], bv[3];
         for (int u = 0; u < 3; ++u) {
             s = xorshift32(s);
@@ -695,7 +697,11 @@ size_t carve_post(void *ws, int W, int H, int step, PostWs *o) {
     p.flags = cv.take<DevFlags>(1);
     p.cs = cv.take<unsigned char>(sizeof(SlicCenter) * nca);
     p.win = cv.take<int4>(nca);
-    p.dist = cv.take<unsigned long long>(N);
+    // the jump matrices lie where SLIC's distances were
+    const size_t words = (size_t)kDrawBits * 32 * sizeof(uint32_t);
+    p.dist = cv.take<unsigned long long>(N * sizeof(unsigned long long) > words ? N
+                                             : words / sizeof(unsigned long long));
+    p.draw = reinterpret_cast<uint32_t *>(p.dist);
     p.labtmp = cv.take<int>(N);
     p.lab = cv.take<int>(N);
     p.count = cv.take<int>(nca);
@@ -704,7 +710,6 @@ size_t carve_post(void *ws, int W, int H, int step, PostWs *o) {
     p.inl = cv.take<int>(N);
     p.nvalid = cv.take<int>(nca);
     p.state = cv.take<uint32_t>(nca);
-    p.draw = cv.take<uint32_t>(kGfTab * kDrawBits);
     p.valid = cv.take<uint8_t>(N);
     p.tmp = cv.take<double>(N);
     if (o) *o = p;

@@ -21,7 +21,7 @@ struct PostWs {
     int *pts, *inl;             // per segment: valid pixels, inliers (same offsets)
     int *nvalid;
     uint32_t *state;            // per segment: xorshift32 state at its first draw
-    uint32_t *draw;             // jumps over 3 * 2^j draws
+    uint32_t *draw;             // jumps over 3 * 2^j draws, over dist after the last SLIC
     uint8_t *valid;             // status == 0 (refine_disparity)
     double *tmp;                // intermediate disparity
 };
