@@ -61,8 +61,10 @@ SIGNATURES = {
     "sv_aggregate_path": (_I, [_VP, _VP, _I, _I, _I, _I, _I, _I, _I, _VP, _VP]),
     "sv_left_to_right": (_I, [_VP, _I, _I, _VP, _VP]),
     "sv_refine_workspace_size": (_SZ, [_I, _I, _PRM]),
+    "sv_refine_workspace_least": (_SZ, [_I, _I, _PRM]),
     "sv_refine_fullres": (_I, [_VP, _VP, _I, _VP, _I, _I, _PRM, _VP, _VP, _VP, _SZ, _VP]),
     "sv_lr_refine_workspace_size": (_SZ, [_I, _I, _PRM]),
+    "sv_lr_refine_workspace_least": (_SZ, [_I, _I, _PRM]),
     "sv_lr_refine": (_I, [_VP, _VP, _I, _VP, _I, _I, _D, _PRM, _VP, _VP, _VP, _SZ, _VP]),
     "sv_lr_refine_timed": (_I, [_VP, _VP, _I, _VP, _I, _I, _D, _PRM, _VP, _VP, _VP, _SZ, _VP,
                                 ctypes.POINTER(_VP), _I]),
@@ -70,12 +72,14 @@ SIGNATURES = {
     "sv_selftest_wait_timeout": (_I, [ctypes.c_uint, _VP, _VP]),
     "sv_selftest_slot_wait": (_I, [_VP]),
     "sv_batch_lr_refine_workspace_size": (_SZ, [_VP, _I, _PRM]),
+    "sv_batch_lr_refine_workspace_least": (_SZ, [_VP, _I, _PRM]),
     "sv_batch_lr_refine": (_I, [_VP, _I, _I, _D, _PRM, _VP, _SZ, _VP]),
     "sv_batch_config_default": (None, [_VP]),
     "sv_batch_lr_refine_ex": (_I, [_VP, _I, _I, _D, _PRM, _VP, _VP, _SZ, _VP]),
     "sv_netbatch_create": (_I, [_VP, _IP, _IP, _I, _I, _D, _I, _I, _I, _I, _D, _PRM,
                                 ctypes.POINTER(_VP)]),
     "sv_netbatch_workspace_size": (_SZ, [_VP]),
+    "sv_netbatch_workspace_least": (_SZ, [_VP]),
     "sv_netbatch_bind": (_I, [_VP, _VP, _VP, _SZ, _VP]),
     "sv_netbatch_run": (_I, [_VP, _VP]),
     "sv_netbatch_predict": (_I, [_VP, _VP]),
@@ -106,6 +110,7 @@ SIGNATURES = {
     "sv_plane_snap": (_I, [_VP, _VP, _I, _I, _VP, _I, _D, _D, _I, ctypes.c_uint32, _VP, _VP, _SZ,
                            _VP]),
     "sv_refine_disparity_workspace_size": (_SZ, [_I, _I, _PRM, _I]),
+    "sv_refine_disparity_workspace_least": (_SZ, [_I, _I, _PRM, _I]),
     "sv_refine_disparity": (_I, [_VP, _VP, _I, _VP, _VP, _I, _I, _D, _PRM, _I, _I, _D, _D, _VP,
                                  _VP, _VP, _SZ, _VP]),
     "sv_lr_refine_band": (_I, [_VP, _VP, _I, _VP, _VP, _I, _I, _D, _PRM, _VP, _VP, _VP, _SZ,

@@ -33,7 +33,7 @@ import torch
 
 from . import _lib
 from .refine import _data_status, _device, _finite_disp, _image, _params, _ptr, _ret, _stream, \
-    _to_dev, _workspace
+    _to_dev, _workspace, _workspace_or_least
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 DEFAULT_WEIGHTS = os.path.join(HERE, "weights", "band_weights.npz")
@@ -248,7 +248,8 @@ def lr_refine_band(left, right, centre, rad, W, H, tol=2.0, **kw):
     need = lib.sv_lr_refine_workspace_size(W, H, ctypes.byref(p))
     if need == 0:
         _lib.raise_last("lr_refine_band")
-    ws = _workspace(need)
+    ws, need = _workspace_or_least(
+        need, lambda: lib.sv_lr_refine_workspace_least(W, H, ctypes.byref(p)))
     out = torch.empty(N, dtype=torch.float64, device=tc.device)
     st = torch.empty(N, dtype=torch.uint8, device=tc.device)
     _lib.check(lib.sv_lr_refine_band(_ptr(tl), _ptr(tr), code, _ptr(tc), _ptr(trad), W, H,
@@ -279,7 +280,8 @@ class LearnedBandRefiner:
         self.fneed = self.lib.sv_band_features_workspace_size(W, H)
         self.fws = _workspace(self.fneed)
         self.rneed = self.lib.sv_lr_refine_workspace_size(W, H, ctypes.byref(self.p))
-        self.rws = _workspace(self.rneed)
+        self.rws, self.rneed = _workspace_or_least(
+            self.rneed, lambda: self.lib.sv_lr_refine_workspace_least(W, H, ctypes.byref(self.p)))
         self.bws, self.bneed = band._workspace(1, W, H)
 
     def run(self, left, right, code, disp0, out, status, stream, spread, pmax):

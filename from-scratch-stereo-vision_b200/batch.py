@@ -32,7 +32,8 @@ import numpy as np
 import torch
 
 from . import _lib
-from .refine import _device, _image, _kind, _params, _ptr, _ret, _stream, _to_dev, _finite_disp
+from .refine import _device, _image, _kind, _params, _ptr, _ret, _stream, _to_dev, _finite_disp, \
+    _workspace_or_least
 
 
 class PairDesc(ctypes.Structure):
@@ -103,7 +104,9 @@ class BatchRefiner:
                                                                ctypes.byref(self.p))
         if self.need == 0:
             _lib.raise_last("lr_refine_batch")
-        self.ws = torch.empty(self.need, dtype=torch.uint8, device=dev)
+        self.ws, self.need = _workspace_or_least(
+            self.need, lambda: self.lib.sv_batch_lr_refine_workspace_least(
+                self.descs, len(self.sizes), ctypes.byref(self.p)))
 
     @property
     def pixels(self) -> int:
@@ -248,8 +251,9 @@ class NetBatch:
         for i, (W, H) in enumerate(self.sizes):
             self.descs[i] = PairDesc(self.left[i].data_ptr(), self.right[i].data_ptr(), None,
                                      self.out[i].data_ptr(), self.status[i].data_ptr(), W, H)
-        self.need = self.lib.sv_netbatch_workspace_size(self.handle)
-        self.ws = torch.empty(self.need, dtype=torch.uint8, device=dev)
+        self.ws, self.need = _workspace_or_least(
+            self.lib.sv_netbatch_workspace_size(self.handle),
+            lambda: self.lib.sv_netbatch_workspace_least(self.handle))
         _lib.check(self.lib.sv_netbatch_bind(self.handle, self.descs, _ptr(self.ws), self.need,
                                              _stream()), "sv_netbatch_bind")
 

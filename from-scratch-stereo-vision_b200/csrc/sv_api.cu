@@ -73,6 +73,7 @@ int check_refine(int W, int H, const sv_refine_params *p, bool rows, RefineCfg *
 }
 
 struct RefineWs {
+    bool pad;                                // layout of the costs and path costs
     DevFlags *flags;
     int32_t *base0, *base1;
     double *d0r, *dl, *dr;
@@ -81,15 +82,23 @@ struct RefineWs {
     void *L;
 };
 
-static size_t carve_refine(void *ws, int W, int H, const RefineCfg &c, int nviews,
+// pad: the rows of 32 bytes, or of 64 slots, that are the faster ones.  Without it the
+// rows are as short as the slots allow and the census maps, which the band costs alone
+// read, lie where the path costs are written after them: what is left when the caller's
+// workspace, or the device's memory, does not hold the other (1397 x 1101, K = 21: 738
+// MB and 582 us a pass, 960 MB and 540 with it; K = 41 1.38 GB and 1428 us, 1.85 and 1481).
+static size_t carve_refine(void *ws, int W, int H, const RefineCfg &c, int nviews, bool pad,
                            RefineWs *o) {
-    const size_t N = (size_t)W * H, NK = N * cost_row_bytes(c.K);
+    const size_t N = (size_t)W * H, NK = N * cost_row_bytes(c.K, pad);
     Carver cv(ws);
     RefineWs r{};
+    r.pad = pad;
     r.flags = cv.take<DevFlags>(1);
     r.base0 = cv.take<int32_t>(N);
-    r.cen0 = cv.take<uint64_t>(N);
-    r.cen1 = cv.take<uint64_t>(N);
+    if (pad) {
+        r.cen0 = cv.take<uint64_t>(N);
+        r.cen1 = cv.take<uint64_t>(N);
+    }
     r.C0 = cv.take<uint8_t>(NK);
     if (nviews == 2) {
         r.base1 = cv.take<int32_t>(N);
@@ -98,10 +107,26 @@ static size_t carve_refine(void *ws, int W, int H, const RefineCfg &c, int nview
         r.dr = cv.take<double>(N);
         r.C1 = cv.take<uint8_t>(NK);
     }
-    size_t lbytes = (size_t)nviews * c.npaths * N * path_row_bytes(c.K, c.l16, true);
-    r.L = cv.take<uint8_t>(lbytes);
+    const size_t lbytes = (size_t)nviews * c.npaths * N * path_row_bytes(c.K, c.l16, pad);
+    const size_t cbytes = align256(N * sizeof(uint64_t));
+    char *L = cv.take<char>(pad || lbytes > 2 * cbytes ? lbytes : 2 * cbytes);
+    r.L = L;
+    if (!pad && L) {
+        r.cen0 = reinterpret_cast<uint64_t *>(L);
+        r.cen1 = reinterpret_cast<uint64_t *>(L + cbytes);
+    }
     if (o) *o = r;
     return cv.off;
+}
+
+// The caller's workspace in the layout that it has room for.
+static int refine_ws(void *ws, size_t bytes, int W, int H, const RefineCfg &c, int nviews,
+                     RefineWs *o) {
+    const bool pad = bytes >= carve_refine(nullptr, W, H, c, nviews, true, nullptr);
+    const int rc = check_ws(ws, bytes, carve_refine(nullptr, W, H, c, nviews, pad, nullptr));
+    if (rc) return rc;
+    carve_refine(ws, W, H, c, nviews, pad, o);
+    return SV_OK;
 }
 
 int check_ws(void *ws, size_t have, size_t need) {
@@ -228,13 +253,25 @@ int sv_left_to_right(const double *dl, int W, int H, double *dr, void *stream) {
 size_t sv_refine_workspace_size(int W, int H, const sv_refine_params *p) {
     RefineCfg c;
     if (check_refine(W, H, p, false, &c) != SV_OK) return 0;
-    return carve_refine(nullptr, W, H, c, 1, nullptr);
+    return carve_refine(nullptr, W, H, c, 1, true, nullptr);
+}
+
+size_t sv_refine_workspace_least(int W, int H, const sv_refine_params *p) {
+    RefineCfg c;
+    if (check_refine(W, H, p, false, &c) != SV_OK) return 0;
+    return carve_refine(nullptr, W, H, c, 1, false, nullptr);
 }
 
 size_t sv_lr_refine_workspace_size(int W, int H, const sv_refine_params *p) {
     RefineCfg c;
     if (check_refine(W, H, p, true, &c) != SV_OK) return 0;
-    return carve_refine(nullptr, W, H, c, 2, nullptr);
+    return carve_refine(nullptr, W, H, c, 2, true, nullptr);
+}
+
+size_t sv_lr_refine_workspace_least(int W, int H, const sv_refine_params *p) {
+    RefineCfg c;
+    if (check_refine(W, H, p, true, &c) != SV_OK) return 0;
+    return carve_refine(nullptr, W, H, c, 2, false, nullptr);
 }
 
 int sv_refine_fullres(const void *left, const void *right, int dtype, const double *disp0,
@@ -243,19 +280,18 @@ int sv_refine_fullres(const void *left, const void *right, int dtype, const doub
     if (!left || !right || !disp0 || !out) { set_error("NULL argument"); return SV_ERR_NULL; }
     RefineCfg c;
     SV_TRY(check_refine(W, H, p, false, &c));
-    SV_TRY(check_ws(workspace, workspace_bytes, carve_refine(nullptr, W, H, c, 1, nullptr)));
     RefineWs w;
-    carve_refine(workspace, W, H, c, 1, &w);
+    SV_TRY(refine_ws(workspace, workspace_bytes, W, H, c, 1, &w));
     cudaStream_t st = (cudaStream_t)stream;
     const long N = (long)W * H;
     SV_CUDA_TRY(cudaMemsetAsync(w.flags, 0, sizeof(DevFlags), st));
     SV_TRY(launch_base(disp0, N, w.base0, &w.flags->status, st));
     SV_TRY(launch_census(left, right, dtype, W, H, c.rx, c.ry, w.cen0, w.cen1, st));
     SV_TRY(launch_band_costs_slot(w.cen0, w.cen1, w.base0, nullptr, W, H, c.R, c.invalid, w.C0,
-                             nullptr, 1, st));
+                             nullptr, 1, st, nullptr, w.pad));
     SV_TRY(launch_sgm_packed(w.C0, nullptr, w.base0, nullptr, W, H, c.K, c.P1, c.P2, w.L, c.l16,
-                             true, 1, c.npaths, st));
-    SV_TRY(launch_wta_slot(w.L, c.l16, true, c.npaths, 1, W, H, c.R, w.base0, nullptr, disp0, nullptr,
+                             w.pad, 1, c.npaths, st));
+    SV_TRY(launch_wta_slot(w.L, c.l16, w.pad, c.npaths, 1, W, H, c.R, w.base0, nullptr, disp0, nullptr,
                       c.uniq, out, nullptr, conf, st));
     return SV_OK;
 }
@@ -282,9 +318,8 @@ static int lr_refine_impl(const void *left, const void *right, int dtype, const 
         set_error("stage timing needs %d events", SV_LR_STAGES + 1);
         return SV_ERR_PARAM;
     }
-    SV_TRY(check_ws(workspace, workspace_bytes, carve_refine(nullptr, W, H, c, 2, nullptr)));
     RefineWs w;
-    carve_refine(workspace, W, H, c, 2, &w);
+    SV_TRY(refine_ws(workspace, workspace_bytes, W, H, c, 2, &w));
     cudaStream_t st = (cudaStream_t)stream;
     int ev = 0;
     auto mark = [&]() -> int {
@@ -301,12 +336,12 @@ static int lr_refine_impl(const void *left, const void *right, int dtype, const 
         SV_TRY(launch_census(left, right, dtype, W, H, c.rx, c.ry, w.cen0, w.cen1, st));
     SV_TRY(mark());
     SV_TRY(launch_band_costs_slot(w.cen0, w.cen1, w.base0, w.base1, W, H, c.R, c.invalid, w.C0,
-                             w.C1, 2, st, rad));
+                             w.C1, 2, st, rad, w.pad));
     SV_TRY(mark());
     SV_TRY(launch_sgm_packed(w.C0, w.C1, w.base0, w.base1, W, H, c.K, c.P1, c.P2, w.L, c.l16,
-                             true, 2, c.npaths, st));
+                             w.pad, 2, c.npaths, st));
     SV_TRY(mark());
-    SV_TRY(launch_wta_slot(w.L, c.l16, true, c.npaths, 2, W, H, c.R, w.base0, w.base1, disp0, w.d0r,
+    SV_TRY(launch_wta_slot(w.L, c.l16, w.pad, c.npaths, 2, W, H, c.R, w.base0, w.base1, disp0, w.d0r,
                       c.uniq, w.dl, w.dr, nullptr, st));
     SV_TRY(mark());
     SV_TRY(launch_lr_check(w.dl, w.dr, disp0, W, H, tol, out, status, st));

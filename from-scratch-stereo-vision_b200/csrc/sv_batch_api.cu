@@ -23,10 +23,11 @@ constexpr int kTileW = 32, kTileH = 8;   // census tile (k_census)
 }  // namespace
 
 // Sizes and offsets; with ws != nullptr also fills the per-pair pointers.
-int plan_batch(const sv_pair_desc *in, int n, const RefineCfg &c, int px_per_block, char *ws,
-               BatchPlan *pl) {
+int plan_batch(const sv_pair_desc *in, int n, const RefineCfg &c, int px_per_block, bool pad,
+               char *ws, BatchPlan *pl) {
     BatchPlan &P = *pl;
-    const size_t crow = cost_row_bytes(c.K), lrow = path_row_bytes(c.K, c.l16, true);
+    P.pad = pad;
+    const size_t crow = cost_row_bytes(c.K, pad), lrow = path_row_bytes(c.K, c.l16, pad);
     Carver cv(ws);
     cv.take<DevFlags>(1);
     cv.take<int>(64);                                      // queue counter (+ padding)
@@ -73,11 +74,20 @@ int plan_batch(const sv_pair_desc *in, int n, const RefineCfg &c, int px_per_blo
         b.d0r = cv.take<double>(N);
         b.dl = cv.take<double>(N);
         b.dr = cv.take<double>(N);
-        b.cen0 = cv.take<uint64_t>(N);
-        b.cen1 = cv.take<uint64_t>(N);
+        if (pad) {
+            b.cen0 = cv.take<uint64_t>(N);
+            b.cen1 = cv.take<uint64_t>(N);
+        }
         b.C0 = cv.take<uint8_t>(N * crow);
         b.C1 = cv.take<uint8_t>(N * crow);
-        b.L = cv.take<uint8_t>(2 * (size_t)c.npaths * N * lrow);
+        const size_t lbytes = 2 * (size_t)c.npaths * N * lrow;
+        const size_t cbytes = align256(N * sizeof(uint64_t));
+        char *L = cv.take<char>(pad || lbytes > 2 * cbytes ? lbytes : 2 * cbytes);
+        b.L = L;
+        if (!pad && L) {            // the census maps, read before the path costs are written
+            b.cen0 = reinterpret_cast<uint64_t *>(L);
+            b.cen1 = reinterpret_cast<uint64_t *>(L + cbytes);
+        }
         P.px_blk[i + 1] = P.px_blk[i] + (long long)((N + px_per_block - 1) / px_per_block);
         P.row_blk[i + 1] = P.row_blk[i] + d.H;
         P.tile_blk[i + 1] = P.tile_blk[i] + (long long)((d.W + kTileW - 1) / kTileW) *
@@ -158,7 +168,8 @@ BatchTables batch_tables(const BatchPlan &pl, int n, char *ws, const RefineCfg &
     t.queue = reinterpret_cast<int *>(ws + sizeof(DevFlags));
     t.R = c.R;
     t.K = c.K;
-    t.Kp = slot_width(c.K);
+    t.pad = pl.pad;
+    t.Kp = slot_width(c.K, pl.pad);
     t.P1 = c.P1;
     t.P2 = c.P2;
     t.npaths = c.npaths;
@@ -180,8 +191,7 @@ using namespace sv;
 
 extern "C" {
 
-size_t sv_batch_lr_refine_workspace_size(const sv_pair_desc *pairs, int n,
-                                         const sv_refine_params *p) {
+static size_t batch_ws(const sv_pair_desc *pairs, int n, const sv_refine_params *p, bool pad) {
     if (!pairs || n < 1) return 0;
     RefineCfg c;
     if (check_refine(1, 1, p, true, &c) != SV_OK) return 0;
@@ -190,8 +200,18 @@ size_t sv_batch_lr_refine_workspace_size(const sv_pair_desc *pairs, int n,
         return 0;
     }
     BatchPlan pl;
-    if (plan_batch(pairs, n, c, kBatchPxPerBlock, nullptr, &pl) != SV_OK) return 0;
+    if (plan_batch(pairs, n, c, kBatchPxPerBlock, pad, nullptr, &pl) != SV_OK) return 0;
     return pl.total;
+}
+
+size_t sv_batch_lr_refine_workspace_size(const sv_pair_desc *pairs, int n,
+                                         const sv_refine_params *p) {
+    return batch_ws(pairs, n, p, true);
+}
+
+size_t sv_batch_lr_refine_workspace_least(const sv_pair_desc *pairs, int n,
+                                          const sv_refine_params *p) {
+    return batch_ws(pairs, n, p, false);
 }
 
 void sv_batch_config_default(sv_batch_config *cfg) {
@@ -240,9 +260,12 @@ int sv_batch_lr_refine_ex(const sv_pair_desc *pairs, int n, int dtype, double to
         return SV_ERR_PARAM;
     }
     BatchPlan pl;
-    if ((rc = plan_batch(pairs, n, c, cfg->px_per_block, nullptr, &pl))) return rc;
+    if ((rc = plan_batch(pairs, n, c, cfg->px_per_block, true, nullptr, &pl))) return rc;
+    const bool pad = workspace_bytes >= pl.total;
+    if (!pad && (rc = plan_batch(pairs, n, c, cfg->px_per_block, false, nullptr, &pl))) return rc;
     if ((rc = check_ws(workspace, workspace_bytes, pl.total))) return rc;
-    if ((rc = plan_batch(pairs, n, c, cfg->px_per_block, static_cast<char *>(workspace), &pl)))
+    if ((rc = plan_batch(pairs, n, c, cfg->px_per_block, pad, static_cast<char *>(workspace),
+                         &pl)))
         return rc;
     char *ws = static_cast<char *>(workspace);
     cudaStream_t st = (cudaStream_t)stream;

@@ -172,7 +172,7 @@ struct sv_netbatch {
     SlabLayout lay;
     size_t slab;
     // workspace layout
-    size_t off_pairs, off_lt, off_rt, off_pre, off_slabs, off_refine, total;
+    size_t off_pairs, off_lt, off_rt, off_pre, off_slabs, off_refine, total, least;
     BatchPlan plan;
     // bound state
     char *ws;
@@ -424,23 +424,27 @@ int sv_netbatch_create(const sv_net *net, const int *W, const int *H, int n, int
         d[i].W = W[i];
         d[i].H = H[i];
     }
-    if ((rc = plan_batch(d.data(), n, c, nb->cfg.px_per_block, nullptr, &nb->plan))) {
-        delete nb;
-        return rc;
+    for (bool pad : {false, true}) {
+        if ((rc = plan_batch(d.data(), n, c, nb->cfg.px_per_block, pad, nullptr, &nb->plan))) {
+            delete nb;
+            return rc;
+        }
+        (pad ? nb->total : nb->least) = nb->off_refine + nb->plan.total;
     }
-    nb->total = nb->off_refine + nb->plan.total;
     *out = nb;
     return SV_OK;
 }
 
 size_t sv_netbatch_workspace_size(const sv_netbatch *nb) { return nb ? nb->total : 0; }
+size_t sv_netbatch_workspace_least(const sv_netbatch *nb) { return nb ? nb->least : 0; }
 
 int sv_netbatch_bind(sv_netbatch *nb, const sv_pair_desc *pairs, void *workspace,
                      size_t workspace_bytes, void *stream) {
     int rc = nb_check(nb);
     if (rc) return rc;
     if (!pairs) { set_error("NULL pairs"); return SV_ERR_NULL; }
-    if ((rc = check_ws(workspace, workspace_bytes, nb->total))) return rc;
+    const bool pad = workspace_bytes >= nb->total;
+    if ((rc = check_ws(workspace, workspace_bytes, pad ? nb->total : nb->least))) return rc;
     const int n = nb->n;
     char *ws = static_cast<char *>(workspace);
     std::vector<sv_pair_desc> d(pairs, pairs + n);
@@ -462,7 +466,7 @@ int sv_netbatch_bind(sv_netbatch *nb, const sv_pair_desc *pairs, void *workspace
                                                       nb->lay.full);
     }
     std::lock_guard<std::mutex> lock(nb->mu);
-    if ((rc = plan_batch(d.data(), n, nb->rc, nb->cfg.px_per_block, ws + nb->off_refine,
+    if ((rc = plan_batch(d.data(), n, nb->rc, nb->cfg.px_per_block, pad, ws + nb->off_refine,
                          &nb->plan)))
         return rc;
     cudaStream_t st = (cudaStream_t)stream;

@@ -91,12 +91,20 @@ int sv_plane_snap(const double *disp, const double *rgb, int W, int H, const uin
                              (cudaStream_t)stream);
 }
 
-size_t sv_refine_disparity_workspace_size(int W, int H, const sv_refine_params *p,
-                                          int plane_step) {
-    const size_t a = sv_lr_refine_workspace_size(W, H, p);
+static size_t disparity_ws(int W, int H, int plane_step, size_t a) {
     const size_t b = sv_postproc_workspace_size(W, H, plane_step < 1 ? 1 : plane_step);
     if (!a || !b) return 0;
     return align256(a) + b;
+}
+
+size_t sv_refine_disparity_workspace_size(int W, int H, const sv_refine_params *p,
+                                          int plane_step) {
+    return disparity_ws(W, H, plane_step, sv_lr_refine_workspace_size(W, H, p));
+}
+
+size_t sv_refine_disparity_workspace_least(int W, int H, const sv_refine_params *p,
+                                           int plane_step) {
+    return disparity_ws(W, H, plane_step, sv_lr_refine_workspace_least(W, H, p));
 }
 
 int sv_refine_disparity(const void *left, const void *right, int dtype, const double *rgb,
@@ -110,14 +118,16 @@ int sv_refine_disparity(const void *left, const void *right, int dtype, const do
     const size_t a = sv_lr_refine_workspace_size(W, H, p);
     if (!a) return sv_lr_refine(left, right, dtype, disp0, W, H, tol, p, out, status, nullptr, 0,
                                 stream);   // reports the parameter error
-    const size_t need = sv_refine_disparity_workspace_size(W, H, p, plane_step);
-    SV_TRY_POST(check_ws_post(workspace, workspace_bytes, need));
+    // lr_refine's part in the layout that the workspace has room for, then the rest's
+    const bool full = workspace_bytes >= disparity_ws(W, H, plane_step, a);
+    const size_t part = full ? a : sv_lr_refine_workspace_least(W, H, p);
+    SV_TRY_POST(check_ws_post(workspace, workspace_bytes, disparity_ws(W, H, plane_step, part)));
     cudaStream_t st = (cudaStream_t)stream;
     char *base = static_cast<char *>(workspace);
     SV_TRY_POST(sv_lr_refine(left, right, dtype, disp0, W, H, tol, p, out, status, base,
-                             align256(a), stream));
+                             align256(part), stream));
     PostWs w;
-    carve_post(base + align256(a), W, H, plane_step, &w);
+    carve_post(base + align256(part), W, H, plane_step, &w);
     const long N = (long)W * H;
     if (planes && rgb) {
         SV_TRY_POST(launch_status_valid(status, N, w.valid, st));

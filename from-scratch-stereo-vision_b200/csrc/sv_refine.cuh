@@ -48,7 +48,7 @@ inline SgmTasks make_sgm_tasks(int W, int H, int nviews, int npaths, const int *
 
 // Slots per pixel of the fused refinement's layout (K + 2 rounded up to a
 // table width) and the bytes of a pixel's cost and path-cost rows (sv_sgm.cu).
-// pad: path-cost rows of the 24-slot layout padded to 32 bytes.
+// pad: path-cost rows of the 24-slot layout padded to 32 bytes, 64 slots for 48.
 int slot_width(int K, bool pad = true);
 size_t cost_row_bytes(int K, bool pad = true);
 size_t path_row_bytes(int K, bool l16, bool pad);
@@ -94,6 +94,7 @@ struct BatchTables {
     int nseg;
     int *queue;                  // SGM task counter, zeroed per call
     int *flag;                   // data errors (first wins)
+    bool pad;                    // layout of the path costs (slot_width)
     int R, K, Kp, P1, P2, npaths, invalid, rx, ry, dtype, maxW;
     int px_per_block;            // pixels per CTA of the per-pixel stages
     int sgm_fetch;               // scanline tasks a warp claims per queue fetch
@@ -118,12 +119,14 @@ struct BatchPlan {
     std::vector<int> seg_pair, seg_vd;
     long long px_blocks = 0, rows = 0, tiles = 0, tasks = 0;
     int maxW = 1;
+    bool pad = true;             // layout of the costs and path costs
     size_t off_tables = 0, off_pairs = 0, off_px = 0, off_row = 0, off_tile = 0, off_seg = 0,
            off_segp = 0, off_segvd = 0, total = 0;
 };
-// Sizes and offsets; with ws != nullptr also fills the per-pair pointers.
-int plan_batch(const sv_pair_desc *in, int n, const RefineCfg &c, int px_per_block, char *ws,
-               BatchPlan *pl);
+// Sizes and offsets; with ws != nullptr also fills the per-pair pointers.  pad false:
+// the smaller layout (sv_lr_refine_workspace_least).
+int plan_batch(const sv_pair_desc *in, int n, const RefineCfg &c, int px_per_block, bool pad,
+               char *ws, BatchPlan *pl);
 int upload_batch(const BatchPlan &pl, int n, char *ws, cudaStream_t st);
 BatchTables batch_tables(const BatchPlan &pl, int n, char *ws, const RefineCfg &c, int dtype,
                          double tol, const sv_batch_config &cfg);

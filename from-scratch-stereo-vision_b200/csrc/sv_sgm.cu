@@ -1095,7 +1095,11 @@ int launch_batch_refine(const BatchTables &t, long long px_blocks, long long row
     switch (t.Kp) {
         SV_BGO(8, 4, 1)
         SV_BGO(16, 4, 2)
-        SV_BGO(24, 6, 2)
+    case 24:
+        rc = l16 ? batch_sgm_go<6, 2, uint16_t, false>(t, tasks, sgm_threads, sgm_ctas_per_sm, st)
+             : t.pad ? batch_sgm_go<6, 2, uint8_t, true>(t, tasks, sgm_threads, sgm_ctas_per_sm, st)
+                     : batch_sgm_go<6, 2, uint8_t, false>(t, tasks, sgm_threads, sgm_ctas_per_sm, st);
+        break;
         SV_BGO(32, 8, 2)
     default:
         set_error("batched refinement supports bands up to K = 30 (got K = %d)", t.K);
@@ -1106,6 +1110,7 @@ int launch_batch_refine(const BatchTables &t, long long px_blocks, long long row
     count_launch();
     if (l16 && t.Kp <= 16) pdl(k_b_wta<uint16_t, 0, false, 0, 1>, px, 256, 0, st)(t);
     else if (l16) pdl(k_b_wta<uint16_t, 0, false, 0, 2>, px, 256, 0, st)(t);
+    else if (t.Kp == 24 && !t.pad) pdl(k_b_wta<uint8_t, 24, false, 0, 1>, px, 256, 0, st)(t);
     else if (t.Kp == 24 && t.npaths == 8) pdl(k_b_wta<uint8_t, 24, true, 8, 1>, px, 256, 0, st)(t);
     else if (t.Kp == 24) pdl(k_b_wta<uint8_t, 24, true, 0, 1>, px, 256, 0, st)(t);
     else if (t.Kp == 8) pdl(k_b_wta<uint8_t, 8, true, 0, 1>, px, 256, 0, st)(t);

@@ -16,7 +16,7 @@ import torch
 
 from . import _lib
 from .refine import _data_status, _finite_disp, _image, _params, _ptr, _ret, _stream, _to_dev, \
-    _workspace
+    _workspace, _workspace_or_least
 
 
 def _f64(x, n, name):
@@ -86,7 +86,9 @@ def refine_disparity(left, right, rgb, disp0, W, H, R=10, P1=12.0, P2=150.0, rx=
     need = lib.sv_refine_disparity_workspace_size(W, H, ctypes.byref(p), int(plane_step))
     if need == 0:
         _lib.raise_last("refine_disparity")
-    ws = _workspace(need)
+    ws, need = _workspace_or_least(
+        need, lambda: lib.sv_refine_disparity_workspace_least(W, H, ctypes.byref(p),
+                                                              int(plane_step)))
     out = torch.empty(N, dtype=torch.float64, device=td.device)
     st = torch.empty(N, dtype=torch.uint8, device=td.device)
     _lib.check(lib.sv_refine_disparity(_ptr(tl), _ptr(tr), code, _ptr(r), _ptr(td), W, H,

@@ -125,6 +125,16 @@ def _workspace(nbytes: int) -> torch.Tensor:
     return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=_device())
 
 
+def _workspace_or_least(need: int, least) -> tuple[torch.Tensor, int]:
+    """A workspace of `need` bytes, or of least() where the device has no room for it
+    (same results, slower), and its size."""
+    try:
+        return _workspace(need), need
+    except torch.OutOfMemoryError:
+        n = least()
+        return _workspace(n), n
+
+
 def _ptr(t) -> ctypes.c_void_p:
     return ctypes.c_void_p(t.data_ptr()) if t is not None else ctypes.c_void_p(0)
 
@@ -231,7 +241,8 @@ def refine_fullres(left, right, disp0, W, H, R=3, P1=1.0, P2=12.0, ad_weight=0.0
     need = lib.sv_refine_workspace_size(W, H, ctypes.byref(p))
     if need == 0:
         _lib.raise_last("refine_fullres")
-    ws = _workspace(need)
+    ws, need = _workspace_or_least(
+        need, lambda: lib.sv_refine_workspace_least(W, H, ctypes.byref(p)))
     out = torch.empty(N, dtype=torch.float64, device=td.device)
     conf = torch.empty(N, dtype=torch.float64, device=td.device) if return_conf else None
     _lib.check(lib.sv_refine_fullres(_ptr(tl), _ptr(tr), code, _ptr(td), W, H,
@@ -269,7 +280,8 @@ def lr_refine(left, right, disp0, W, H, tol=1.0, **kw):
     need = lib.sv_lr_refine_workspace_size(W, H, ctypes.byref(p))
     if need == 0:
         _lib.raise_last("lr_refine")
-    ws = _workspace(need)
+    ws, need = _workspace_or_least(
+        need, lambda: lib.sv_lr_refine_workspace_least(W, H, ctypes.byref(p)))
     out = torch.empty(N, dtype=torch.float64, device=td.device)
     st = torch.empty(N, dtype=torch.uint8, device=td.device)
     _lib.check(lib.sv_lr_refine(_ptr(tl), _ptr(tr), code, _ptr(td), W, H, float(tol),
@@ -292,7 +304,8 @@ class LRRefiner:
         self.need = self.lib.sv_lr_refine_workspace_size(W, H, ctypes.byref(self.p))
         if self.need == 0:
             raise ValueError("unsupported refinement parameters for %dx%d" % (W, H))
-        self.ws = _workspace(self.need)
+        self.ws, self.need = _workspace_or_least(
+            self.need, lambda: self.lib.sv_lr_refine_workspace_least(W, H, ctypes.byref(self.p)))
 
     def run(self, left: torch.Tensor, right: torch.Tensor, disp0: torch.Tensor,
             out: torch.Tensor, status: torch.Tensor, stream: int | None = None) -> None:

@@ -11,6 +11,9 @@
  *    Nothing synchronises unless the comment says so.
  *  - Scratch memory comes from a caller-owned workspace whose size the
  *    matching *_workspace_size() call returns (256-byte aligned pointer).
+ *    Where a *_workspace_least() call stands beside it, the call also takes a
+ *    workspace of at least that size, with the same results, up to a tenth
+ *    slower: for images and batches that fill the device's memory.
  *    The library itself allocates device memory only for network weights
  *    (sv_net_create).
  *  - Every call returns an SV_* status.  Argument errors are detected before
@@ -104,6 +107,7 @@ int sv_left_to_right(const double *dl, int W, int H, double *dr, void *stream);
  * left/right are [H][W] of `dtype`; disp0 and out are FP64 [H][W];
  * conf (optional, may be NULL) receives the return_conf values. */
 size_t sv_refine_workspace_size(int W, int H, const sv_refine_params *p);
+size_t sv_refine_workspace_least(int W, int H, const sv_refine_params *p);
 int sv_refine_fullres(const void *left, const void *right, int dtype,
                       const double *disp0, int W, int H,
                       const sv_refine_params *p, double *out, double *conf,
@@ -112,6 +116,9 @@ int sv_refine_fullres(const void *left, const void *right, int dtype,
 /* lr_refine, stereonet.py:5343-5391: both views, left-right check and the
  * occlusion / mismatch fills.  status: 0 ok, 1 occluded, 2 mismatch. */
 size_t sv_lr_refine_workspace_size(int W, int H, const sv_refine_params *p);
+/* Two views at K = 15 to 22 and 8-bit path costs: 624 bytes per pixel, the least 480;
+ * at K = 31 to 46 (64 or 48 slots) 1,200 and 896. */
+size_t sv_lr_refine_workspace_least(int W, int H, const sv_refine_params *p);
 int sv_lr_refine(const void *left, const void *right, int dtype,
                  const double *disp0, int W, int H, double tol,
                  const sv_refine_params *p, double *out, uint8_t *status,
@@ -146,6 +153,8 @@ typedef struct sv_pair_desc {
 } sv_pair_desc;
 size_t sv_batch_lr_refine_workspace_size(const sv_pair_desc *pairs, int n,
                                          const sv_refine_params *p);
+size_t sv_batch_lr_refine_workspace_least(const sv_pair_desc *pairs, int n,
+                                          const sv_refine_params *p);
 int sv_batch_lr_refine(const sv_pair_desc *pairs, int n, int dtype, double tol,
                        const sv_refine_params *p, void *workspace,
                        size_t workspace_bytes, void *stream);
@@ -317,6 +326,7 @@ int sv_netbatch_create(const sv_net *net, const int *W, const int *H, int n, int
                        int precision, double tol, const sv_refine_params *p,
                        sv_netbatch **out);
 size_t sv_netbatch_workspace_size(const sv_netbatch *nb);
+size_t sv_netbatch_workspace_least(const sv_netbatch *nb);
 int sv_netbatch_bind(sv_netbatch *nb, const sv_pair_desc *pairs, void *workspace,
                      size_t workspace_bytes, void *stream);
 int sv_netbatch_run(sv_netbatch *nb, void *stream);
@@ -381,6 +391,8 @@ int sv_plane_snap(const double *disp, const double *rgb, int W, int H,
  * status-0 pixels when planes != 0 and rgb != NULL, 3x3 median */
 size_t sv_refine_disparity_workspace_size(int W, int H, const sv_refine_params *p,
                                           int plane_step);
+size_t sv_refine_disparity_workspace_least(int W, int H, const sv_refine_params *p,
+                                           int plane_step);
 int sv_refine_disparity(const void *left, const void *right, int dtype,
                         const double *rgb, const double *disp0, int W, int H,
                         double tol, const sv_refine_params *p, int planes,
