@@ -5,8 +5,8 @@
 // bit-identical to refining it alone); what changes is the scheduling: the
 // workspace holds one slice per pair, small device tables map blocks and
 // SGM tasks to pairs, and the SGM stage is a persistent kernel draining a
-// device-side queue of (pair, view, direction, scanline) tasks, longest
-// scanlines first.
+// device-side queue of (pair, view, direction, scanline) tasks: the largest
+// pair's first, and of a pair the longest scanlines.
 
 #include <algorithm>
 #include <cmath>

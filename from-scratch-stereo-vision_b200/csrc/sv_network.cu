@@ -411,7 +411,7 @@ __device__ __forceinline__ void conv_level(int lv, int Hw, int Ww, int &H, int &
     }
 }
 
-// 3x3 convolutions (padding = dilation; stride S = 1, or 2 with dilation 1)
+// 3x3 convolutions (padding and dilation 1, stride S = 1 or 2: the feature net)
 // with every output channel in one thread and PX pixels per thread, CTB_TW /
 // PX columns apart: the register-blocked form of k_conv2d_tiled<IC, OC, *,
 // ACT, CS>.  It keeps that kernel's arithmetic exactly -- each of the CS
@@ -425,10 +425,9 @@ constexpr int CTB_TW = 32, CTB_TH = 4;          // output tile of a CTA
 
 template <int IC, int OC, int ACT, int CS, int PX, int S>
 __device__ __forceinline__ void conv2d_wide_body(int bx, int by, const float *__restrict__ x,
-                                                 int H, int W, int OH, int OW, int dil,
+                                                 int H, int W, int OH, int OW,
                                                  const float *__restrict__ w,
-                                                 const float *__restrict__ b, float *y,
-                                                 const float *__restrict__ resid) {
+                                                 const float *__restrict__ b, float *y) {
     constexpr int CPS = IC / CS, TXP = CTB_TW / PX, NT = TXP * CTB_TH;
     constexpr int OCP = (OC + 3) / 4 * 4;
     static_assert(IC % CS == 0 && (CS == 1 || CS == 2 || CS == 4) && OC <= 16, "shape");
@@ -443,8 +442,8 @@ __device__ __forceinline__ void conv2d_wide_body(int bx, int by, const float *__
     }
     if (tid < OCP) sb[tid] = tid < OC ? b[tid] : 0.f;
     const int ox0 = bx * CTB_TW, oy0 = by * CTB_TH;
-    const int ix0 = ox0 * S - dil, iy0 = oy0 * S - dil;
-    const int tw = (CTB_TW - 1) * S + 2 * dil + 1, th = (CTB_TH - 1) * S + 2 * dil + 1;
+    const int ix0 = ox0 * S - 1, iy0 = oy0 * S - 1;
+    const int tw = (CTB_TW - 1) * S + 3, th = (CTB_TH - 1) * S + 3;
     const long HW = (long)H * W;
     for (int i = tid; i < IC * th * tw; i += NT) {
         const int c = i / (th * tw);
@@ -471,12 +470,12 @@ __device__ __forceinline__ void conv2d_wide_body(int bx, int by, const float *__
             const float *tc = tile + c * th * tw;
 #pragma unroll
             for (int ky = 0; ky < 3; ++ky) {
-                const float *row = tc + (ly * S + ky * dil) * tw + lx * S;
+                const float *row = tc + (ly * S + ky) * tw + lx * S;
 #pragma unroll
                 for (int kx = 0; kx < 3; ++kx) {
                     float v[PX];
 #pragma unroll
-                    for (int q = 0; q < PX; ++q) v[q] = row[kx * dil + q * TXP * S];
+                    for (int q = 0; q < PX; ++q) v[q] = row[kx + q * TXP * S];
                     const float *wt = sw + (c * 9 + ky * 3 + kx) * OCP;
 #pragma unroll
                     for (int o4 = 0; o4 < OCP; o4 += 4) {
@@ -506,10 +505,6 @@ __device__ __forceinline__ void conv2d_wide_body(int bx, int by, const float *__
             else s = acc[0][q][o];
             float v = s + sb[o];
             if (ACT == 1) v = v > 0.f ? v : v * 0.2f;
-            if (ACT == 2) {
-                v = resid[oi] + v;
-                v = v > 0.f ? v : v * 0.f;
-            }
             y[o * OHW + oi] = v;
         }
     }
@@ -545,9 +540,9 @@ __global__ void __launch_bounds__(CT2_TW *CT2_TH * 4)
 // The batched form: level lv of conv_level, Z images (1 or 2) per pair.
 template <int IC, int OC, int ACT, int CS, int PX, int S>
 __global__ void __launch_bounds__(CTB_TW / PX * CTB_TH)
-    k_b_conv2d_wide(NetLaunch L, int lv, int Z, const float *x0, const float *x1, int dil,
+    k_b_conv2d_wide(NetLaunch L, int lv, int Z, const float *x0, const float *x1,
                     const float *__restrict__ w, const float *__restrict__ b, float *y0,
-                    float *y1, const float *resid) {
+                    float *y1) {
     pdl_sync();
     long long c;
     const int p = net_pair(L, c);
@@ -561,25 +556,19 @@ __global__ void __launch_bounds__(CTB_TW / PX * CTB_TH)
     const int bx = (int)(t % tx), by = (int)(t / tx);
     if (by >= ty) return;
     conv2d_wide_body<IC, OC, ACT, CS, PX, S>(bx, by, net_slab(img ? x1 : x0, L, p), H, W, OH,
-                                             OW, dil, w, b, net_slab(img ? y1 : y0, L, p),
-                                             net_slab(resid, L, p));
-}
-
-static size_t conv2d_wide_bytes(int IC, int S, int dil) {
-    return (size_t)IC * ((CTB_TW - 1) * S + 2 * dil + 1) * ((CTB_TH - 1) * S + 2 * dil + 1) *
-           sizeof(float);
+                                             OW, w, b, net_slab(img ? y1 : y0, L, p));
 }
 
 template <int IC, int OC, int ACT, int CS, int PX, int S>
 static int b_conv2d_wide(const NetLaunch &L, unsigned ctas, int lv, int Z, const float *x0,
-                         const float *x1, int dil, const float *w, const float *b, float *y0,
-                         float *y1, const float *resid, cudaStream_t st) {
-    const size_t smem = conv2d_wide_bytes(IC, S, dil);
-    const int rc = allow_smem(k_b_conv2d_wide<IC, OC, ACT, CS, PX, S>, smem,
-                              conv2d_wide_bytes(IC, S, 1));      // the feature net: dilation 1
+                         const float *x1, const float *w, const float *b, float *y0, float *y1,
+                         cudaStream_t st) {
+    constexpr size_t smem =
+        (size_t)IC * ((CTB_TW - 1) * S + 3) * ((CTB_TH - 1) * S + 3) * sizeof(float);
+    const int rc = allow_smem(k_b_conv2d_wide<IC, OC, ACT, CS, PX, S>, smem, smem);
     if (rc) return rc;
     pdl(k_b_conv2d_wide<IC, OC, ACT, CS, PX, S>, ctas, CTB_TW / PX * CTB_TH, smem, st)(
-        L, lv, Z, x0, x1, dil, w, b, y0, y1, resid);
+        L, lv, Z, x0, x1, w, b, y0, y1);
     return SV_OK;
 }
 
@@ -1790,7 +1779,7 @@ static void stage_ctas_impl(const NetView &n, int Hm, int Wm, long long *o) {
     constexpr int FG = C % 4 == 0 ? 4 : C;
     constexpr int S1 = C % 4 == 0 ? 4 : 2, S2 = CM % 4 == 0 && CM > 4 ? 4 : 2;
     constexpr int RG = RC % 4 == 0 ? 4 : RC;
-    // one table serves k_b_conv2d_tiled and k_b_conv2d_wide launches alike
+    // one count of tiles serves k_b_conv2d_up and k_b_conv2d_wide alike
     static_assert(CTB_TW == CT2_TW && CTB_TH == CT2_TH, "the two 2-D tile shapes must agree");
     auto t2 = [](int OW, int OH) {
         return (long long)((OW + CT2_TW - 1) / CT2_TW) * ((OH + CT2_TH - 1) / CT2_TH);
@@ -1843,20 +1832,20 @@ static int b_forward_impl(const NetView &n, const NetStageLaunch &g, const NetSl
     // FeatureNet, both images: every output channel and 2 pixels per thread
     // (the arithmetic of k_conv2d_tiled<.., FG, .., 1 or 2>)
     count_launch();
-    if ((rc = b_conv2d_wide<1, C, 1, 1, 2, 2>(L(NK_C1W), B(NK_C1W), 0, 2, s.lw, s.rw, 1, n.fw[0], n.fb[0],
-                                              s.f.fa[0], s.f.fa[1], nullptr, st)))
+    if ((rc = b_conv2d_wide<1, C, 1, 1, 2, 2>(L(NK_C1W), B(NK_C1W), 0, 2, s.lw, s.rw, n.fw[0],
+                                              n.fb[0], s.f.fa[0], s.f.fa[1], st)))
         return rc;
     count_launch();
-    if ((rc = b_conv2d_wide<C, C, 1, 2, 2, 2>(L(NK_C2W), B(NK_C2W), 1, 2, s.f.fa[0], s.f.fa[1], 1,
-                                              n.fw[1], n.fb[1], s.f.fb[0], s.f.fb[1], nullptr, st)))
+    if ((rc = b_conv2d_wide<C, C, 1, 2, 2, 2>(L(NK_C2W), B(NK_C2W), 1, 2, s.f.fa[0], s.f.fa[1],
+                                              n.fw[1], n.fb[1], s.f.fb[0], s.f.fb[1], st)))
         return rc;
     count_launch();
-    if ((rc = b_conv2d_wide<C, C, 1, 2, 2, 1>(L(NK_C2W), B(NK_C2W), 2, 2, s.f.fb[0], s.f.fb[1], 1,
-                                              n.fw[2], n.fb[2], s.f.fa[0], s.f.fa[1], nullptr, st)))
+    if ((rc = b_conv2d_wide<C, C, 1, 2, 2, 1>(L(NK_C2W), B(NK_C2W), 2, 2, s.f.fb[0], s.f.fb[1],
+                                              n.fw[2], n.fb[2], s.f.fa[0], s.f.fa[1], st)))
         return rc;
     count_launch();
-    if ((rc = b_conv2d_wide<C, C, 0, 2, 2, 1>(L(NK_C2W), B(NK_C2W), 2, 2, s.f.fa[0], s.f.fa[1], 1,
-                                              n.fw[3], n.fb[3], s.f.fb[0], s.f.fb[1], nullptr, st)))
+    if ((rc = b_conv2d_wide<C, C, 0, 2, 2, 1>(L(NK_C2W), B(NK_C2W), 2, 2, s.f.fa[0], s.f.fa[1],
+                                              n.fw[3], n.fb[3], s.f.fb[0], s.f.fb[1], st)))
         return rc;
     SV_LAUNCH_CHECK();
     constexpr int S1 = C % 4 == 0 ? 4 : 2, S2 = CM % 4 == 0 && CM > 4 ? 4 : 2;

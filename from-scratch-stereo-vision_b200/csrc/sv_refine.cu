@@ -90,10 +90,11 @@ __device__ __forceinline__ void census_tile(const T *__restrict__ img, int W, in
     const int x = tx0 + threadIdx.x, y = ty0 + threadIdx.y;
     if (x >= W || y >= H) return;
     const T *ctr = tile + (threadIdx.y + ry) * sw + threadIdx.x + rx;
-    if (rx == 4 && ry == 3) {       // the 9 x 7 window of refine_disparity
-        out[(long)y * W + x] = census_bits<T, 4, 3>(ctr);
-        return;
-    }
+    if constexpr (sizeof(T) > 1)    // (8-bit images: census_tile_u8)
+        if (rx == 4 && ry == 3) {   // the 9 x 7 window of refine_disparity
+            out[(long)y * W + x] = census_bits<T, 4, 3>(ctr);
+            return;
+        }
     const T c = *ctr;
     uint64_t s = 0;
     for (int dy = -ry; dy <= ry; ++dy) {
@@ -237,8 +238,8 @@ __global__ void k_band_costs(const uint64_t *__restrict__ cl,
 }
 
 // ------------------------------------------------------------------- SGM
-// stereonet.py:5192-5241.  One warp sweeps one scanline of one direction of
-// one view.  Band index k lives at flat position i = lane*V + j + 1 (so
+// stereonet.py:5192-5241: one path of one view, added to S (sv_aggregate_path).  One
+// warp sweeps one scanline.  Band index k lives at flat position i = lane*V + j + 1 (so
 // position 0 stands for k = -1 and position K+1 for k = K); V values per lane
 // cover K + 2 <= 32V.  Per pixel:
 //   t(k)   = min(Lq(k), Lq(k-1)+P1, Lq(k+1)+P1)        (INF outside 0..K-1)
@@ -275,20 +276,14 @@ __device__ __forceinline__ void shift_band(const int (&t)[V], int (&o)[V], int s
     }
 }
 
-template <int V, typename LT, bool ADD_S>
+template <int V>
 __global__ void __launch_bounds__(256)
-    k_sgm(const uint8_t *__restrict__ C0, const uint8_t *__restrict__ C1,
-          const int32_t *__restrict__ base0, const int32_t *__restrict__ base1,
-          int W, int H, int K, int P1, int P2, LT *__restrict__ Lout, int npaths,
-          SgmTasks tasks) {
+    k_sgm(const uint8_t *__restrict__ C, const int32_t *__restrict__ base, int W, int H, int K,
+          int P1, int P2, int dir, int lines, uint16_t *__restrict__ S) {
     pdl_sync();
     const int lane = threadIdx.x & 31;
-    const int gw = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5);
-    if (gw >= tasks.start[tasks.nseg]) return;
-    int sg = 0;
-    while (gw >= tasks.start[sg + 1]) ++sg;
-    const int j0 = gw - tasks.start[sg];
-    const int view = tasks.view[sg], dir = tasks.dir[sg];
+    const int j0 = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5);
+    if (j0 >= lines) return;
     const int dx = c_dirs[dir][0], dy = c_dirs[dir][1];
 
     int x0, y0, n;
@@ -308,10 +303,6 @@ __global__ void __launch_bounds__(256)
         int ny = dy > 0 ? H - y0 : y0 + 1;
         n = min(nx, ny);
     }
-    const uint8_t *__restrict__ C = view ? C1 : C0;
-    const int32_t *__restrict__ base = view ? base1 : base0;
-    const long N = (long)W * H;
-    LT *__restrict__ Lo = ADD_S ? Lout : Lout + (long)(view * npaths + dir) * N * K;
     const long step = (long)dy * W + dx;
     const long p0 = (long)y0 * W + x0;
 
@@ -374,15 +365,8 @@ __global__ void __launch_bounds__(256)
             bprev = bg[u];
             mq = (int)__reduce_min_sync(kFull, (unsigned)lmin);
 #pragma unroll
-            for (int j = 0; j < V; ++j) {
-                if (kv[j]) {
-                    if (ADD_S) {
-                        Lo[pp * K + kk[j]] = (LT)(Lo[pp * K + kk[j]] + L[j]);
-                    } else {
-                        Lo[pp * K + kk[j]] = (LT)L[j];
-                    }
-                }
-            }
+            for (int j = 0; j < V; ++j)
+                if (kv[j]) S[pp * K + kk[j]] = (uint16_t)(S[pp * K + kk[j]] + L[j]);
             int up = __shfl_up_sync(kFull, L[V - 1], 1);
             int dn = __shfl_down_sync(kFull, L[0], 1);
             if (lane == 0) up = kInf;
@@ -633,36 +617,26 @@ int launch_band_costs(const uint64_t *cl, const uint64_t *cr, const int32_t *bas
 
 static int band_vals(int K) { return (K + 2 + 31) / 32; }
 
-template <int V, typename LT, bool ADD>
-static int sgm_dispatch_lt(const uint8_t *C0, const uint8_t *C1, const int32_t *b0,
-                           const int32_t *b1, int W, int H, int K, int P1, int P2,
-                           void *Lout, int npaths, const SgmTasks &tasks,
-                           cudaStream_t st) {
-    long warps = tasks.start[tasks.nseg];
-    int blocks = (int)((warps * 32 + 255) / 256);
-    count_launch(); pdl(k_sgm<V, LT, ADD>, blocks, 256, 0, st)(C0, C1, b0, b1, W, H, K, P1, P2,
-                                              (LT *)Lout, npaths, tasks);
+template <int V>
+static int sgm_add(const uint8_t *C, const int32_t *base, int W, int H, int K, int P1, int P2,
+                   int dir, uint16_t *S, cudaStream_t st) {
+    const int lines = dir < 2 ? H : dir < 4 ? W : W + H - 1;
+    count_launch();
+    pdl(k_sgm<V>, (unsigned)((lines * 32L + 255) / 256), 256, 0, st)(C, base, W, H, K, P1, P2, dir,
+                                                                     lines, S);
     SV_LAUNCH_CHECK();
     return SV_OK;
 }
 
-template <typename LT, bool ADD>
-static int sgm_dispatch(const uint8_t *C0, const uint8_t *C1, const int32_t *b0,
-                        const int32_t *b1, int W, int H, int K, int P1, int P2,
-                        void *Lout, int npaths, const SgmTasks &tasks, cudaStream_t st) {
-    switch (band_vals(K)) {
-    case 1: return sgm_dispatch_lt<1, LT, ADD>(C0, C1, b0, b1, W, H, K, P1, P2, Lout, npaths, tasks, st);
-    case 2: return sgm_dispatch_lt<2, LT, ADD>(C0, C1, b0, b1, W, H, K, P1, P2, Lout, npaths, tasks, st);
-    case 3:
-    case 4: return sgm_dispatch_lt<4, LT, ADD>(C0, C1, b0, b1, W, H, K, P1, P2, Lout, npaths, tasks, st);
-    default: return sgm_dispatch_lt<8, LT, ADD>(C0, C1, b0, b1, W, H, K, P1, P2, Lout, npaths, tasks, st);
-    }
-}
-
 int launch_sgm_add_path(const uint8_t *C, const int32_t *base, int W, int H, int K,
                         int P1, int P2, int dir, uint16_t *S, cudaStream_t st) {
-    SgmTasks t = make_sgm_tasks(W, H, 1, 8, &dir, 1);
-    return sgm_dispatch<uint16_t, true>(C, C, base, base, W, H, K, P1, P2, S, 1, t, st);
+    switch (band_vals(K)) {
+    case 1: return sgm_add<1>(C, base, W, H, K, P1, P2, dir, S, st);
+    case 2: return sgm_add<2>(C, base, W, H, K, P1, P2, dir, S, st);
+    case 3:
+    case 4: return sgm_add<4>(C, base, W, H, K, P1, P2, dir, S, st);
+    default: return sgm_add<8>(C, base, W, H, K, P1, P2, dir, S, st);
+    }
 }
 
 // Shared memory of a row kernel: a row of doubles, integers and bytes.

@@ -8,44 +8,6 @@
 
 namespace sv {
 
-// Scanline work table of the SGM kernels: segment i covers the scanlines of
-// (view[i], dir[i]); start[] are cumulative scanline counts.
-struct SgmTasks {
-    int nseg;
-    int start[17];
-    int view[16];
-    int dir[16];
-};
-
-// Longest scanlines first (horizontal, vertical, diagonal) so that the
-// longest-running warps start in the first wave.  dirs_only restricts the
-// table to the listed directions (one view).
-inline SgmTasks make_sgm_tasks(int W, int H, int nviews, int npaths, const int *dirs_only,
-                               int ndirs_only) {
-    SgmTasks t{};
-    int order[8] = {0, 1, 2, 3, 4, 5, 6, 7};
-    if (H > W) { order[0] = 2; order[1] = 3; order[2] = 0; order[3] = 1; }
-    t.start[0] = 0;
-    for (int oi = 0; oi < 8; ++oi) {
-        const int d = order[oi];
-        if (dirs_only) {
-            bool keep = false;
-            for (int i = 0; i < ndirs_only; ++i) keep |= dirs_only[i] == d;
-            if (!keep) continue;
-        } else if (d >= npaths) {
-            continue;
-        }
-        const int cnt = d < 2 ? H : d < 4 ? W : W + H - 1;
-        for (int v = 0; v < nviews; ++v) {
-            t.view[t.nseg] = v;
-            t.dir[t.nseg] = d;
-            t.start[t.nseg + 1] = t.start[t.nseg] + cnt;
-            t.nseg++;
-        }
-    }
-    return t;
-}
-
 // Slots per pixel of the fused refinement's layout (K + 2 rounded up to a
 // table width) and the bytes of a pixel's cost and path-cost rows (sv_sgm.cu).
 // pad: path-cost rows of the 24-slot layout padded to 32 bytes, 64 slots for 48.

@@ -899,7 +899,9 @@ static int sgm_dispatch(const uint8_t *C0, const uint8_t *C1, const int32_t *b0,
     case 16: SV_SGM(4, 2);
     case 24: SV_SGM(6, 2);
     case 32: SV_SGM(8, 2);
-    case 48: SV_SGM(6, 4);
+    case 48:                                       // slot_width: only without padding
+        if constexpr (!PAD) SV_SGM(6, 4);
+        break;
     case 64: SV_SGM(8, 4);
     case 96: SV_SGM(12, 4);
     case 128: SV_SGM(8, 8);
@@ -963,14 +965,15 @@ int launch_wta_slot(const void *L, bool l16, bool pad, int npaths, int nviews, i
 // ====================================================================
 // Batched lr_refine, middle stages.  Costs and WTA run one block per
 // px_per_block pixels of a pair (blockIdx.y = view).  The SGM is a
-// persistent kernel over a device-side queue: every warp takes sgm_fetch
-// (32 by default) scanline tasks at a time from one atomic counter, tasks
-// ordered longest scanline first (segments of (pair, view, direction) sorted by length on the host),
-// so all pairs' scanlines share one launch and finish together.
+// persistent kernel over a device-side queue: every warp takes sgm_fetch / GL
+// scanlines (sgm_fetch 32 by default) at a time from one atomic counter.  The
+// host orders them pair by pair, the largest pair first, and within a pair by
+// length (segments of (view, direction)), so all pairs share one launch, a
+// pair's directions find its costs in L2, and the small pairs come last.
 // ====================================================================
 
-// KPC / KC / NPC > 0: the band geometry fixed at compile time, as in the
-// single-pair kernels (the whole batch shares K).
+// KC > 0: K fixed at compile time, as in the single-pair kernel (the whole batch
+// shares K).
 template <bool KP24, int KC>
 __global__ void __launch_bounds__(256) k_b_costs(BatchTables t) {
     pdl_sync();
