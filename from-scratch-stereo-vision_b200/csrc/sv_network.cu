@@ -411,7 +411,7 @@ __device__ __forceinline__ void conv_level(int lv, int Hw, int Ww, int &H, int &
     }
 }
 
-// 3x3 convolutions (padding and dilation 1, stride S = 1 or 2: the feature net)
+// 3x3 convolutions (padding = dilation, here 1; stride S = 1 or 2: the feature net)
 // with every output channel in one thread and PX pixels per thread, CTB_TW /
 // PX columns apart: the register-blocked form of k_conv2d_tiled<IC, OC, *,
 // ACT, CS>.  It keeps that kernel's arithmetic exactly -- each of the CS
@@ -421,11 +421,13 @@ __device__ __forceinline__ void conv_level(int lv, int Hw, int Ww, int &H, int &
 // -- so its results are bit-identical to that kernel's, from one staged
 // input tile for all output channels and one 16-byte weight vector per 4
 // output channels, read by the whole warp at once.
+// The dilation is an argument: with the constant 1 in its place the 12 -> 12 stride-2
+// layer of 20 uneven pairs took 238 us instead of 177.
 constexpr int CTB_TW = 32, CTB_TH = 4;          // output tile of a CTA
 
 template <int IC, int OC, int ACT, int CS, int PX, int S>
 __device__ __forceinline__ void conv2d_wide_body(int bx, int by, const float *__restrict__ x,
-                                                 int H, int W, int OH, int OW,
+                                                 int H, int W, int OH, int OW, int dil,
                                                  const float *__restrict__ w,
                                                  const float *__restrict__ b, float *y) {
     constexpr int CPS = IC / CS, TXP = CTB_TW / PX, NT = TXP * CTB_TH;
@@ -442,8 +444,8 @@ __device__ __forceinline__ void conv2d_wide_body(int bx, int by, const float *__
     }
     if (tid < OCP) sb[tid] = tid < OC ? b[tid] : 0.f;
     const int ox0 = bx * CTB_TW, oy0 = by * CTB_TH;
-    const int ix0 = ox0 * S - 1, iy0 = oy0 * S - 1;
-    const int tw = (CTB_TW - 1) * S + 3, th = (CTB_TH - 1) * S + 3;
+    const int ix0 = ox0 * S - dil, iy0 = oy0 * S - dil;
+    const int tw = (CTB_TW - 1) * S + 2 * dil + 1, th = (CTB_TH - 1) * S + 2 * dil + 1;
     const long HW = (long)H * W;
     for (int i = tid; i < IC * th * tw; i += NT) {
         const int c = i / (th * tw);
@@ -470,12 +472,12 @@ __device__ __forceinline__ void conv2d_wide_body(int bx, int by, const float *__
             const float *tc = tile + c * th * tw;
 #pragma unroll
             for (int ky = 0; ky < 3; ++ky) {
-                const float *row = tc + (ly * S + ky) * tw + lx * S;
+                const float *row = tc + (ly * S + ky * dil) * tw + lx * S;
 #pragma unroll
                 for (int kx = 0; kx < 3; ++kx) {
                     float v[PX];
 #pragma unroll
-                    for (int q = 0; q < PX; ++q) v[q] = row[kx + q * TXP * S];
+                    for (int q = 0; q < PX; ++q) v[q] = row[kx * dil + q * TXP * S];
                     const float *wt = sw + (c * 9 + ky * 3 + kx) * OCP;
 #pragma unroll
                     for (int o4 = 0; o4 < OCP; o4 += 4) {
@@ -540,7 +542,7 @@ __global__ void __launch_bounds__(CT2_TW *CT2_TH * 4)
 // The batched form: level lv of conv_level, Z images (1 or 2) per pair.
 template <int IC, int OC, int ACT, int CS, int PX, int S>
 __global__ void __launch_bounds__(CTB_TW / PX * CTB_TH)
-    k_b_conv2d_wide(NetLaunch L, int lv, int Z, const float *x0, const float *x1,
+    k_b_conv2d_wide(NetLaunch L, int lv, int Z, const float *x0, const float *x1, int dil,
                     const float *__restrict__ w, const float *__restrict__ b, float *y0,
                     float *y1) {
     pdl_sync();
@@ -556,7 +558,7 @@ __global__ void __launch_bounds__(CTB_TW / PX * CTB_TH)
     const int bx = (int)(t % tx), by = (int)(t / tx);
     if (by >= ty) return;
     conv2d_wide_body<IC, OC, ACT, CS, PX, S>(bx, by, net_slab(img ? x1 : x0, L, p), H, W, OH,
-                                             OW, w, b, net_slab(img ? y1 : y0, L, p));
+                                             OW, dil, w, b, net_slab(img ? y1 : y0, L, p));
 }
 
 template <int IC, int OC, int ACT, int CS, int PX, int S>
@@ -568,7 +570,7 @@ static int b_conv2d_wide(const NetLaunch &L, unsigned ctas, int lv, int Z, const
     const int rc = allow_smem(k_b_conv2d_wide<IC, OC, ACT, CS, PX, S>, smem, smem);
     if (rc) return rc;
     pdl(k_b_conv2d_wide<IC, OC, ACT, CS, PX, S>, ctas, CTB_TW / PX * CTB_TH, smem, st)(
-        L, lv, Z, x0, x1, w, b, y0, y1);
+        L, lv, Z, x0, x1, 1, w, b, y0, y1);
     return SV_OK;
 }
 
@@ -1610,9 +1612,10 @@ static int forward_bf16_front(const NetView &n, const float *left, const float *
 }
 
 // Refinement levels of at least so many pixels take k_conv2d_rows; below, its blocks
-// are fewer than the SMs and k_conv2d_tiled's shorter chains win (a 450 x 375 pair,
-// levels up to 38,000 pixels: 399 us, 407 with k_conv2d_rows from 12,000 on; a 320 x
-// 266 forward: 246 us without it at 85,000, 224 with).
+// are fewer than the SMs and k_conv2d_tiled's shorter chains win.  A forward of the
+// 12/6/8 net among others, every level with k_conv2d_tiled / k_conv2d_rows: 30,000
+// pixels 83 / 86 us, 37,600 84 / 87, 43,200 97 / 94, 53,600 120 / 118, 66,000 127 / 124,
+// 85,000 151 / 136, 165,600 248 / 213.
 constexpr long kRowsMin = 40000;
 
 // The network shapes this build instantiates: the reference's shipped
