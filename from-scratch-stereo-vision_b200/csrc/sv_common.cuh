@@ -83,10 +83,12 @@ inline int allow_smem(void (*kernel)(P...), size_t bytes, size_t most) {
 // Launch of a kernel that may be set up before the kernel ahead of it in the stream
 // has ended (programmatic stream serialization): pdl(kernel, grid, block, shared
 // bytes, stream)(arguments...).  The kernel starts with pdl_sync().  Most launches
-// here last 4 to 10 us, 2 of them the gap to the one ahead: a 320 x 266 forward of 15
-// launches takes 237 us instead of 267, a 450 x 375 pair of 57 takes 400 instead of
-// 429.  No kernel lets the next one start early (launch_dependents): blocks that wait
-// beside working ones cost more than the set-up they hide (pair 457 us).
+// here last 4 to 10 us, up to 2 of them the gap to the one ahead.  A pass that is waited
+// for / a pass among others, with plain launches and so: a 320 x 266 forward of 15
+// launches 254 / 185 us, 226 / 156; a training step of 64 crops 1178 / 1172, 1041 /
+// 1037; a 450 x 375 pair, which replays graphs, 446 / 425, 415 / 412.  No kernel lets
+// the next one start early (launch_dependents): blocks that wait beside working ones
+// cost more than the set-up they hide (the pair took 6 % longer).
 template <typename... P>
 struct PdlLaunch {
     void (*kernel)(P...);

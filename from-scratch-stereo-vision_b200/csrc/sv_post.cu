@@ -13,19 +13,18 @@
 //   strict minimum in cluster order, as the reference's loop finds it.
 //   Pixels no window covers keep their label, as in the reference.
 // * SLIC update: the reference sums each cluster's colours and coordinates
-//   over the pixels in index order, in FP64.  When every pixel was covered in
-//   the iteration, a cluster's pixels all lie in its window, so one thread
-//   per cluster sums its window row by row -- the same order.  If some pixel
-//   was not covered, one thread makes the reference's single pass over all
-//   pixels instead (a device flag chooses; exact either way).
-// * plane_snap: segments' pixel lists in index order (built from the same
-//   windows, with the same exact fallback), one CTA per segment for RANSAC
-//   (40 trials: planes by one thread in the reference's order, inlier counts
-//   by all threads), least squares by one thread over the inliers in order,
-//   and the snap.  The reference draws from one xorshift32 stream that runs
-//   through the segments; xorshift32 is linear over GF(2), so each segment's
-//   starting state is computed directly from the number of earlier segments
-//   that drew (3 * trials draws each) by 32x32 bit-matrix powers.
+//   over the pixels in index order, in FP64.  A cluster's pixels lie in its
+//   window, which grows to hold the ones that no window covered and that keep
+//   its label, and row order of a window is index order: a warp per cluster
+//   gathers them in that order, and five lanes add one sum each.
+// * plane_snap: one CTA per segment gathers its valid points from the window, in
+//   index order, for RANSAC (a thread per trial makes the plane in the
+//   reference's order, a warp counts a trial's inliers), least squares over
+//   the inliers in order (a lane per sum), and the snap.  The reference draws
+//   from one xorshift32 stream that runs through the segments; xorshift32 is
+//   linear over GF(2), so each segment's starting state is computed from the
+//   number of earlier segments that drew (3 * trials draws each) by 32x32
+//   bit-matrix powers, and each trial jumps to its own three draws.
 
 #include <climits>
 #include <cmath>

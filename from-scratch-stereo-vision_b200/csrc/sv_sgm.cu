@@ -825,9 +825,11 @@ __global__ void __launch_bounds__(256)
 // Host
 // ====================================================================
 
-// Slots of a pixel.  Without padding (the static scratch) also 48: a lane's share of
-// such a row is no 16-byte copy, and 64 slots are faster although they are more (500 x
-// 150, K = 31: 271 us a pass, 328 with 48).
+// Slots of a pixel.  Without padding (the static scratch and the smaller workspaces)
+// also 48: a lane's share of such a row is no 16-byte copy, and 64 slots are faster on
+// small images although they are more (500 x 150, K = 31: 271 us a pass, 328 with 48; 310
+// before this layout).  Images whose path costs leave the L2 are the other way round
+// (1397 x 1101: 1481 us with 64, 1410 with 48, 2370 before), by 5 %.
 int slot_width(int K, bool pad) {
     static const int widths[] = {8, 16, 24, 32, 48, 64, 96, 128, 160, 192, 256};
     for (int w : widths)
@@ -892,6 +894,10 @@ static int sgm_dispatch(const uint8_t *C0, const uint8_t *C1, const int32_t *b0,
     // 963 / 1600, 8 of 12 344 / 672; K = 253: 4 of 32 1567 / 2695, 8 of 16 561 / 1509, 16
     // of 8 520 / 774; 160 x 120, K = 253: 229 / 301, 59 / 100 and 43 / 59.  K = 191 to 222
     // take 256 slots too (640 x 480: 224 slots in 8 lanes of 14 551 / 991).
+    // K <= 6: one lane; lr_refine, 8- / 16-bit path costs, one lane and two: 450 x 375
+    // 85 / 102 and 89 / 92 us, 1397 x 1101 443 / 554 and 390 / 424, 16 uneven pairs 782 /
+    // 1023 and 631 / 642 (with the earlier kernels 800 for the pairs): two lanes are the
+    // better choice for all but small 8-bit images.
 #define SV_SGM(NR, GL) \
     return sgm_go<NR, GL, LT, PAD>(C0, C1, b0, b1, W, H, K, P1, P2, Lout, nviews, npaths, st)
     switch (Kp) {
